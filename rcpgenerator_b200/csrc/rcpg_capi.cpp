@@ -619,6 +619,7 @@ int32_t rcpg_pairs_forces_scan(uint64_t N, int32_t ndim, const double* x_dev, co
         a.caps_alt = u32(N);
         a.ref_rank = u32(N);
         a.ref_rank_alt = u32(N);
+        a.fpos = static_cast<float*>(sc.get(N * rcpg::search_stride(ndim) * sizeof(float)));
         a.x_last = dbl(N * ndim);
         a.F = dbl(N * ndim);
         a.nbr = u32(static_cast<std::size_t>(row_capacity) * N);

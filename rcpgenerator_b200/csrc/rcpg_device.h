@@ -83,7 +83,7 @@ struct DevCtl {
     std::uint32_t unit_w;
     std::uint32_t unit_chunks;
     std::uint32_t unit_count;
-    std::uint32_t pad1;
+    std::uint32_t stray;  // some particle of this build's search records lies outside the box
 };
 
 // In graph mode every pair-list build stores the particles in cell order
@@ -154,6 +154,10 @@ struct DevArrays {
     std::uint32_t* caps_alt;
     std::uint32_t* ref_rank;
     std::uint32_t* ref_rank_alt;
+    // [N*search_stride(ndim)] FP32 search records in cell order, written by the
+    // builds whose rows k_build_rows searches: position, then the diameter of
+    // the build
+    float* fpos;
     // Captured step graphs with conditional nodes (graph mode): the handle of
     // the step's pair-kernel switch (0 = FP64 kernel, 1 = mixed kernel,
     // 2 = none), set by the step gate and by the build's last kernel; 0 when
@@ -180,6 +184,10 @@ RCPG_HD DevArrays bound_arrays(DevArrays a, std::uint32_t buf) {
 
 constexpr int kForceBlock = 256;
 
+// Floats per search record (DevArrays::fpos): ndim coordinates and the
+// diameter, in whole 16-byte words.
+RCPG_HD constexpr int search_stride(int ndim) { return (ndim + 4) & ~3; }
+
 RCPG_HD unsigned force_blocks(std::uint64_t N) {
     return static_cast<unsigned>((N + kForceBlock - 1) / kForceBlock);
 }
@@ -189,7 +197,7 @@ RCPG_HD unsigned force_blocks(std::uint64_t N) {
 void launch_adam_refresh(const DevArrays& a, int do_adam, int do_refresh, cudaStream_t st);
 void launch_rebuild(const DevArrays& a, cudaStream_t st);
 // the same, with e0 / e1 recorded just before and after the search kernels
-// (the tiled build and the warp search; the one that has nothing to do returns)
+// (the cell-unit or tiled search and the row or warp search; those that have nothing to do return)
 void launch_rebuild_timed(const DevArrays& a, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1);
 void launch_forces(const DevArrays& a, int exact_terms, cudaStream_t st);
 // One variant of the pair kernel (mixed = 0: FP64 pair terms, 1: FP32 pair

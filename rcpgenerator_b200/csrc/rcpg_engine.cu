@@ -178,6 +178,7 @@ void Engine::alloc_device() {
         a_.caps_alt = static_cast<std::uint32_t*>(dalloc(N * 4));
         a_.ref_rank = static_cast<std::uint32_t*>(dalloc(N * 4));
         a_.ref_rank_alt = static_cast<std::uint32_t*>(dalloc(N * 4));
+        a_.fpos = static_cast<float*>(dalloc(N * search_stride(nd) * sizeof(float)));
     } else {
         // the reorder's gather targets and the sorted position copy of the build
         a_.pos_tmp = static_cast<double*>(dalloc(N * P_ * sizeof(double)));
@@ -747,7 +748,7 @@ void Engine::destroy_graph() {
 // (one kernel, or three for more than 4096 tiles of cells), scatter, cell
 // sort, the permutation of cell-order storage, the cell-unit search
 // (ndim <= 3, N >= 20,000; one kernel per pair precision the run may use) or
-// the tiled search, and the warp search.
+// the tiled search, and the row search (graph mode) or the warp search.
 std::uint64_t Engine::kernels_per_build() const {
     const std::uint64_t cells = static_cast<std::uint64_t>(a_.C_alloc) + 1;
     const std::uint64_t scans = cells <= 4096 ? 1 : 3;

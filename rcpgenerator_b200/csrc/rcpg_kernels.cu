@@ -246,6 +246,7 @@ __global__ void k_build_prepare(DevArrays a) {
         // (only with unsorted rows: a sorted row is summed after its sort)
         ctl->forces_done = a.sorted_rows ? 0u : ctl->fuse_forces;
         ctl->row_need = 0u;
+        ctl->stray = 0u;
         ctl->nbuilds += 1u;
     }
 }
@@ -338,7 +339,7 @@ template <int ND>
 __device__ __forceinline__ bool tiled_build_ok(const DevCtl* ctl);
 
 // Particles below which the tiled search is not used: a small packing has too
-// few tiles to fill the GPU, and the warp search (k_build_search) spreads one
+// few tiles to fill the GPU, and the warp and row searches spread one
 // particle over 32 lanes instead.
 constexpr std::uint64_t kTiledMinN = 20000;
 
@@ -416,6 +417,32 @@ __global__ void __launch_bounds__(256) k_build_cell_sort(DevArrays a) {
     }
 }
 
+// FP32 search record of particle q (DevArrays::fpos). A coordinate outside the
+// box (by more than a millionth of it) becomes NaN, which fails no FP32 test of
+// k_build_rows, and DevCtl::stray keeps its geometric pruning off: such a
+// particle sits in a boundary cell that its position does not belong to.
+template <int ND>
+__device__ __forceinline__ void store_search_record(const DevArrays& a, DevCtl* ctl, std::uint64_t q,
+                                                    const double* x, double D0) {
+    constexpr int FP = search_stride(ND);
+    float r[FP];
+    RCPG_UNROLL
+    for (int d = 0; d < FP; ++d) r[d] = 0.0f;
+    bool inside = true;
+    RCPG_UNROLL
+    for (int d = 0; d < ND; ++d) {
+        const double L = ctl->g.box[d];
+        const bool in = x[d] >= -1e-6 * L && x[d] <= (1.0 + 1e-6) * L;
+        r[d] = in ? static_cast<float>(x[d]) : __int_as_float(0x7fffffff);
+        inside = inside && in;
+    }
+    if (!inside) ctl->stray = 1u;
+    r[ND] = static_cast<float>(xmul(D0, ctl->build_kappa));
+    float4* dst = reinterpret_cast<float4*>(a.fpos + q * FP);
+    RCPG_UNROLL
+    for (int h = 0; h < FP / 4; ++h) dst[h] = make_float4(r[4 * h], r[4 * h + 1], r[4 * h + 2], r[4 * h + 3]);
+}
+
 // Cell-order storage (graph mode): particle q of the new order is particle
 // work[q] of the current one (cells in grid order, each cell's members in
 // their current order, written by k_build_cell_sort). Moves the per-particle
@@ -429,6 +456,7 @@ __global__ void __launch_bounds__(256) k_build_permute(DevArrays a) {
     const std::uint32_t b = ctl->buf;
     const DevArrays src = bound_arrays(a, b), dst = bound_arrays(a, b ^ 1u);
     constexpr int P = pos_stride(ND);
+    const bool search = !use_cells<ND>(a);  // k_build_rows reads the FP32 search records
     const std::uint64_t N = a.N;
     // two particles per thread, every load of both before any store
     const std::uint64_t stride = static_cast<std::uint64_t>(gridDim.x) * blockDim.x;
@@ -475,6 +503,17 @@ __global__ void __launch_bounds__(256) k_build_permute(DevArrays a) {
             dst.origin[q] = org[u];
             dst.caps[q] = cap[u];
             dst.ref_rank[q] = rr[u];
+            if (search) {
+                double xq[ND], D0q = 0.0;
+                RCPG_UNROLL
+                for (int h = 0; h < P / 2; ++h) {
+                    if (2 * h < ND) xq[2 * h] = rec[u][h].x;
+                    else if (2 * h == ND) D0q = rec[u][h].x;
+                    if (2 * h + 1 < ND) xq[2 * h + 1] = rec[u][h].y;
+                    else if (2 * h + 1 == ND) D0q = rec[u][h].y;
+                }
+                store_search_record<ND>(a, ctl, q, xq, D0q);
+            }
         }
     }
     __syncthreads();
@@ -488,16 +527,15 @@ __global__ void __launch_bounds__(256) k_build_permute(DevArrays a) {
     }
 }
 
-// Warp search (every build the tiled search does not take: ndim > 3, small
-// packings, grids narrower than a tile). One warp per row slot t (particle
-// work[t]). The neighbour cells are taken 32 at a time: each lane reads one
-// cell's member range, a warp scan numbers the chunk's candidates, and the
-// lanes test consecutive candidates (each finds its cell by a binary search
-// over the lanes' ranges), so every lane has a candidate in every round
-// whatever the cell occupancy. Accepted partners take row slots in candidate
-// order (ballot + popc): the row is in a fixed scan order. Rows that must be
-// sorted (sorted_rows: exact mode) are then sorted ascending by a bitonic
-// sort in the warp.
+// Warp search of the builds with sorted rows (exact mode and the stand-alone
+// pair build) that the tiled search does not take: ndim > 3, small packings,
+// grids narrower than a tile. One warp per row slot t (particle work[t]). The
+// neighbour cells are taken 32 at a time: each lane reads one cell's member
+// range, a warp scan numbers the chunk's candidates, and the lanes test
+// consecutive candidates (each finds its cell by a binary search over the
+// lanes' ranges), so every lane has a candidate in every round whatever the
+// cell occupancy. Accepted partners take row slots in candidate order
+// (ballot + popc) and are then sorted ascending by a bitonic sort in the warp.
 constexpr int kWarpSearchWarps = 4;    // warps per block
 constexpr int kWarpRowSmem = 256;      // row entries held (and sorted) in shared memory
 
@@ -505,14 +543,7 @@ template <int ND>
 __global__ void __launch_bounds__(32 * kWarpSearchWarps) k_build_search(DevArrays a) {
     DevCtl* ctl = a.ctl;
     const std::uint64_t N = a.N;
-    const bool other = use_tiled<ND>(a) || use_cells<ND>(a);
-    if (a.cond_forces && blockIdx.x == 0 && threadIdx.x == 0 && !build_off(ctl)) {
-        // last kernel of the build in a step graph: the pair kernel runs
-        // unless another search computed this step's forces
-        const std::uint32_t fd = other ? ctl->forces_done : 0u;
-        cudaGraphSetConditional(a.cond_forces, forces_case(fd == 0u, ctl->pair_fp32, a.mixed));
-    }
-    if (build_off(ctl) || other) return;
+    if (build_off(ctl) || use_tiled<ND>(a)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->forces_done = 0u;
     __shared__ std::uint32_t buf[kWarpSearchWarps][kWarpRowSmem];
     __shared__ std::uint32_t block_need;
@@ -530,15 +561,10 @@ __global__ void __launch_bounds__(32 * kWarpSearchWarps) k_build_search(DevArray
     }
     const int K = ctl->nclass > 1 ? ctl->nclass : 1;
     std::uint32_t* row = buf[w];
-    // cell-order storage: slot t is particle t, and the cells' members are
-    // contiguous in pos itself
-    bind_buffers(a);
-    const bool perm = a.permute != 0;
-    const double* cpos = perm ? a.pos : a.spos;
+    const double* cpos = a.spos;
     const std::uint64_t warps = static_cast<std::uint64_t>(gridDim.x) * kWarpSearchWarps;
     for (std::uint64_t t = blockIdx.x * static_cast<std::uint64_t>(kWarpSearchWarps) + w; t < N; t += warps) {
-        const std::uint32_t i = perm ? static_cast<std::uint32_t>(t) : a.work[t];
-        const std::uint32_t ri = perm ? a.ref_rank[i] : i;  // the reference's index (half-row count)
+        const std::uint32_t i = a.work[t];
         double xi[ND], D0i;
         load_pos<ND>(cpos, t, xi, D0i);
         const double Di = xmul(D0i, kap);
@@ -619,7 +645,7 @@ __global__ void __launch_bounds__(32 * kWarpSearchWarps) k_build_search(DevArray
                     const std::uint32_t own_cnt = __shfl_sync(0xffffffffu, cntc, own);
                     if (k < tot) {
                         const std::uint32_t q = own_q0 + (k - (own_incl - own_cnt));
-                        j = perm ? q : a.work[q];
+                        j = a.work[q];
                         if (j != i) {
                             double xj[ND], D0j;
                             load_pos<ND>(cpos, q, xj, D0j);
@@ -634,7 +660,7 @@ __global__ void __launch_bounds__(32 * kWarpSearchWarps) k_build_search(DevArray
                         const std::uint32_t slot = n + __popc(mask & ((1u << lane) - 1u));
                         if (slot < static_cast<std::uint32_t>(kWarpRowSmem)) row[slot] = j;
                         else if (slot < S) a.nbr[static_cast<std::uint64_t>(slot) * N + t] = j;
-                        if (perm ? (a.ref_rank[j] > ri) : (j > i)) ++n_half;
+                        if (j > i) ++n_half;
                     }
                     n += static_cast<std::uint32_t>(__popc(mask));
                 }
@@ -645,16 +671,12 @@ __global__ void __launch_bounds__(32 * kWarpSearchWarps) k_build_search(DevArray
         for (int o = 16; o > 0; o >>= 1) n_half += __shfl_xor_sync(0xffffffffu, n_half, o);
         if (lane == 0) {
             const std::uint32_t cap = a.caps[i];
-            if (n_half > cap) report_cap_error(ctl, ri, cap);
+            if (n_half > cap) report_cap_error(ctl, i, cap);
             atomicMax(&block_need, n);
             a.nbr_cnt[t] = n > S ? 0u : n;  // overflow: empty row, rebuilt after the capacity grows
         }
         if (n > S) continue;
-        if (!a.sorted_rows) {
-            // scan-order row: the shared part goes out as it is
-            const std::uint32_t ns = n < static_cast<std::uint32_t>(kWarpRowSmem) ? n : kWarpRowSmem;
-            for (std::uint32_t e = lane; e < ns; e += 32) a.nbr[static_cast<std::uint64_t>(e) * N + t] = row[e];
-        } else if (n <= static_cast<std::uint32_t>(kWarpRowSmem)) {
+        if (n <= static_cast<std::uint32_t>(kWarpRowSmem)) {
             // bitonic sort of the row padded to a power of two
             std::uint32_t p2 = 1;
             while (p2 < n) p2 <<= 1;
@@ -696,6 +718,459 @@ __global__ void __launch_bounds__(32 * kWarpSearchWarps) k_build_search(DevArray
     }
     __syncthreads();
     if (threadIdx.x == 0 && block_need) atomicMax(&ctl->row_need, block_need);
+}
+
+// Row search of the graph engine (cell-order storage, rows in scan order):
+// every build the cell-unit search does not take (ndim > 3, several size
+// classes, small packings, narrow grids). Along axis 0 the neighbour cells of
+// a particle are consecutive, so in cell-order storage their members are one
+// contiguous range of particles (two where the range wraps): a particle scans
+// nn_1 * nn_2 * ... such ranges per size class instead of nn_0 times as many
+// cells.
+//
+// Two tests keep candidates away from the FP64 predicate. (1) A range whose
+// cells lie farther from the particle than the largest cutoff to a member of
+// their class is not visited, and the others are shortened to the cells within
+// that cutoff (a ball touches a third to two thirds of the cells of its
+// bounding cube in 3 and 4 dimensions, fewer where the particle is smaller
+// than the grid's). (2) A candidate is tested in FP32 on its search record
+// with the minimum image min(|t|, L - |t|): four instructions per axis, no
+// branch and no round, where the FP64 predicate takes seven at half the rate.
+// Both are widened past every rounding (kSearchRel, kSearchAbs), so neither
+// drops a partner; the candidates left are listed in scan order in shared
+// memory and tested by the FP64 predicate, densely.
+//
+// G lanes share a particle. G = 1: one thread walks the ranges in order
+// (consecutive threads are neighbours in space, so their ranges overlap and
+// stay in L1). G > 1: the lanes read the ranges of G grid rows, number
+// their candidates with a scan over the lanes and test G consecutive
+// candidates at a time; ballots keep the scan order. The scan
+// order -- size classes, then the cells with axis 0 fastest, then the
+// members -- does not depend on G, so neither do the rows. row_lanes() picks G
+// per size class: the particles of a class are consecutive, and those of a
+// larger class have several times the candidates (one G for all classes left
+// the few large particles of a power law running alone: 404 us against 212).
+//
+// Bound by instruction issue (about 20 ranges of 1 to 2 candidates per particle
+// where cells hold half a particle) and, for small packings, by the latency of
+// cell start -> record -> test. One B200, per build, against the
+// warp-per-particle search over single cells in FP64 that it replaces: 3-D
+// power law N = 300,007 790 -> 212 us; 4-D log-normal N = 12,001 255 -> 96 us
+// early in the run.
+constexpr int kRowThreads = 128;
+constexpr int kRowList = 24;          // listed candidates per lane
+// In box sides: the FP32 rounding of a position, of t and of L - |t| is at most
+// 1.2e-7 per axis (3.4e-7 in 8 dimensions), and positions may lie 1e-6 outside
+// the box; relative: the sum of squares and the cutoff round by less than 1e-6.
+constexpr float kSearchAbs = 3e-6f, kSearchRel = 1.000004f;
+
+template <int ND>
+struct SearchRecord {
+    float x[ND], D;
+};
+
+template <int ND>
+__device__ __forceinline__ SearchRecord<ND> load_search_record(const float* fpos, std::uint32_t q) {
+    constexpr int FP = search_stride(ND);
+    float w[FP];
+    const float4* p = reinterpret_cast<const float4*>(fpos + static_cast<std::uint64_t>(q) * FP);
+    RCPG_UNROLL
+    for (int h = 0; h < FP / 4; ++h) {
+        const float4 v = __ldg(p + h);
+        w[4 * h] = v.x;
+        w[4 * h + 1] = v.y;
+        w[4 * h + 2] = v.z;
+        w[4 * h + 3] = v.w;
+    }
+    SearchRecord<ND> r;
+    RCPG_UNROLL
+    for (int d = 0; d < ND; ++d) r.x[d] = w[d];
+    r.D = w[ND];
+    return r;
+}
+
+// FP32 test of candidate j for particle i: false only for a pair outside the
+// shell. half_i = widened Di/2 + t.
+template <int ND>
+__device__ __forceinline__ bool maybe_partner(const SearchRecord<ND>& i, float half_i, const SearchRecord<ND>& j,
+                                              const float* side) {
+    float d2 = 0.0f;
+    RCPG_UNROLL
+    for (int d = 0; d < ND; ++d) {
+        const float t = fabsf(j.x[d] - i.x[d]);
+        const float m = fminf(t, side[d] - t);
+        d2 = __fmaf_rn(m, m, d2);
+    }
+    const float rc = __fmaf_rn(j.D, 0.5f * kSearchRel, half_i);
+    return !(d2 > rc * rc);
+}
+
+// The neighbourhood of particle (xi, Di) in the grid of size class kc: cells
+// lo .. lo + nn - 1 per axis (periodic), nn_1 * nn_2 * ... ranges along axis 0.
+template <int ND>
+struct RowScan {
+    int nc[ND], nn[ND], lo[ND];
+    std::uint32_t base;
+    int rows;
+    float x[ND], cell[ND];  // position, cell width
+    float rcut, rcut2;      // widened largest cutoff; infinite: no pruning
+
+    __device__ __forceinline__ void open(const DevCtl* ctl, int kc, int K, double kap, double t_shell,
+                                         const double* xi, double Di, const float* side, float widest, bool prune) {
+        const double dmax = K > 1 ? xmul(ctl->class_d0max[kc], kap) : ctl->build_Dmax;
+        const double rc = (Di + dmax) * 0.5 + t_shell;
+        rows = 1;
+        RCPG_UNROLL
+        for (int d = 0; d < ND; ++d) {
+            const double scale = ctl->cls_scale[kc][d];
+            nc[d] = ctl->cls_ncell[kc][d];
+            // cells per cutoff on this axis: 1 with one grid (cells are at
+            // least one cutoff wide), computed per class otherwise
+            double mm = 1.0;
+            if (K > 1) {
+                mm = ceil(rc * scale * (1.0 + 1e-6));
+                if (!(mm >= 1.0)) mm = 1.0;
+            }
+            if (!(2.0 * mm + 1.0 <= static_cast<double>(nc[d]))) {
+                nn[d] = nc[d];  // every cell of the axis, once
+                lo[d] = 0;
+            } else {
+                const int m = static_cast<int>(mm);
+                nn[d] = 2 * m + 1;
+                lo[d] = cell_coord(xi[d], scale, nc[d]) - m;
+            }
+            if (d > 0) rows *= nn[d];
+            x[d] = static_cast<float>(xi[d]);
+            cell[d] = __fdividef(side[d], static_cast<float>(nc[d]));
+        }
+        base = ctl->cls_base[kc];
+        rcut = prune ? __fmaf_rn(static_cast<float>(rc), kSearchRel * kSearchRel, 2.0f * kSearchAbs * widest) : HUGE_VALF;
+        rcut2 = rcut * rcut;
+    }
+    // Cell k of axis d: its periodic index, and far2 plus its squared distance
+    // on that axis from the particle.
+    __device__ __forceinline__ float axis(int d, int k, const float* side, float far2, int& c) const {
+        c = lo[d] + k;
+        if (c < 0) c += nc[d];
+        else if (c >= nc[d]) c -= nc[d];
+        float t = fabsf(__fmaf_rn(static_cast<float>(c) + 0.5f, cell[d], -x[d]));
+        t = fmaxf(fminf(t, side[d] - t) - 0.5f * cell[d], 0.0f);
+        return __fmaf_rn(t, t, far2);
+    }
+    // The particle ranges [q0, q1), then [q2, q3), of the grid row that starts
+    // at cell `row` and lies far2 away over the other axes (far2 <= rcut2); the
+    // cells beyond the rest of the cutoff are left out.
+    __device__ __forceinline__ void ranges(const std::uint32_t* cell_start, std::uint32_t row, float far2,
+                                           const float* side, std::uint32_t& q0, std::uint32_t& q1,
+                                           std::uint32_t& q2, std::uint32_t& q3) const {
+        q0 = q1 = q2 = q3 = 0u;
+        int b = lo[0], e = lo[0] + nn[0];
+        if (nn[0] < nc[0] && rcut2 < HUGE_VALF) {
+            const float r = sqrtf(rcut2 - far2);
+            const float inv = __fdividef(static_cast<float>(nc[0]), side[0]);
+            b = max(b, __float2int_rd((x[0] - r) * inv));
+            e = min(e, __float2int_rd((x[0] + r) * inv) + 1);
+            if (b >= e) return;
+        }
+        const std::uint32_t* cs = cell_start + base + row;
+        if (b < 0 || e > nc[0]) {
+            if (b >= nc[0] || e <= 0) {  // wholly beyond one end
+                const int shift = e <= 0 ? nc[0] : -nc[0];
+                b += shift;
+                e += shift;
+            } else {
+                q2 = cs[0];
+                q3 = cs[b < 0 ? e : e - nc[0]];
+                if (b < 0) b += nc[0];
+                e = nc[0];
+            }
+        }
+        q0 = cs[b];
+        q1 = cs[e];
+    }
+    // body(q0, q1, q2, q3) for every grid row within the cutoff, in order (axis 1 fastest)
+    template <int D = ND - 1, typename Body>
+    __device__ __forceinline__ void each_row(const std::uint32_t* cell_start, const float* side, const Body& body,
+                                             std::uint32_t part = 0, float far2 = 0.0f) const {
+        for (int k = 0; k < nn[D]; ++k) {
+            int c;
+            const float f = axis(D, k, side, far2, c);
+            if (f > rcut2) continue;
+            const std::uint32_t row = (part + static_cast<std::uint32_t>(c)) * static_cast<std::uint32_t>(nc[D - 1]);
+            if constexpr (D == 1) {
+                std::uint32_t q0, q1, q2, q3;
+                ranges(cell_start, row, f, side, q0, q1, q2, q3);
+                body(q0, q1, q2, q3);
+            } else {
+                each_row<D - 1>(cell_start, side, body, row, f);
+            }
+        }
+    }
+    // the ranges of row number r in that order (empty beyond the cutoff)
+    __device__ __forceinline__ void row_ranges(int r, const std::uint32_t* cell_start, const float* side,
+                                               std::uint32_t& q0, std::uint32_t& q1, std::uint32_t& q2,
+                                               std::uint32_t& q3) const {
+        int off[ND];
+        RCPG_UNROLL
+        for (int d = 1; d < ND; ++d) {
+            const int up = static_cast<int>((static_cast<float>(r) + 0.5f) * __frcp_rn(static_cast<float>(nn[d])));
+            off[d] = r - up * nn[d];
+            r = up;
+        }
+        std::uint32_t row = 0;
+        float f = 0.0f;
+        RCPG_UNROLL
+        for (int d = ND - 1; d > 0; --d) {
+            int c;
+            f = axis(d, off[d], side, f, c);
+            row = (row + static_cast<std::uint32_t>(c)) * static_cast<std::uint32_t>(nc[d - 1]);
+        }
+        q0 = q1 = q2 = q3 = 0u;
+        if (!(f > rcut2)) ranges(cell_start, row, f, side, q0, q1, q2, q3);
+    }
+};
+
+// The row's end: capacity checks and the published length (as in k_cells).
+template <int ND>
+__device__ __forceinline__ void close_row(const DevArrays& a, DevCtl* ctl, std::uint32_t t, std::uint32_t n) {
+    const std::uint64_t N = a.N;
+    const std::uint32_t cap = a.caps[t];
+    if (n > cap && n <= a.S) {
+        // the reference's capacity check counts the partners after t in its own
+        // order; a row that fits the capacity in full needs no count
+        const std::uint32_t rt = a.ref_rank[t];
+        std::uint32_t n_half = 0;
+        for (std::uint32_t k = 0; k < n; ++k)
+            n_half += a.ref_rank[a.nbr[static_cast<std::uint64_t>(k) * N + t]] > rt;
+        if (n_half > cap) report_cap_error(ctl, rt, cap);
+    }
+    a.nbr_cnt[t] = n > a.S ? 0u : n;  // overflow: empty row, rebuilt after the capacity grows
+}
+
+// Lanes per particle of size class k, g0 those of the two smallest classes (for
+// the second a thread per particle still measured faster: 212 us against 247).
+__device__ __forceinline__ int row_lanes(int g0, int k) {
+    const int g = k <= 1 ? g0 : (2 * g0) << (k < 6 ? k - 1 : 5);
+    return g < 32 ? g : 32;
+}
+
+// One particle's search state (k_build_rows).
+template <int ND>
+struct RowSearch {
+    std::uint32_t t, n, listed;  // particle; row length and listed candidates so far
+    double xi[ND], Di;
+    SearchRecord<ND> ri;
+    float half_i;
+
+    __device__ __forceinline__ void begin(const DevArrays& a, std::uint32_t p, double kap, double t_shell, float widest) {
+        t = p;
+        n = listed = 0;
+        double D0;
+        load_pos<ND>(a.pos, t, xi, D0);
+        Di = xmul(D0, kap);
+        ri = load_search_record<ND>(a.fpos, t);
+        half_i = __fmaf_rn(__fmaf_rn(ri.D, 0.5f, static_cast<float>(t_shell)), kSearchRel, kSearchAbs * widest);
+    }
+    // FP64 predicate of listed candidate q
+    __device__ __forceinline__ bool partner(const DevArrays& a, const DevCtl* ctl, std::uint32_t q, double kap,
+                                            double t_shell) const {
+        double xj[ND], D0j;
+        load_pos_g<ND>(a.pos, q, xj, D0j, 1);
+        const double Dj = xmul(D0j, kap);
+        return q != t && ((ND <= 3 || q > t) ? in_shell<ND>(xi, xj, Di, Dj, ctl->g.box, ctl->g.inv_box, t_shell)
+                                             : in_shell<ND>(xi, xj, Dj, Di, ctl->g.box, ctl->g.inv_box, t_shell));
+    }
+};
+
+template <int ND>
+__global__ void __launch_bounds__(kRowThreads) k_build_rows(DevArrays a, int g0) {
+    DevCtl* ctl = a.ctl;
+    const bool other = use_cells<ND>(a);
+    if (a.cond_forces && blockIdx.x == 0 && threadIdx.x == 0 && !build_off(ctl)) {
+        // last kernel of the build in a step graph: the pair kernel runs
+        // unless another search computed this step's forces
+        const std::uint32_t fd = other ? ctl->forces_done : 0u;
+        cudaGraphSetConditional(a.cond_forces, forces_case(fd == 0u, ctl->pair_fp32, a.mixed));
+    }
+    if (build_off(ctl) || other) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->forces_done = 0u;
+    bind_buffers(a);
+    const std::uint32_t S = a.S;
+    const std::uint64_t N = a.N;
+    const double kap = ctl->build_kappa, t_shell = ctl->build_t_shell;
+    const int K = ctl->nclass > 1 ? ctl->nclass : 1;
+    const float* const fpos = a.fpos;
+    const bool prune = ctl->stray == 0u;
+    float side[ND], widest = 0.0f;
+    RCPG_UNROLL
+    for (int d = 0; d < ND; ++d) {
+        side[d] = static_cast<float>(ctl->g.box[d]);
+        widest = fmaxf(widest, side[d]);
+    }
+    // each warp has its own lists and ranges (the warps of a block may be at units with different G)
+    __shared__ std::uint32_t s_list[kRowThreads / 32][32 * (kRowList + 1)];
+    // up to two ranges per lane: first particle - candidates before the range; candidates up to and including it
+    __shared__ std::uint32_t s_q[kRowThreads / 32][64], s_end[kRowThreads / 32][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // work units of a block's width, the largest class first: first unit and first particle of each class
+    __shared__ std::uint32_t s_unit[kMaxClass + 1], s_first[kMaxClass + 1];
+    if (threadIdx.x == 0) {
+        std::uint32_t units = 0;
+        s_first[K] = static_cast<std::uint32_t>(N);
+        for (int k = K - 1; k >= 0; --k) {
+            s_first[k] = a.cell_start[ctl->cls_base[k]];
+            s_unit[k + 1] = units;
+            const std::uint32_t per = static_cast<std::uint32_t>(kRowThreads / row_lanes(g0, k));
+            units += (s_first[k + 1] - s_first[k] + per - 1) / per;
+        }
+        s_unit[0] = units;
+    }
+    __syncthreads();
+    const std::uint32_t units = s_unit[0];
+    std::uint32_t need = 0;
+    int kcls = K - 1;  // class of the unit: units of class k are s_unit[k+1] .. s_unit[k] - 1
+    for (std::uint32_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        __syncwarp();  // every group of the warp is done with the previous unit's lists
+        while (unit >= s_unit[kcls]) --kcls;
+        const int G = row_lanes(g0, kcls);
+        const std::uint32_t t = s_first[kcls] + (unit - s_unit[kcls + 1]) * static_cast<std::uint32_t>(kRowThreads / G) +
+                                static_cast<std::uint32_t>(threadIdx.x / G);
+        const bool live = t < s_first[kcls + 1];
+        if (G == 1) {
+            if (!live) continue;
+            std::uint32_t* const list = s_list[warp] + lane * (kRowList + 1);  // odd stride: no bank conflicts
+            RowSearch<ND> rs;
+            rs.begin(a, t, kap, t_shell, widest);
+            auto flush = [&]() {
+                for (std::uint32_t k = 0; k < rs.listed; ++k) {
+                    const std::uint32_t q = list[k];
+                    if (rs.partner(a, ctl, q, kap, t_shell)) {
+                        if (rs.n < S) a.nbr[static_cast<std::uint64_t>(rs.n) * N + t] = q;
+                        ++rs.n;
+                    }
+                }
+                rs.listed = 0;
+            };
+            for (int kc = 0; kc < K; ++kc) {
+                RowScan<ND> sc;
+                sc.open(ctl, kc, K, kap, t_shell, rs.xi, rs.Di, side, widest, prune);
+                sc.each_row(a.cell_start, side, [&](std::uint32_t q, std::uint32_t qe, std::uint32_t q2, std::uint32_t q3) {
+                    for (;;) {
+                        if (q >= qe) {  // the wrapped part of the range, then done
+                            if (q2 >= q3) break;
+                            q = q2;
+                            qe = q3;
+                            q2 = q3;
+                        }
+                        constexpr std::uint32_t U = 2;  // candidates in flight
+                        bool hit[U];
+                        RCPG_UNROLL
+                        for (std::uint32_t u = 0; u < U; ++u)
+                            hit[u] = maybe_partner<ND>(rs.ri, rs.half_i,
+                                                       load_search_record<ND>(fpos, min(q + u, qe - 1)), side) &&
+                                     q + u < qe;
+                        RCPG_UNROLL
+                        for (std::uint32_t u = 0; u < U; ++u)
+                            if (hit[u]) list[rs.listed++] = q + u;
+                        q += U;
+                        if (rs.listed > static_cast<std::uint32_t>(kRowList) - U) flush();
+                    }
+                });
+            }
+            flush();
+            close_row<ND>(a, ctl, t, rs.n);
+            need = max(need, rs.n);
+        } else {
+            if (!live) continue;  // whole groups
+            const int s = lane & (G - 1), grp = lane / G;
+            const unsigned gmask = (0xffffffffu >> (32 - G)) << (lane & ~(G - 1));
+            const unsigned below = (1u << lane) - 1u;
+            const std::uint32_t L = static_cast<std::uint32_t>(kRowList * G);
+            std::uint32_t* const list = s_list[warp] + grp * L;
+            std::uint32_t* const sq = s_q[warp] + grp * 2 * G;
+            std::uint32_t* const se = s_end[warp] + grp * 2 * G;
+            RowSearch<ND> rs;
+            rs.begin(a, t, kap, t_shell, widest);
+            // partners among the listed candidates, appended to the row in order
+            auto flush = [&]() {
+                __syncwarp(gmask);
+                for (std::uint32_t k0 = 0; k0 < rs.listed; k0 += G) {
+                    const std::uint32_t k = k0 + s;
+                    const std::uint32_t q = k < rs.listed ? list[k] : t;
+                    const bool ok = k < rs.listed && rs.partner(a, ctl, q, kap, t_shell);
+                    const unsigned hits = __ballot_sync(gmask, ok) & gmask;
+                    const std::uint32_t slot = rs.n + __popc(hits & below);
+                    if (ok && slot < S) a.nbr[static_cast<std::uint64_t>(slot) * N + t] = q;
+                    rs.n += static_cast<std::uint32_t>(__popc(hits));
+                }
+                rs.listed = 0;
+                __syncwarp(gmask);
+            };
+            for (int kc = 0; kc < K; ++kc) {
+                RowScan<ND> sc;
+                sc.open(ctl, kc, K, kap, t_shell, rs.xi, rs.Di, side, widest, prune);
+                for (int r0 = 0; r0 < sc.rows; r0 += G) {
+                    // the ranges of row r0 + s; numbers of the non-empty ranges and of their candidates
+                    std::uint32_t q0 = 0, q1 = 0, q2 = 0, q3 = 0;
+                    if (r0 + s < sc.rows) sc.row_ranges(r0 + s, a.cell_start, side, q0, q1, q2, q3);
+                    const std::uint32_t n0 = q1 - q0, n1 = q3 - q2;
+                    std::uint32_t ci = n0 + n1, ei = (n0 != 0u) + (n1 != 0u);
+                    for (int o = 1; o < G; o <<= 1) {
+                        const std::uint32_t cv = __shfl_up_sync(gmask, ci, o, G), ev = __shfl_up_sync(gmask, ei, o, G);
+                        if (s >= o) {
+                            ci += cv;
+                            ei += ev;
+                        }
+                    }
+                    const std::uint32_t T = __shfl_sync(gmask, ci, G - 1, G);
+                    if (T == 0) continue;
+                    ci -= n0 + n1;
+                    ei -= (n0 != 0u) + (n1 != 0u);
+                    __syncwarp(gmask);  // the previous ranges are no longer read
+                    if (n0) {
+                        sq[ei] = q0 - ci;
+                        ci += n0;
+                        se[ei++] = ci;
+                    }
+                    if (n1) {
+                        sq[ei] = q2 - ci;
+                        se[ei] = ci + n1;
+                    }
+                    __syncwarp(gmask);
+                    // G consecutive candidates per round, two rounds in flight
+                    int e = 0;
+                    for (std::uint32_t k0 = 0; k0 < T; k0 += 2 * G) {
+                        if (rs.listed > L - 2 * G) flush();
+                        std::uint32_t q[2];
+                        bool hit[2];
+                        RCPG_UNROLL
+                        for (int u = 0; u < 2; ++u) {
+                            const std::uint32_t k = k0 + static_cast<std::uint32_t>(u * G + s);
+                            hit[u] = k < T;
+                            if (hit[u])
+                                while (k >= se[e]) ++e;
+                            q[u] = hit[u] ? k + sq[e] : t;
+                        }
+                        RCPG_UNROLL
+                        for (int u = 0; u < 2; ++u)
+                            hit[u] = maybe_partner<ND>(rs.ri, rs.half_i, load_search_record<ND>(fpos, q[u]), side) && hit[u];
+                        RCPG_UNROLL
+                        for (int u = 0; u < 2; ++u) {
+                            const unsigned hits = __ballot_sync(gmask, hit[u]) & gmask;
+                            if (hit[u]) list[rs.listed + __popc(hits & below)] = q[u];
+                            rs.listed += static_cast<std::uint32_t>(__popc(hits));
+                        }
+                    }
+                }
+            }
+            flush();
+            if (s == 0) close_row<ND>(a, ctl, t, rs.n);
+            need = max(need, rs.n);
+        }
+    }
+    // longest row: one atomic per warp
+    need = __reduce_max_sync(0xffffffffu, need);
+    if ((threadIdx.x & 31) == 0 && need) atomicMax(&ctl->row_need, need);
 }
 
 // ---- tiled search (ndim 2, 3) ---------------------------------------------
@@ -2333,6 +2808,30 @@ void launch_cells(const DevArrays& a, cudaStream_t st) {
     if (a.mixed) launch_cells_variant<ND, true>(a, st);
 }
 
+template <int ND>
+void launch_warp_search(const DevArrays& a, cudaStream_t st) {
+    const unsigned need = static_cast<unsigned>((a.N + kWarpSearchWarps - 1) / kWarpSearchWarps),
+                   g = resident_grid<k_build_search<ND>>(32 * kWarpSearchWarps);
+    k_build_search<ND><<<need < g ? need : g, 32 * kWarpSearchWarps, 0, st>>>(a);
+}
+
+// Lanes per particle of k_build_rows (the smallest size class): one once the
+// packing alone fills the GPU, more below that. Measured per build on one
+// B200: 3-D log-normal N = 50,003 65 us (1 lane) against 113 (4); N = 8,000 28
+// us (8) against 43 (4) and 37 (32); N = 2,000 11 us (32) against 15 (8). In
+// 4-D a particle has ten times the candidates: N = 30,000 208 us (8) against
+// 251 (4) and 214 (32), N = 12,001 128 us (32) against 151 (8).
+template <int ND>
+int search_lanes(std::uint64_t N) {
+    if (ND <= 3) return N >= 32768 ? 1 : (N >= 4096 ? 8 : 32);
+    return N >= 20000 ? 8 : 32;
+}
+
+template <int ND>
+void launch_rows(const DevArrays& a, cudaStream_t st) {
+    k_build_rows<ND><<<resident_grid<k_build_rows<ND>>(kRowThreads), kRowThreads, 0, st>>>(a, search_lanes<ND>(a.N));
+}
+
 // e0 / e1 (optional): events recorded around the search kernels only
 template <int ND>
 void rebuild_impl(const DevArrays& a, cudaStream_t st, cudaEvent_t e0 = nullptr, cudaEvent_t e1 = nullptr) {
@@ -2349,16 +2848,15 @@ void rebuild_impl(const DevArrays& a, cudaStream_t st, cudaEvent_t e0 = nullptr,
         k_build_permute<ND><<<need < g ? need : g, 256, 0, st>>>(a);
     }
     if (e0) cudaEventRecord(e0, st);
-    if (ND <= 3 && a.N >= kTiledMinN) {  // smaller packings take the warp search
+    if (ND <= 3 && a.N >= kTiledMinN) {  // smaller packings take the row or the warp search
         if (a.permute) {
             launch_cells<ND>(a, st);
         } else if (a.sorted_rows) {
             launch_tiled<ND>(a, st);
         }
     }
-    const unsigned need = static_cast<unsigned>((a.N + kWarpSearchWarps - 1) / kWarpSearchWarps),
-                   g = resident_grid<k_build_search<ND>>(32 * kWarpSearchWarps);
-    k_build_search<ND><<<need < g ? need : g, 32 * kWarpSearchWarps, 0, st>>>(a);
+    if (a.permute) launch_rows<ND>(a, st);
+    else launch_warp_search<ND>(a, st);
     if (e1) cudaEventRecord(e1, st);
 }
 
