@@ -258,11 +258,10 @@ RCPG_HD bool pair_force(const double* xi, double Di, const double* xj, double Dj
 
 // Flat walls and the curved container acting on particle i, added to its
 // force after all pair terms, in the reference's order (ENG:4198-4257:
-// axes ascending, wall 0 then wall 1, then the container). The scalar
-// contributions are added in that same order to the three wall_* sums.
-template <int ND, typename CountT>
-RCPG_HD void wall_forces(const double* xi, double Di, const Geometry& g, double* fi,
-                         double& U, double& dk, double& Fm, CountT& count) {
+// axes ascending, wall 0 then wall 1, then the container). Each contact's
+// scalar terms go to sink(U, dk, Fm), in that order.
+template <int ND, typename Sink>
+RCPG_HD void wall_terms(const double* xi, double Di, const Geometry& g, double* fi, Sink&& sink) {
     if (g.any_flat_wall) {
 RCPG_UNROLL
         for (int d = 0; d < ND; ++d) {
@@ -273,11 +272,8 @@ RCPG_UNROLL
                 const double dist = xabs(dxw);
                 if (dist < r) {
                     const double F_mag = xmul(-2.0, xsub(xdiv(r, dist), 1.0));
-                    U = xadd(U, xmul(2.0, xsub(1.0, xdiv(dist, r))));
-                    ++count;
                     fi[d] = xadd(fi[d], xmul(F_mag, dxw));
-                    dk = xadd(dk, xmul(xmul(2.0, r), xsub(dist, r)));
-                    Fm = xadd(Fm, F_mag);
+                    sink(xmul(2.0, xsub(1.0, xdiv(dist, r))), xmul(xmul(2.0, r), xsub(dist, r)), F_mag);
                 }
             }
         }
@@ -308,15 +304,24 @@ RCPG_UNROLL
             }
             dij = xsqrt(dij);
             const double F_mag = xmul(-2.0, xabs(xsub(xdiv(r, dij), 1.0)));
-            U = xadd(U, xsub(1.0, xdiv(dij, r)));
-            ++count;
             RCPG_UNROLL
             for (int M = 0; M < ND; ++M)
                 if (M < tk) fi[M] = xadd(fi[M], xmul(F_mag, dxc[M]));
-            dk = xadd(dk, xmul(xmul(2.0, r), xsub(dij, r)));
-            Fm = xadd(Fm, F_mag);
+            sink(xsub(1.0, xdiv(dij, r)), xmul(xmul(2.0, r), xsub(dij, r)), F_mag);
         }
     }
+}
+
+// The same with the terms added to the three wall_* sums.
+template <int ND, typename CountT>
+RCPG_HD void wall_forces(const double* xi, double Di, const Geometry& g, double* fi,
+                         double& U, double& dk, double& Fm, CountT& count) {
+    wall_terms<ND>(xi, Di, g, fi, [&](double u, double k, double f) {
+        U = xadd(U, u);
+        dk = xadd(dk, k);
+        Fm = xadd(Fm, f);
+        ++count;
+    });
 }
 
 // |F_i|^2 in the reference's order (ENG:787-791).

@@ -2191,51 +2191,189 @@ __global__ void __launch_bounds__(kForceBlock, EXACT ? 1 : ((MIXED && ND == 2) ?
 // Sums in the one-thread order of the reference: all pair terms row after
 // row, then the wall terms particle after particle (ENG:4086-4257), the
 // diameter sum and the force-magnitude sum in index order (ENG:4262, :785).
+//
+// The six sums are six serial chains, independent of one another, and an FP64
+// addition waits for the one before it; what a single thread lost on top was
+// the latency of every load. Here 256 producer threads bring the terms of a
+// tile of 256 particles, compacted in order, into one half of a double buffer
+// in shared memory while six threads in warps of their own each add one chain
+// from the other half. Bound by the chains: the longest one (overlapping pairs
+// + wall contacts) times the latency of an FP64 addition. Exact run of 96 steps,
+// 3-D N = 2,000, on one B200: 129.6 -> 14.6 ms (1.3 ms of a step were this
+// reduction).
+constexpr int kRedTile = 256;     // particles per tile, one per producer thread
+constexpr int kRedCap = 1024;     // terms per buffer (a tile with more takes several)
+constexpr int kRedThreads = kRedTile + 6 * 32;
+
+struct ExactBuffer {
+    double U[kRedCap], Lc[kRedCap], dk[kRedCap], Fm[kRedCap];  // pair or wall terms in order
+    double D[kRedTile], mag[kRedTile];                         // per particle (0 where not counted)
+    std::uint32_t terms, particles;
+};
+
+// s += v[0] + v[1] + ..., one after the other
+__device__ __forceinline__ double chain_add(double s, const double* v, std::uint32_t n) {
+    std::uint32_t k = 0;
+    for (; k + 8 <= n; k += 8) {
+        double w[8];
+        RCPG_UNROLL
+        for (int u = 0; u < 8; ++u) w[u] = v[k + u];
+        RCPG_UNROLL
+        for (int u = 0; u < 8; ++u) s = xadd(s, w[u]);
+    }
+    for (; k < n; ++k) s = xadd(s, v[k]);
+    return s;
+}
+
 template <int ND>
-__global__ void k_reduce_exact(DevArrays a) {
+__global__ void __launch_bounds__(kRedThreads) k_reduce_exact(DevArrays a) {
     DevCtl* ctl = a.ctl;
     if (ctl_idle(ctl)) return;
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    extern __shared__ __align__(16) unsigned char red_smem[];
+    ExactBuffer* const buf = reinterpret_cast<ExactBuffer*>(red_smem);  // [2]
+    __shared__ std::uint32_t s_scan[kRedTile / 32];
+    __shared__ double s_max[kRedTile / 32], s_sum[6];
+    __shared__ std::uint32_t s_nmag[kRedTile / 32];
+    __shared__ unsigned long long s_count[2];
     const std::uint64_t N = a.N;
-    ForceSums s;
-    sums_zero(s);
-    for (std::uint64_t i = 0; i < N; ++i) {
-        const std::uint32_t n = a.pterm_cnt[i];
-        for (std::uint32_t k = 0; k < n; ++k) {
-            const PairTerms pt = a.pterm[static_cast<std::uint64_t>(k) * N + i];
-            s.pair_U = xadd(s.pair_U, pt.U);
-            s.pair_count += 1ull;
-            s.pair_Lc = xadd(s.pair_Lc, pt.Lc);
-            if (pt.U > s.pair_maxov) s.pair_maxov = pt.U;
-            s.pair_dk = xadd(s.pair_dk, pt.dk);
-            s.pair_Fm = xadd(s.pair_Fm, pt.Fm);
-        }
-    }
     const Geometry g = ctl->g;  // register copy: the loops below store through other pointers
     const double kap = ctl->force_kappa;
-    for (std::uint64_t i = 0; i < N; ++i) {
-        double xi[ND], D0i, fdummy[ND];
-        load_pos<ND>(a.pos, i, xi, D0i);
-#pragma unroll
-        for (int d = 0; d < ND; ++d) fdummy[d] = 0.0;
-        // wall terms continue the pair chains, as in the reference
-        wall_forces<ND>(xi, xmul(D0i, kap), g, fdummy, s.pair_U, s.pair_dk, s.pair_Fm, s.wall_count);
-    }
-    for (std::uint64_t i = 0; i < N; ++i) {
-        double xi[ND], D0i;
-        load_pos<ND>(a.pos, i, xi, D0i);
-        s.sum_D = xadd(s.sum_D, xmul(D0i, kap));
-    }
-    std::uint32_t mc = 0;
-    for (std::uint64_t i = 0; i < N; ++i) {
-        const double f2 = force_norm2<ND>(a.F + i * ND);
-        if (f2 > 1.0E-16) {
-            s.sum_mag = xadd(s.sum_mag, xsqrt(f2));
-            ++mc;
+    const bool walls = g.any_flat_wall || g.circle_k > 0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool producer = tid < kRedTile;
+    const int chain = (!producer && lane == 0) ? warp - kRedTile / 32 : -1;  // 0..5: U, Lc, dk, Fm, D, mag
+    double sum = 0.0, maxov = 0.0;
+    unsigned long long count[2] = {0ull, 0ull};  // terms added per phase
+    std::uint32_t nmag = 0, turn = 0;
+    // phase 0: pair terms (and the per-particle terms); phase 1: wall terms
+    for (int phase = 0; phase < (walls ? 2 : 1); ++phase) {
+        for (std::uint64_t i0 = 0; i0 < N; i0 += kRedTile) {
+            const std::uint64_t i = i0 + static_cast<std::uint64_t>(tid);
+            std::uint32_t n = 0, off = 0, total = 0;
+            double xi[ND], D0i = 0.0, fdummy[ND];
+            if (producer) {
+                if (i < N) {
+                    load_pos<ND>(a.pos, i, xi, D0i);
+                    if (phase == 0) {
+                        n = a.pterm_cnt[i];
+                    } else {
+                        RCPG_UNROLL
+                        for (int d = 0; d < ND; ++d) fdummy[d] = 0.0;
+                        wall_terms<ND>(xi, xmul(D0i, kap), g, fdummy, [&](double, double, double) { ++n; });
+                    }
+                }
+                // exclusive scan of the term counts over the producers
+                std::uint32_t incl = n;
+                RCPG_UNROLL
+                for (int o = 1; o < 32; o <<= 1) {
+                    const std::uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                if (lane == 31) s_scan[warp] = incl;
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                std::uint32_t before = 0;
+                RCPG_UNROLL
+                for (int w = 0; w < kRedTile / 32; ++w) {
+                    const std::uint32_t v = s_scan[w];
+                    before += w < warp ? v : 0u;
+                    total += v;
+                }
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                off = before + incl - n;
+            }
+            // the tile's terms kRedCap at a time; one barrier per buffer
+            // handed over (producers and chains agree on the number of turns
+            // through the buffer itself: terms | more << 31)
+            for (std::uint32_t w0 = 0;; w0 += kRedCap) {
+                ExactBuffer& b = buf[turn & 1u];
+                bool more = false;
+                if (producer) {
+                    more = total > w0 + kRedCap;
+                    if (phase == 0) {
+                        for (std::uint32_t k = off < w0 ? w0 - off : 0u; k < n && off + k < w0 + kRedCap; ++k) {
+                            const PairTerms pt = a.pterm[static_cast<std::uint64_t>(k) * N + i];
+                            const std::uint32_t p = off + k - w0;
+                            b.U[p] = pt.U;
+                            b.Lc[p] = pt.Lc;
+                            b.dk[p] = pt.dk;
+                            b.Fm[p] = pt.Fm;
+                            if (pt.U > maxov) maxov = pt.U;
+                        }
+                        if (w0 == 0 && i < N) {
+                            b.D[tid] = xmul(D0i, kap);
+                            const double f2 = force_norm2<ND>(a.F + i * ND);
+                            const bool counted = f2 > 1.0E-16;
+                            b.mag[tid] = counted ? xsqrt(f2) : 0.0;
+                            nmag += counted;
+                        }
+                    } else if (n) {
+                        std::uint32_t p = off;
+                        wall_terms<ND>(xi, xmul(D0i, kap), g, fdummy, [&](double u, double k, double f) {
+                            if (p >= w0 && p < w0 + kRedCap) {
+                                b.U[p - w0] = u;
+                                b.dk[p - w0] = k;
+                                b.Fm[p - w0] = f;
+                            }
+                            ++p;
+                        });
+                    }
+                    if (tid == 0) {
+                        const std::uint32_t here = total - w0 < static_cast<std::uint32_t>(kRedCap) ? total - w0 : kRedCap;
+                        b.terms = here | (more ? 0x80000000u : 0u);
+                        b.particles = (phase == 0 && w0 == 0) ? static_cast<std::uint32_t>(N - i0 < kRedTile ? N - i0 : kRedTile) : 0u;
+                    }
+                }
+                __syncthreads();  // the buffer is full, and the other one has been added
+                ++turn;
+                if (!producer) {
+                    const std::uint32_t t = b.terms & 0x7fffffffu;
+                    more = (b.terms >> 31) != 0u;
+                    count[0] += phase == 0 ? t : 0u;
+                    count[1] += phase == 0 ? 0u : t;
+                    if (chain == 0) sum = chain_add(sum, b.U, t);
+                    else if (chain == 1) sum = phase == 0 ? chain_add(sum, b.Lc, t) : sum;
+                    else if (chain == 2) sum = chain_add(sum, b.dk, t);
+                    else if (chain == 3) sum = chain_add(sum, b.Fm, t);
+                    else if (chain == 4) sum = chain_add(sum, b.D, b.particles);
+                    else if (chain == 5) sum = chain_add(sum, b.mag, b.particles);
+                }
+                if (!more) break;
+            }
         }
     }
-    s.mag_count = mc;
-    ctl->sums = s;
+    // the totals
+    RCPG_UNROLL
+    for (int o = 16; o > 0; o >>= 1) {
+        maxov = fmax(maxov, __shfl_down_sync(0xffffffffu, maxov, o));
+        nmag += __shfl_down_sync(0xffffffffu, nmag, o);
+    }
+    if (producer && lane == 0) {
+        s_max[warp] = maxov;
+        s_nmag[warp] = nmag;
+    }
+    if (chain == 0) {
+        s_count[0] = count[0];
+        s_count[1] = count[1];
+    }
+    if (chain >= 0) s_sum[chain] = sum;
+    __syncthreads();
+    if (tid == 0) {
+        ForceSums s;
+        sums_zero(s);
+        for (int w = 0; w < kRedTile / 32; ++w) {
+            s.pair_maxov = fmax(s.pair_maxov, s_max[w]);
+            s.mag_count += s_nmag[w];
+        }
+        s.pair_U = s_sum[0];  // the wall terms continue the pair chains, as in the reference
+        s.pair_Lc = s_sum[1];
+        s.pair_dk = s_sum[2];
+        s.pair_Fm = s_sum[3];
+        s.sum_D = s_sum[4];
+        s.sum_mag = s_sum[5];
+        s.pair_count = s_count[0];
+        s.wall_count = s_count[1];
+        ctl->sums = s;
+    }
 }
 
 // Fixed-order reduction of the per-block partial sums by one block.
@@ -2911,8 +3049,15 @@ void launch_step_gate(const DevArrays& a, unsigned long long cond_build, cudaStr
     k_step_gate<<<1, 1, 0, st>>>(a, cond_build);
 }
 
+template <int ND>
+void reduce_exact_nd(const DevArrays& a, cudaStream_t st) {
+    constexpr int smem = static_cast<int>(2 * sizeof(ExactBuffer));
+    cudaFuncSetAttribute(k_reduce_exact<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    k_reduce_exact<ND><<<1, kRedThreads, smem, st>>>(a);
+}
+
 void launch_reduce_exact(const DevArrays& a, cudaStream_t st) {
-    RCPG_DISPATCH_ND(a.ndim, (k_reduce_exact<ND><<<1, 1, 0, st>>>(a)));
+    RCPG_DISPATCH_ND(a.ndim, (reduce_exact_nd<ND>(a, st)));
 }
 
 // max |ref| and max |cmp - ref| (mixed-precision error report): a

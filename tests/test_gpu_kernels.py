@@ -125,3 +125,24 @@ def test_pairs_row_capacity_overflow_reports_need(cuda_device, golden):
                                G.hp(np.ascontiguousarray(g["walls"]), C.POINTER(C.c_int8)), 0.5 * float(g["D"].max()),
                                4, G.vp(nbr), G.vp(cnt), C.byref(need), None, err, len(err))
     assert rc == N.RCPG_ENOSPC and need.value > 4
+
+
+# particles around the reduction's tile (256), with more overlapping pairs per tile than one of its
+# buffers holds (phi 3: about 12 pairs per particle), between hard walls and in a container
+@pytest.mark.parametrize("n,nd,walls", [(2, 2, [0, 0]), (255, 2, [1, 1]), (256, 2, [0, 0]), (257, 2, [1, 0]),
+                                        (1025, 2, [1, 1]), (700, 3, [-3, 0, 0])])
+def test_exact_order_sums_of_dense_states_against_oracle(cuda_device, oracle, native, n, nd, walls):
+    from tests import gpu_util as G
+    rng = np.random.default_rng(n)
+    x = rng.random((n, nd))
+    D = rng.uniform(0.8, 1.2, n)
+    D *= (3.0 / ((np.pi / 4 if nd == 2 else np.pi / 6) * D ** nd).sum()) ** (1.0 / nd)
+    D = np.minimum(D, 0.4)
+    box = np.ones(nd)
+    t = oracle.t_shell(D)
+    counts, ids = oracle.pairs_full(x, D, box, t)
+    F, sc = oracle.forces(x, D, box, np.asarray(walls, np.int8), counts, ids, 2.5e-4)
+    nbr, cnt, cap = G.pairs_full(x, D, box, walls, t)
+    F2, sc2 = G.forces(x, D, box, walls, nbr, cnt, cap, 2.5e-4, 1)
+    assert np.array_equal(F2, F)
+    assert np.array_equal(sc2[:5], sc[:5])
