@@ -160,18 +160,22 @@ RCPG_UNROLL
     return d2;
 }
 
-// Force and scalar terms of an overlapping pair (d2 < r_ij^2) from its
-// displacement, FP64 as in the reference (ENG:4105-4139).
-template <int ND>
-RCPG_HD void pair_terms_f64(const double* dx, double d2, double r_ij, double* fi, PairTerms& pt) {
+// Scalar terms of an overlapping pair (d2 < r_ij^2), FP64 as in the reference
+// (ENG:4105-4139).
+RCPG_HD void pair_scalars_f64(double d2, double r_ij, PairTerms& pt) {
     const double dist = xsqrt(d2);
-    const double F_mag = -xsub(xdiv(r_ij, dist), 1.0);
-RCPG_UNROLL
-    for (int d = 0; d < ND; ++d) fi[d] = xadd(fi[d], xmul(F_mag, dx[d]));
+    pt.Fm = -xsub(xdiv(r_ij, dist), 1.0);
     pt.U = xsub(1.0, xdiv(dist, r_ij));
     pt.Lc = r_ij;
     pt.dk = xmul(r_ij, xsub(dist, r_ij));
-    pt.Fm = F_mag;
+}
+
+// The same, and the pair's force added to fi.
+template <int ND>
+RCPG_HD void pair_terms_f64(const double* dx, double d2, double r_ij, double* fi, PairTerms& pt) {
+    pair_scalars_f64(d2, r_ij, pt);
+RCPG_UNROLL
+    for (int d = 0; d < ND; ++d) fi[d] = xadd(fi[d], xmul(pt.Fm, dx[d]));
 }
 
 #if defined(__CUDACC__)
@@ -216,6 +220,12 @@ RCPG_UNROLL
 struct PairTermsF {
     float U, Lc, dk, Fm;
 };
+
+// dist - r of an overlapping pair. Where a kernel adds the dkappa term r (dist
+// - r) to an FP32 sum, the product and the sum are one fused multiply-add.
+__device__ __forceinline__ float mixed_gap(float d2, float rsum) {
+    return __fsub_rn(__fmul_rn(d2, rsqrtf(d2)), rsum);
+}
 
 template <int ND>
 __device__ __forceinline__ void pair_terms_mixed_f(const float* dxf, float d2, float rsum, float* fi,

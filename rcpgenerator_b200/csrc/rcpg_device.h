@@ -215,6 +215,11 @@ void launch_diff_max(const double* ref, const double* cmp, std::uint64_t n, unsi
                      cudaStream_t st);
 void launch_controller(const DevArrays& a, int open_only, cudaStream_t st);
 void launch_reorder(const DevArrays& a, cudaStream_t st);
+// Up to `steps` steps of a small packing in one launch (rcpg_small.cu), from
+// the same state and to the same state as the step graph; small_steps_ok: the
+// packing and its cell grid are small enough.
+bool small_steps_ok(const DevArrays& a);
+void launch_small_steps(const DevArrays& a, std::uint32_t steps, cudaStream_t st);
 void launch_fix_height(const DevArrays& a, cudaStream_t st);
 
 void launch_pack(std::uint64_t N, int ndim, const double* x, const double* D, double* pos,
@@ -232,19 +237,30 @@ void launch_rows_to_particle_order(std::uint64_t N, const std::uint32_t* work, c
                                    const std::uint32_t* src_cnt, std::uint32_t* dst,
                                    std::uint32_t* dst_cnt, cudaStream_t st);
 
-// Host-side finalisation shared with the controller kernel (ENG:4259-4268, :769-803).
-RCPG_HD StepScalars finalize_sums(const ForceSums& s, double mu_eff, int ndim) {
-    StepScalars r;
-    const double count = static_cast<double>(1ull + s.pair_count + s.wall_count);
+// Finalisation shared by the host and the controllers (ENG:4259-4268, :769-803),
+// in two parts: what the schedule depends on, and what is only reported.
+RCPG_HD double contact_count(const ForceSums& s) { return static_cast<double>(1ull + s.pair_count + s.wall_count); }
+
+RCPG_HD void finalize_schedule(const ForceSums& s, double mu_eff, StepScalars& r) {
+    r.max_overlap = s.pair_maxov;
+    r.dkappa = xadd(xadd(s.pair_dk, s.wall_dk), xmul(mu_eff, s.sum_D));
+}
+
+RCPG_HD void finalize_report(const ForceSums& s, int ndim, StepScalars& r) {
+    const double count = contact_count(s);
     const double U_tot = xadd(s.pair_U, s.wall_U);
     r.U = pow(xdiv(U_tot, count), 2.0);
-    r.max_overlap = s.pair_maxov;
     r.Lc = xdiv(s.pair_Lc, count);
-    r.dkappa = xadd(xadd(s.pair_dk, s.wall_dk), xmul(mu_eff, s.sum_D));
     r.Fmean = xdiv(-xadd(s.pair_Fm, s.wall_Fm), count);
     const double mean_mag = xdiv(s.sum_mag, static_cast<double>(static_cast<std::uint32_t>(s.mag_count)));
     r.mean_force = xdiv(mean_mag, xsqrt(static_cast<double>(ndim)));
     r.count = count;
+}
+
+RCPG_HD StepScalars finalize_sums(const ForceSums& s, double mu_eff, int ndim) {
+    StepScalars r;
+    finalize_schedule(s, mu_eff, r);
+    finalize_report(s, ndim, r);
     return r;
 }
 

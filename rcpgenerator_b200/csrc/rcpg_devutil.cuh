@@ -179,8 +179,10 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T* smem, T& total) {
 __device__ __forceinline__ void publish_step(DevCtl* ctl, const Controller& c, int ndim) {
     ctl->forces_done = 0u;
     for (int d = 0; d < ndim; ++d) {
-        ctl->g.box[d] = c.box[d];
-        ctl->g.inv_box[d] = 1.0 / c.box[d];
+        if (ctl->g.box[d] != c.box[d]) {  // fix_height only: a division saved in every other step
+            ctl->g.box[d] = c.box[d];
+            ctl->g.inv_box[d] = 1.0 / c.box[d];
+        }
     }
     ctl->refresh_kappa = c.kappa_D;
     ctl->force_kappa = c.kappa_D;

@@ -852,6 +852,10 @@ void Engine::after_stop() {
     }
 }
 
+namespace {
+constexpr std::uint64_t kSmallSlice = 512;  // steps per launch of the small-packing kernel
+}
+
 bool Engine::advance_graph(std::uint64_t max_new_steps) {
     Controller& c = host_c_;
     const std::uint64_t start = c.hist_filled;
@@ -882,10 +886,17 @@ bool Engine::advance_graph(std::uint64_t max_new_steps) {
         const std::uint64_t done_steps = c.hist_filled - start;
         if (max_new_steps && done_steps >= max_new_steps) break;
         const std::uint64_t want = max_new_steps ? max_new_steps - done_steps : ~0ull;
-        if (!graph_exec_) capture_graph();
+        const bool small = small_steps_ok(a_);
+        if (!small && !graph_exec_) capture_graph();
         const std::uint64_t b0 = hctl_.nbuilds, f0 = hctl_.pair_kernel_runs;
         bool replay = false;
-        if (want >= static_cast<std::uint64_t>(graph_steps_)) {
+        if (small) {
+            // the steps of a small packing as one cluster kernel, short enough
+            // (a few ms) that other engines' work interleaves
+            launch_small_steps(a_, static_cast<std::uint32_t>(std::min<std::uint64_t>(want, kSmallSlice)), st_);
+            check(cudaGetLastError(), "small steps");
+            ++launches_;
+        } else if (want >= static_cast<std::uint64_t>(graph_steps_)) {
             check(cudaGraphLaunch(graph_exec_, st_), "graph launch");
             replay = true;
         } else {

@@ -154,11 +154,25 @@ struct HistStats {
     double f_3000_2500;    // hist_mean(h.force, step - 3000, step - 2500)
 };
 
+// Parts of the schedule that are known before a step's forces: the powers of
+// the bias corrections at the current counter t, and for the step that
+// begin_step() opens next the growth rung's boost factor and the phi of 250
+// steps before. A controller that waits for the forces may compute them
+// meanwhile (the same functions of the same arguments).
+struct StepPre {
+    double pb1, pb2;        // 0.9^t, 0.999^t
+    double inv_b1, inv_b2;  // 1 / (1 - pb1), 1 / (1 - pb2)
+    double boost;           // exp(-step / 350)
+    double phi_250;         // h.phi[step - 250]; only for step > 251
+};
+
 // ---- top of step (ENG:5520-6042) ------------------------------------------
 // Everything the reference does before its pair refresh, except the two
 // particle-wide actions it requests through flags: reorder and lock_now.
-// `pre` (optional) holds the history window statistics of this step.
-RCPG_HD void begin_step(Controller& c, const Histories& h, std::uint64_t step, const HistStats* pre = nullptr) {
+// `pre` (optional) holds the history window statistics of this step, `ahead`
+// (optional) the parts computed before the previous step's forces.
+RCPG_HD void begin_step(Controller& c, const Histories& h, std::uint64_t step, const HistStats* pre = nullptr,
+                        const StepPre* ahead = nullptr) {
     const std::uint64_t cooldown = 250;
     const double flat = 5e-3, decay = 0.85;
     c.steps = step;
@@ -251,11 +265,12 @@ RCPG_HD void begin_step(Controller& c, const Histories& h, std::uint64_t step, c
     // learning rate (ENG:5665-5721)
     {
         const std::uint64_t s250 = (step > 251) ? step - 250 : 1;  // max(step-250, 1)
-        if ((step - c.last_alpha_update > 500) && (xsub(c.phi, h.phi[s250]) < 5e-4) &&
+        const bool known = ahead && step > 251;
+        if ((step - c.last_alpha_update > 500) && (xsub(c.phi, known ? ahead->phi_250 : h.phi[s250]) < 5e-4) &&
             (step > 2500) && static_cast<double>(step) > xadd(c.mu_change, 500.0)) {
             double trend1 = pre ? xdiv(pre->f_450_250, pre->f_75_1)
                                 : xdiv(hist_mean(h.force, step - 450, step - 250), hist_mean(h.force, step - 75, step - 1));
-            const double trend2 = xsub(c.phi, h.phi[s250]);
+            const double trend2 = xsub(c.phi, known ? ahead->phi_250 : h.phi[s250]);
             if ((c.mu_flag < 1 && trend1 < 0.85) || trend2 < -5E-4) {
                 c.last_alpha_update = step;
                 c.alpha = xdiv(c.alpha, 1.5);
@@ -329,7 +344,7 @@ RCPG_HD void begin_step(Controller& c, const Histories& h, std::uint64_t step, c
     }
     c.theta = xmul(xmul(c.Dmin, 0.25), ts);
     c.mu_eff = (c.mu_flag == 1)
-                   ? xmul(c.mu, xadd(1.0, xmul(4.0, exp(xdiv(-static_cast<double>(step), 350.0)))))
+                   ? xmul(c.mu, xadd(1.0, xmul(4.0, ahead ? ahead->boost : exp(xdiv(-static_cast<double>(step), 350.0)))))
                    : c.mu;
     const double Dmin_cur = xmul(c.D0_min, kap);
     const double Dmed_cur = xmul(c.D0_med, kap);
@@ -380,12 +395,19 @@ RCPG_HD void finish_lock(Controller& c, const Histories& h, std::uint64_t step, 
 }
 
 // ---- end of step (ENG:6249-6577) ------------------------------------------
-RCPG_HD void end_step(Controller& c, const Histories& h, const StepScalars& s) {
-    const std::uint64_t step = c.steps;
+// With `ahead` the powers are taken from it and the energy and the force
+// magnitude are left to end_step_report(), which no later step depends on.
+RCPG_HD void end_step_report(Controller& c, const Histories& h, const StepScalars& s) {
     c.U = s.U;
-    c.max_min_dist = s.max_overlap;
+    h.energy[c.steps - 1] = c.U;
     c.F_magnitude = xdiv(s.mean_force, s.Fmean);
-    h.force[step - 1] = c.F_magnitude;
+    h.force[c.steps - 1] = c.F_magnitude;
+}
+
+RCPG_HD void end_step(Controller& c, const Histories& h, const StepScalars& s, const StepPre* ahead = nullptr) {
+    const std::uint64_t step = c.steps;
+    c.max_min_dist = s.max_overlap;
+    if (!ahead) end_step_report(c, h, s);
     h.max_overlap[step - 1] = c.max_min_dist;
     h.mu[step - 1] = c.mu;
     h.alpha[step - 1] = c.alpha;
@@ -394,16 +416,15 @@ RCPG_HD void end_step(Controller& c, const Histories& h, const StepScalars& s) {
     const double dk = s.dkappa;
     c.m_kappa = xsub(xmul(0.9, c.m_kappa), xmul(xsub(1.0, 0.9), dk));
     c.v_kappa = xadd(xmul(0.999, c.v_kappa), xmul(xsub(1.0, 0.999), xmul(dk, dk)));
-    const double pb1 = pow(0.9, c.t);
-    const double pb2 = pow(0.999, c.t);
+    const double pb1 = ahead ? ahead->pb1 : pow(0.9, c.t);
+    const double pb2 = ahead ? ahead->pb2 : pow(0.999, c.t);
     c.m_hat_kappa = xdiv(c.m_kappa, xsub(1.0, pb1));
     c.v_hat_kappa = xdiv(c.v_kappa, xsub(1.0, pb2));
     if (!c.runtime_fix_diameter)
         c.kappa = xsub(c.kappa, xdiv(xmul(c.alpha, c.m_hat_kappa), xadd(xsqrt(c.v_hat_kappa), 1e-8)));
     c.adam_alpha = c.alpha;
-    c.inv_b1 = xdiv(1.0, xsub(1.0, pb1));
-    c.inv_b2 = xdiv(1.0, xsub(1.0, pb2));
-    h.energy[step - 1] = c.U;
+    c.inv_b1 = ahead ? ahead->inv_b1 : xdiv(1.0, xsub(1.0, pb1));
+    c.inv_b2 = ahead ? ahead->inv_b2 : xdiv(1.0, xsub(1.0, pb2));
     c.hist_filled = step;
 }
 
