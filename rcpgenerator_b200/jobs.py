@@ -79,13 +79,13 @@ def overlap_report(packing, frac_def="sum", verbose=False, device: int = 0):
         box = np.ascontiguousarray(box, dtype=np.float64)
         boxp = box.ctypes.data_as(N._dp)
     ncand, nov = C.c_uint64(0), C.c_uint64(0)
-    cap = 0
-    pairs = np.zeros((0, 2), np.uint32)
-    fs = fm = np.zeros(0)
-    for _ in range(2):  # first call sizes the output
-        pairs = np.zeros((max(cap, 1), 2), np.uint32)
-        fs = np.zeros(max(cap, 1))
-        fm = np.zeros(max(cap, 1))
+    # room for a jammed packing's contacts (2 d pairs of neighbours, d per particle) and as many rattling
+    # overlaps; a state with more is reported by a second call with the exact size
+    cap = 2 * ndim * n
+    for _ in range(2):
+        pairs = np.empty((max(cap, 1), 2), np.uint32)
+        fs = np.empty(max(cap, 1))
+        fm = np.empty(max(cap, 1))
         err = N.errbuf()
         rc = N.lib.rcpg_overlap_report(n, ndim, pos.ctypes.data_as(N._dp), D.ctypes.data_as(N._dp), boxp,
                                        C.byref(ncand), C.byref(nov), cap,

@@ -122,3 +122,11 @@ def test_run_jobs_default_split_meets_the_gate(cuda_device):
     for r in rows[:-1]:
         assert 0.0 < r["max_overlap"] < 5e-4
         assert 0.5 < r["phi"] < 0.9
+
+
+# around a tile of the scans (2,048) and over several, more cells than particles, and more overlaps than
+# the first call has room for
+@pytest.mark.parametrize("n,nd,dmax,periodic", [(2047, 2, 0.03, True), (2049, 3, 0.06, False), (5000, 2, 0.004, True),
+                                               (4500, 3, 0.05, True), (300, 2, 0.5, True)])
+def test_overlap_report_matches_oracle_across_scan_tiles(cuda_device, n, nd, dmax, periodic):
+    test_overlap_report_matches_oracle(cuda_device, n, nd, dmax, periodic)
