@@ -2357,14 +2357,16 @@ void launch_warp_search(const DevArrays& a, cudaStream_t st) {
 
 // Lanes per particle of k_build_rows (the smallest size class): one once the
 // packing alone fills the GPU, more below that. Measured per build on one
-// B200: 3-D log-normal N = 50,003 65 us (1 lane) against 113 (4); N = 8,000 28
-// us (8) against 43 (4) and 37 (32); N = 2,000 11 us (32) against 15 (8). In
-// 4-D a particle has ten times the candidates: N = 30,000 208 us (8) against
-// 251 (4) and 214 (32), N = 12,001 128 us (32) against 151 (8).
+// B200: 3-D log-normal N = 50,003 85 us (1 lane) against 91 (2); N = 12,000 31
+// us (4) against 40 (2), 38 (8) and 46 (16). In 4-D a particle has ten times
+// the candidates and more as it grows: log-normal N = 12,001 over 240 steps 126
+// us (16) against 124 (4, but 155 at the end against 138) and 136 (8); N =
+// 30,000 182 us (8) against 193 (16). Below 8,192 particles only the first build of a run and those
+// after a spatial reorder come here.
 template <int ND>
 int search_lanes(std::uint64_t N) {
-    if (ND <= 3) return N >= 32768 ? 1 : (N >= 4096 ? 8 : 32);
-    return N >= 20000 ? 8 : 32;
+    if (ND <= 3) return N >= 32768 ? 1 : (N >= 4096 ? 4 : 32);
+    return N >= 20000 ? 8 : 16;
 }
 
 template <int ND>

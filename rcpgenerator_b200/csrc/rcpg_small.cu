@@ -22,8 +22,8 @@
 // Bound by latency: two barriers, the chain partner index -> record -> square
 // root -> division of the longest row, and the controller's serial divisions;
 // what is known earlier (bias corrections, boost) is computed beside them.
-// Whole calls on one B200, set-up included: N = 64 2-D, 3,000 steps 118.9 ->
-// 27.5 ms; N = 2,000 3-D, 1,500 steps of which 1,150 rebuild 113.0 -> 58.5 ms;
+// Whole calls on one B200, set-up included: N = 64 2-D, 3,000 steps 131 -> 28.8
+// ms; N = 2,000 3-D, 1,500 steps of which 1,150 rebuild 118.6 -> 50.7 ms;
 // a batch of 96 packings of up to 4,096 particles (400 steps) 1,284 -> 459 ms.
 //
 // Work is dealt out by warps of 32 consecutive particles: warp w of the
@@ -49,6 +49,8 @@ constexpr int kSmallThreads = 512;
 constexpr int kSmallWarps = kSmallThreads / 32;
 constexpr int kSmallBlocks = 16;                                  // most blocks of the cluster
 constexpr int kSmallN = kSmallBlocks * kSmallThreads;             // 8,192 particles
+constexpr int kSmallUnits = kSmallN / 32;                         // warps of particles
+constexpr int kSmallSums = 9;                                     // sums per warp of particles
 constexpr std::uint32_t kSmallCells = 12288;                      // cell offsets held in shared memory
 
 // per pair: the force (up to 8 components), U, Lc, dk, Fm
@@ -56,14 +58,14 @@ constexpr int kTermFields = kMaxDim + 4;
 
 struct SmallShared {
     DevCtl ctl;                               // this block's copy of the control block
-    ForceSums warp_sums[kSmallWarps];         // of this block's warps of particles (read by the other blocks)
     ForceSums total;
     StepPre ahead;                            // for the step being computed
     double hred[(kCtlThreads / 32) * 6];
     HistStats stats;
     std::uint32_t trigger[2];                 // some particle asks for a build (written by any block)
     std::uint32_t scan[kSmallWarps];
-    int go;
+    std::uint32_t row_need, cap_error;        // as the last build left them
+    int go, have_stats;
     // pair terms of a round (one column per lane), then each particle's sums
     double terms[kSmallWarps][kTermFields][33];
     double maxov[kSmallWarps][32];
@@ -91,6 +93,10 @@ __device__ void scan_cells(const std::uint32_t* count, std::uint32_t n, SmallSha
             run += v;
         }
     __syncthreads();
+}
+
+__device__ __forceinline__ unsigned long long bits_of(double v) {
+    return static_cast<unsigned long long>(__double_as_longlong(v));
 }
 
 // StepPre of the step that is open now, each part by another warp (one lane).
@@ -150,15 +156,22 @@ __device__ __forceinline__ void pair_sums(const DevArrays& b, const DevCtl* ctl,
         return k < n ? b.nbr[static_cast<std::uint64_t>(k) * N + t] : 0xffffffffu;
     };
     const std::uint32_t most = __reduce_max_sync(0xffffffffu, n);
-    std::uint32_t next = row_id(s);
+    // the next round's record and the row id after it are on their way while a round computes
+    double xn[ND], D0n = 0.0;
+    std::uint32_t jn = row_id(s), jnn = row_id(lanes + s);
+    RCPG_UNROLL
+    for (int d = 0; d < ND; ++d) xn[d] = xi[d];
+    if (jn < N) load_pos<ND>(b.pos, jn, xn, D0n);
     for (std::uint32_t k0 = 0; k0 < most; k0 += lanes) {
-        const std::uint32_t j = next;
+        const std::uint32_t j = jn;
         const bool in = j < N;
-        next = row_id(k0 + lanes + s);
-        double xj[ND], D0j = 0.0;
+        double xj[ND];
+        const double D0j = D0n;
         RCPG_UNROLL
-        for (int d = 0; d < ND; ++d) xj[d] = xi[d];
-        if (in) load_pos<ND>(b.pos, j, xj, D0j);
+        for (int d = 0; d < ND; ++d) xj[d] = xn[d];
+        jn = jnn;
+        jnn = row_id(k0 + 2 * lanes + s);
+        if (jn < N) load_pos<ND>(b.pos, jn, xn, D0n);
         T dx[ND], d2, r;
         if constexpr (MX) {
             d2 = mixed_disp<ND>(xi, xj, bx, hbf, dx);
@@ -255,13 +268,20 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
     const bool mine = unit < units && i < N;
     DevCtl* const g = a.ctl;
     DevCtl* const ctl = &sh.ctl;
+    // the warps' sums of a step, [sum][warp of the packing] (through L2: eight
+    // times as fast here as loads from the other blocks' shared memory)
+    unsigned long long* const sums = reinterpret_cast<unsigned long long*>(a.block_sums);
+    static_assert(kSmallSums * kSmallUnits * 8 <= 4096 * sizeof(ForceSums), "room in the block sums");
     static_assert(sizeof(DevCtl) % 8 == 0, "control block copied by 8-byte words");
     {
         const unsigned long long* src = reinterpret_cast<const unsigned long long*>(g);
         unsigned long long* dst = reinterpret_cast<unsigned long long*>(ctl);
         for (int w = tid; w < static_cast<int>(sizeof(DevCtl) / 8); w += kSmallThreads) dst[w] = src[w];
     }
-    if (tid == 0) sh.trigger[0] = sh.trigger[1] = 0u;
+    if (tid == 0) {
+        sh.trigger[0] = sh.trigger[1] = 0u;
+        sums_zero(sh.total);  // the wall terms join the pair sums: their own stay zero
+    }
     __syncthreads();
     if (lane == 0) prepare_ahead(ctl->c, a.hist, sh.ahead, warp);
     if (ctl->stopped | ctl->halted) return;  // the same in every block
@@ -421,30 +441,37 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
             }
             if (unit < units) {
                 warp_reduce_sums(s);
-                if (lane == 0) sh.warp_sums[warp] = s;
+                if (lane == 0) {
+                    unsigned long long* w = sums + unit;
+                    w[0 * kSmallUnits] = bits_of(s.pair_U);
+                    w[1 * kSmallUnits] = bits_of(s.pair_Lc);
+                    w[2 * kSmallUnits] = bits_of(s.pair_dk);
+                    w[3 * kSmallUnits] = bits_of(s.pair_Fm);
+                    w[4 * kSmallUnits] = bits_of(s.pair_maxov);
+                    w[5 * kSmallUnits] = bits_of(s.sum_mag);
+                    w[6 * kSmallUnits] = bits_of(s.sum_D);
+                    w[7 * kSmallUnits] = s.pair_count;
+                    w[8 * kSmallUnits] = s.mag_count;
+                }
             }
         }
         cluster.sync();
         // ---- controller (k_controller), in every block ----------------------
         {
-            std::uint32_t row_need = 0, cap_error = 0;
-            if (tid == 0 && build) {
-                row_need = *reinterpret_cast<volatile std::uint32_t*>(&g->row_need);
-                cap_error = *reinterpret_cast<volatile std::uint32_t*>(&g->cap_error);
+            if (tid == kSmallThreads - 1) {
+                sh.row_need = build ? *reinterpret_cast<volatile std::uint32_t*>(&g->row_need) : ctl->row_need;
+                sh.cap_error = build ? *reinterpret_cast<volatile std::uint32_t*>(&g->cap_error) : ctl->cap_error;
             }
             // one warp per sum: lane k takes the eight warps of the particles
             // 256 k .. 256 k + 255 in order, then the controller's tree over
             // the lanes (absent warps and blocks add zero)
-            if (warp < 10) {
-                auto field = [&](std::uint32_t u, int f) -> unsigned long long {
-                    const ForceSums* src = cluster.map_shared_rank(&sh.warp_sums[u / C], u % C);
-                    return reinterpret_cast<const unsigned long long*>(src)[f];
-                };
-                // sums 0..4 pair_U, Lc, dk, Fm, maxov; 8, 9 sum_mag, sum_D; 10, 12 pair_count, mag_count
-                const int f = warp < 5 ? warp : (warp < 7 ? warp + 3 : (warp == 7 ? 10 : 12));
+            if (warp < kSmallSums) {
                 unsigned long long w[8];
                 RCPG_UNROLL
-                for (std::uint32_t k = 0; k < 8; ++k) w[k] = 8u * lane + k < units ? field(8u * lane + k, f) : 0ull;
+                for (std::uint32_t k = 0; k < 8; ++k)
+                    w[k] = 8u * lane + k < units ? __ldcg(sums + warp * kSmallUnits + 8 * lane + k) : 0ull;
+                // members of ForceSums: pair_U, Lc, dk, Fm, maxov, sum_mag, sum_D, pair_count, mag_count
+                const int f = warp < 5 ? warp : (warp < 7 ? warp + 3 : (warp == 7 ? 10 : 12));
                 if (f >= 10) {
                     unsigned long long n = 0;
                     RCPG_UNROLL
@@ -468,9 +495,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
                     v = f == 4 ? v : xadd(v, 0.0);
                     if (lane == 0) reinterpret_cast<double*>(&sh.total)[f] = v;
                 }
-            } else if (warp == 10 && lane == 0) {
-                sh.total.wall_U = sh.total.wall_dk = sh.total.wall_Fm = 0.0;
-                sh.total.wall_count = 0ull;
             }
             __syncthreads();
             if (tid == 0) {
@@ -479,11 +503,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
                 ctl->sums = sh.total;
                 ctl->nsum_blocks = (units + 7) / 8;
                 ctl->pair_kernel_runs += 1ull;
-                if (build) {
-                    ctl->row_need = row_need;
-                    ctl->cap_error = cap_error;
-                }
-                if (ctl->row_need > a.S || ctl->cap_error) {
+                ctl->row_need = sh.row_need;
+                ctl->cap_error = sh.cap_error;
+                if (sh.row_need > a.S || sh.cap_error) {
                     ctl->halted = 1u;
                     ctl->adam_go = 0u;
                     go = false;
@@ -510,9 +532,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
                 sh.go = go ? 1 : 0;
             } else if (tid == 32) {
                 // what is only reported (not after a halt, whose step is redone)
-                const std::uint32_t need = build ? *reinterpret_cast<volatile std::uint32_t*>(&g->row_need) : ctl->row_need;
-                const std::uint32_t err = build ? *reinterpret_cast<volatile std::uint32_t*>(&g->cap_error) : ctl->cap_error;
-                if (!(need > a.S || err)) {
+                if (!(sh.row_need > a.S || sh.cap_error)) {
                     finalize_report(sh.total, ND, ctl->scal);
                     end_step_report(ctl->c, a.hist, ctl->scal);
                 }
@@ -521,22 +541,26 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
             const std::uint64_t next = ctl->c.steps + 1;
             const bool stats = sh.go && need_hist_stats(ctl->c, a.hist, next, &sh.ahead);
             if (stats) hist_stats_block<kCtlThreads>(a.hist, next, sh.stats, sh.hred);
-            __syncthreads();
-            if (tid == 0 && sh.go) {
-                Controller& c = ctl->c;
-                begin_step(c, a.hist, next, stats ? &sh.stats : nullptr, &sh.ahead);
-                ctl->fix_height_scale = c.reorder ? 1.0 : c.fix_height_scale;
-                if (c.done || c.reorder || c.lock_now) ctl->stopped = 1u;
-                else publish_step(ctl, c, ND);
-            }
+            if (tid == 0) sh.have_stats = stats ? 1 : 0;
             __syncthreads();
         }
         if (ctl->halted) break;
-        // ---- ADAM step + refresh trigger (k_adam_refresh) -------------------
-        const bool refresh = !ctl->stopped && ctl->c.rebuild_mode == REBUILD_CHECK;
-        bool trig = false;
+        // ---- ADAM step (k_adam_refresh); the last thread opens the next step
+        // meanwhile (with fix_height first: the step's stretch comes from it)
+        auto open_next = [&]() {
+            if (tid != kSmallThreads - 1 || !sh.go) return;
+            Controller& c = ctl->c;
+            begin_step(c, a.hist, c.steps + 1, sh.have_stats ? &sh.stats : nullptr, &sh.ahead);
+            ctl->fix_height_scale = c.reorder ? 1.0 : c.fix_height_scale;
+            if (c.done || c.reorder || c.lock_now) ctl->stopped = 1u;
+            else publish_step(ctl, c, ND);
+        };
+        const bool stretch = ctl->c.fix_height != 0;
+        if (stretch) {
+            open_next();
+            __syncthreads();
+        }
         if (mine) {
-            const double fh = ctl->fix_height_scale;
             RCPG_UNROLL
             for (int d = 0; d < ND; ++d) {
                 const std::uint64_t e = static_cast<std::uint64_t>(i) * ND + d;
@@ -545,17 +569,21 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
                 b.m[e] = mi[d];
                 b.v[e] = vi[d];
             }
-            if (fh != 1.0) xi[ND - 1] = xmul(xi[ND - 1], fh);
+            if (stretch && ctl->fix_height_scale != 1.0) xi[ND - 1] = xmul(xi[ND - 1], ctl->fix_height_scale);
             store_pos<ND>(b.pos, i, xi, D0i);
-            if (refresh) {
-                double d2 = 0.0;
-                RCPG_UNROLL
-                for (int d = 0; d < ND; ++d) {
-                    const double dd = xsub(xi[d], xl[d]);
-                    d2 = xadd(d2, xmul(dd, dd));
-                }
-                trig = refresh_trigger(d2, xmul(D0i, ctl->refresh_kappa), xmul(D0i, ctl->kappa_min), ctl->theta);
+        }
+        if (!stretch) open_next();
+        __syncthreads();
+        // ---- refresh trigger -------------------------------------------------
+        bool trig = false;
+        if (mine && !ctl->stopped && ctl->c.rebuild_mode == REBUILD_CHECK) {
+            double d2 = 0.0;
+            RCPG_UNROLL
+            for (int d = 0; d < ND; ++d) {
+                const double dd = xsub(xi[d], xl[d]);
+                d2 = xadd(d2, xmul(dd, dd));
             }
+            trig = refresh_trigger(d2, xmul(D0i, ctl->refresh_kappa), xmul(D0i, ctl->kappa_min), ctl->theta);
         }
         // meanwhile, the parts of the next step's schedule that are known now
         if (lane == 0) prepare_ahead(ctl->c, a.hist, sh.ahead, warp);

@@ -140,9 +140,7 @@ __device__ __forceinline__ void store_search_record(float* fpos, const DevCtl* c
 //
 // G lanes share a particle. G = 1: one thread walks the ranges in order
 // (consecutive threads are neighbours in space, so their ranges overlap and
-// stay in L1). G > 1: the lanes read the ranges of G grid rows, number
-// their candidates with a scan over the lanes and test G consecutive
-// candidates at a time; ballots keep the scan order. The scan
+// stay in L1). G > 1: search_row_group(). The scan
 // order -- size classes, then the cells with axis 0 fastest, then the
 // members -- does not depend on G, so neither do the rows. row_lanes() picks G
 // per size class: the particles of a class are consecutive, and those of a
@@ -153,10 +151,11 @@ __device__ __forceinline__ void store_search_record(float* fpos, const DevCtl* c
 // where cells hold half a particle) and, for small packings, by the latency of
 // cell start -> record -> test. One B200, per build, against the
 // warp-per-particle search over single cells in FP64 that it replaces: 3-D
-// power law N = 300,007 790 -> 212 us; 4-D log-normal N = 12,001 255 -> 96 us
+// power law N = 300,007 790 -> 212 us; 4-D log-normal N = 12,001 255 -> 74 us
 // early in the run.
 constexpr int kRowThreads = 128;
 constexpr int kRowList = 24;          // listed candidates per lane
+constexpr int kSliceLanes = 8;        // groups up to this size deal out ranges, larger ones candidates
 // In box sides: the FP32 rounding of a position, of t and of L - |t| is at most
 // 1.2e-7 per axis (3.4e-7 in 8 dimensions), and positions may lie 1e-6 outside
 // the box; relative: the sum of squares and the cutoff round by less than 1e-6.
@@ -455,18 +454,20 @@ __device__ __forceinline__ std::uint32_t search_row_one(const DevArrays& a, cons
     return rs.n;
 }
 
-// The row of particle t by the G lanes of its group (a power of two, 2 to 32,
-// aligned in the warp). All 32 lanes enter, groups without a particle with
-// live = false: the loops run to the longest group of the warp and every vote
-// and shuffle has the full mask, since votes on per-group masks run one group
-// after the other. The three arrays are the warp's: 32 * kRowList listed
-// candidates, 64 range starts and 64 range ends. Returns the row length in
-// every lane of the group.
+// Rows by the G lanes of a particle's group (a power of two, 2 to 32, aligned
+// in the warp). All 32 lanes enter, groups without a particle with live =
+// false: the loops run to the longest group of the warp and every vote and
+// shuffle has the full mask, since votes on per-group masks run one group
+// after the other. The three arrays are the warp's: 32 * (kRowList + 1) listed
+// candidates, 64 range starts and 64 range ends.
+//
+// One size class by candidates: the ranges of G grid rows at a time are
+// numbered by a scan over the lanes, each round tests G consecutive candidates.
 template <int ND, bool NC>
-__device__ __forceinline__ std::uint32_t search_row_group(const DevArrays& a, const DevCtl* ctl,
-                                                          const SearchParams<ND>& sp, const std::uint32_t* cell_start,
-                                                          std::uint32_t t, bool live, int G, std::uint32_t* s_list,
-                                                          std::uint32_t* s_q, std::uint32_t* s_end) {
+__device__ __forceinline__ void search_class_group(const DevArrays& a, const DevCtl* ctl, const SearchParams<ND>& sp,
+                                                   const std::uint32_t* cell_start, const RowScan<ND>& sc,
+                                                   RowSearch<ND, NC>& rs, int G, std::uint32_t* s_list,
+                                                   std::uint32_t* s_q, std::uint32_t* s_end) {
     constexpr unsigned kAll = 0xffffffffu;
     const std::uint64_t N = a.N;
     const std::uint32_t S = a.S;
@@ -478,8 +479,7 @@ __device__ __forceinline__ std::uint32_t search_row_group(const DevArrays& a, co
     std::uint32_t* const list = s_list + first * kRowList;
     std::uint32_t* const sq = s_q + 2 * first;
     std::uint32_t* const se = s_end + 2 * first;
-    RowSearch<ND, NC> rs;
-    rs.begin(a, live ? t : 0u, sp.kap, sp.t_shell, sp.widest);
+    rs.listed = 0;
     // partners among the listed candidates, appended to the row in order
     auto flush = [&]() {
         __syncwarp();
@@ -506,68 +506,145 @@ __device__ __forceinline__ std::uint32_t search_row_group(const DevArrays& a, co
         rs.listed = 0;
         __syncwarp();
     };
-    for (int kc = 0; kc < sp.K; ++kc) {
-        RowScan<ND> sc;
-        sc.open(ctl, kc, sp.K, sp.kap, sp.t_shell, rs.xi, rs.Di, sp.side, sp.widest, sp.prune);
-        if (!live) sc.rows = 0;
-        const int most_rows = __reduce_max_sync(kAll, sc.rows);
-        for (int r0 = 0; r0 < most_rows; r0 += G) {
-            // the ranges of row r0 + s; numbers of the non-empty ranges and of their candidates
-            std::uint32_t q0 = 0, q1 = 0, q2 = 0, q3 = 0;
-            if (r0 + s < sc.rows) sc.row_ranges(r0 + s, cell_start, sp.side, q0, q1, q2, q3);
-            const std::uint32_t n0 = q1 - q0, n1 = q3 - q2;
-            std::uint32_t ci = n0 + n1, ei = (n0 != 0u) + (n1 != 0u);
-            for (int o = 1; o < G; o <<= 1) {
-                const std::uint32_t cv = __shfl_up_sync(kAll, ci, o, G), ev = __shfl_up_sync(kAll, ei, o, G);
-                if (s >= o) {
-                    ci += cv;
-                    ei += ev;
-                }
+    const int most_rows = __reduce_max_sync(kAll, sc.rows);
+    for (int r0 = 0; r0 < most_rows; r0 += G) {
+        // the ranges of row r0 + s; numbers of the non-empty ranges and of their candidates
+        std::uint32_t q0 = 0, q1 = 0, q2 = 0, q3 = 0;
+        if (r0 + s < sc.rows) sc.row_ranges(r0 + s, cell_start, sp.side, q0, q1, q2, q3);
+        const std::uint32_t n0 = q1 - q0, n1 = q3 - q2;
+        std::uint32_t ci = n0 + n1, ei = (n0 != 0u) + (n1 != 0u);
+        for (int o = 1; o < G; o <<= 1) {
+            const std::uint32_t cv = __shfl_up_sync(kAll, ci, o, G), ev = __shfl_up_sync(kAll, ei, o, G);
+            if (s >= o) {
+                ci += cv;
+                ei += ev;
             }
-            const std::uint32_t T = __shfl_sync(kAll, ci, G - 1, G);
-            const std::uint32_t most = __reduce_max_sync(kAll, T);
-            if (most == 0) continue;
-            ci -= n0 + n1;
-            ei -= (n0 != 0u) + (n1 != 0u);
-            __syncwarp();  // the previous ranges are no longer read
-            if (n0) {
-                sq[ei] = q0 - ci;
-                ci += n0;
-                se[ei++] = ci;
+        }
+        const std::uint32_t T = __shfl_sync(kAll, ci, G - 1, G);
+        const std::uint32_t most = __reduce_max_sync(kAll, T);
+        if (most == 0) continue;
+        ci -= n0 + n1;
+        ei -= (n0 != 0u) + (n1 != 0u);
+        __syncwarp();  // the previous ranges are no longer read
+        if (n0) {
+            sq[ei] = q0 - ci;
+            ci += n0;
+            se[ei++] = ci;
+        }
+        if (n1) {
+            sq[ei] = q2 - ci;
+            se[ei] = ci + n1;
+        }
+        __syncwarp();
+        // G consecutive candidates per round, U rounds in flight
+        constexpr int U = 4;
+        int e = 0;
+        for (std::uint32_t k0 = 0; k0 < most; k0 += U * G) {
+            if (__any_sync(kAll, rs.listed > L - U * G)) flush();
+            std::uint32_t q[U];
+            bool hit[U];
+            RCPG_UNROLL
+            for (int u = 0; u < U; ++u) {
+                const std::uint32_t k = k0 + static_cast<std::uint32_t>(u * G + s);
+                hit[u] = k < T;
+                if (hit[u])
+                    while (k >= se[e]) ++e;
+                q[u] = hit[u] ? k + sq[e] : rs.t;
             }
-            if (n1) {
-                sq[ei] = q2 - ci;
-                se[ei] = ci + n1;
-            }
-            __syncwarp();
-            // G consecutive candidates per round, U rounds in flight
-            constexpr int U = 4;
-            int e = 0;
-            for (std::uint32_t k0 = 0; k0 < most; k0 += U * G) {
-                if (__any_sync(kAll, rs.listed > L - U * G)) flush();
-                std::uint32_t q[U];
-                bool hit[U];
-                RCPG_UNROLL
-                for (int u = 0; u < U; ++u) {
-                    const std::uint32_t k = k0 + static_cast<std::uint32_t>(u * G + s);
-                    hit[u] = k < T;
-                    if (hit[u])
-                        while (k >= se[e]) ++e;
-                    q[u] = hit[u] ? k + sq[e] : rs.t;
-                }
-                SearchRecord<ND> r[U];
-                RCPG_UNROLL
-                for (int u = 0; u < U; ++u) r[u] = load_search_record<ND, NC>(fpos, q[u]);
-                RCPG_UNROLL
-                for (int u = 0; u < U; ++u) {
-                    const unsigned hits = (__ballot_sync(kAll, maybe_partner<ND>(rs.ri, rs.half_i, r[u], sp.side) && hit[u]) >> first) & group;
-                    if ((hits >> s) & 1u) list[rs.listed + __popc(hits & below)] = q[u];
-                    rs.listed += static_cast<std::uint32_t>(__popc(hits));
-                }
+            SearchRecord<ND> r[U];
+            RCPG_UNROLL
+            for (int u = 0; u < U; ++u) r[u] = load_search_record<ND, NC>(fpos, q[u]);
+            RCPG_UNROLL
+            for (int u = 0; u < U; ++u) {
+                const unsigned hits =
+                    (__ballot_sync(kAll, maybe_partner<ND>(rs.ri, rs.half_i, r[u], sp.side) && hit[u]) >> first) & group;
+                if ((hits >> s) & 1u) list[rs.listed + __popc(hits & below)] = q[u];
+                rs.listed += static_cast<std::uint32_t>(__popc(hits));
             }
         }
     }
     flush();
+}
+
+// The row of particle t by its group, each size class in one of two ways. Few
+// ranges per lane (small groups): each lane walks its own slice of the class's
+// ranges and keeps its partners in its own list, and the lists are appended in
+// lane order; a list that overflows makes the warp repeat the class by
+// candidates. Many lanes for few ranges: by candidates at once. Returns the
+// row length in every lane of the group.
+template <int ND, bool NC>
+__device__ __forceinline__ std::uint32_t search_row_group(const DevArrays& a, const DevCtl* ctl,
+                                                          const SearchParams<ND>& sp, const std::uint32_t* cell_start,
+                                                          std::uint32_t t, bool live, int G, std::uint32_t* s_list,
+                                                          std::uint32_t* s_q, std::uint32_t* s_end) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const std::uint64_t N = a.N;
+    const std::uint32_t S = a.S;
+    const float* const fpos = a.fpos;
+    const int lane = threadIdx.x & 31, s = lane & (G - 1);
+    RowSearch<ND, NC> rs;
+    rs.begin(a, live ? t : 0u, sp.kap, sp.t_shell, sp.widest);
+    for (int kc = 0; kc < sp.K; ++kc) {
+        RowScan<ND> sc;
+        sc.open(ctl, kc, sp.K, sp.kap, sp.t_shell, rs.xi, rs.Di, sp.side, sp.widest, sp.prune);
+        if (!live) sc.rows = 0;
+        bool by_candidates = G > kSliceLanes;
+        if (!by_candidates) {
+            std::uint32_t* const list = s_list + lane * (kRowList + 1);
+            std::uint32_t cnt = 0;
+            const int r1 = sc.rows * (s + 1) / G;
+            for (int r = sc.rows * s / G; r < r1; ++r) {
+                std::uint32_t q, qe, q2, q3;
+                sc.row_ranges(r, cell_start, sp.side, q, qe, q2, q3);
+                for (;;) {
+                    if (q >= qe) {  // the wrapped part of the range, then done
+                        if (q2 >= q3) break;
+                        q = q2;
+                        qe = q3;
+                        q2 = q3;
+                    }
+                    constexpr std::uint32_t U = 4;  // candidates in flight
+                    SearchRecord<ND> rec[U];
+                    RCPG_UNROLL
+                    for (std::uint32_t u = 0; u < U; ++u) rec[u] = load_search_record<ND, NC>(fpos, min(q + u, qe - 1));
+                    RCPG_UNROLL
+                    for (std::uint32_t u = 0; u < U; ++u) {
+                        if (q + u < qe && maybe_partner<ND>(rs.ri, rs.half_i, rec[u], sp.side)) {
+                            if (cnt < static_cast<std::uint32_t>(kRowList)) list[cnt] = q + u;
+                            ++cnt;
+                        }
+                    }
+                    q += U;
+                }
+            }
+            by_candidates = __any_sync(kAll, cnt > static_cast<std::uint32_t>(kRowList));
+            if (!by_candidates) {
+                std::uint32_t m = 0;  // partners kept
+                for (std::uint32_t k = 0; k < cnt; k += 2) {
+                    const std::uint32_t qa = list[k], qb = k + 1 < cnt ? list[k + 1] : qa;
+                    const bool oa = rs.partner(a, ctl, qa, sp.kap, sp.t_shell);
+                    const bool ob = rs.partner(a, ctl, qb, sp.kap, sp.t_shell) && k + 1 < cnt;
+                    if (oa) list[m++] = qa;
+                    if (ob) list[m++] = qb;
+                }
+                __syncwarp();
+                std::uint32_t incl = m;
+                for (int o = 1; o < G; o <<= 1) {
+                    const std::uint32_t v = __shfl_up_sync(kAll, incl, o, G);
+                    if (s >= o) incl += v;
+                }
+                for (std::uint32_t k = 0; k < m; ++k) {
+                    const std::uint32_t slot = rs.n + incl - m + k;
+                    if (slot < S) a.nbr[static_cast<std::uint64_t>(slot) * N + rs.t] = list[k];
+                }
+                rs.n += __shfl_sync(kAll, incl, G - 1, G);
+            }
+        }
+        if (by_candidates) {
+            __syncwarp();  // the lanes' lists are no longer read
+            search_class_group<ND, NC>(a, ctl, sp, cell_start, sc, rs, G, s_list, s_q, s_end);
+        }
+    }
     return rs.n;
 }
 

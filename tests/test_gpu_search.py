@@ -27,7 +27,7 @@ def _state(n, nd, ratio, phi, stray, seed=7):
     return x, D
 
 
-# n: one particle, around a warp, each rule of search_lanes (32, 8 and 1 lanes; 4-D: 32 and 8)
+# n: one particle, around a warp, each rule of search_lanes (32, 4 and 1 lanes; 4-D: 16 and 8)
 @pytest.mark.parametrize("n,nd,ratio,phi,stray", [
     (1, 2, 1.0, 0.1, False), (2, 3, 1.0, 0.3, False), (33, 2, 1.3, 0.5, False), (63, 3, 1.0, 0.3, True),
     (129, 4, 2.0, 0.15, False), (500, 2, 12.0, 0.5, False), (4095, 3, 1.4, 0.3, False),
