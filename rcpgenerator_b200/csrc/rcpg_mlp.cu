@@ -1,8 +1,8 @@
 // Learned warm start: a small MLP (BF16 weights and activations, FP32
 // accumulation, FP32 master weights) mapping size-distribution descriptors to
 // a predicted phi_J and a growth schedule. Hand-written training and inference
-// kernels: a strided tensor-core GEMM (mma.sync BF16 -> FP32), GELU, mean
-// squared error, Adam.
+// kernels: tensor-core tile products (mma.sync BF16 -> FP32) with GELU, mean
+// squared error and their gradients in the epilogues, and Adam.
 //
 // Parameters of an L-layer MLP with widths w[0..L] are packed in one FP32
 // array: layer l holds W_l [w[l+1] x w[l]] row-major, then b_l [w[l+1]]. The
@@ -20,84 +20,24 @@
 
 namespace {
 
-// Tensor-core GEMM: C[m, n] = sum_k A[m*sam + k*sak] * B[k*sbk + n*sbn] (+ bias[n]).
-// A 64x64 tile of C per block of 4 warps (2x2), each warp 32x32 as 2x4
-// mma.sync.m16n8k16 BF16 tiles with FP32 accumulators. Any operand strides:
-// every K step of 16 stages the A (m, k) and B (n, k) slices in shared memory,
-// zero-filled outside the matrices, with rows padded to 24 elements (12
-// words) so that the fragment loads of a warp fall in distinct banks.
-constexpr int kBM = 64, kBN = 64, kBK = 16, kPad = 24, kGemmThreads = 128;
+// Tensor-core tile products: C[m, n] = sum_k A[m, k] B[k, n] by mma.sync
+// m16n8k16 (BF16 operands, FP32 accumulators, k ascending). These layers are
+// 256 wide, so a product of a training batch is a few hundred tiles at most and
+// a launch is bound by latency, not by the tensor cores: a block takes a 32x32
+// tile of C (64 blocks where 64x64 tiles gave 16) and stages up to 256 of k at
+// once, every load of the chunk in flight before the first mma, instead of 16
+// with two barriers each; activation, loss, gradient and bias sums are the
+// tiles' epilogues, and the two products of a layer's backward pass and its
+// bias sums share a launch. A training step of batch 256 is 9 launches (it was
+// 26). A step of batch 256 on one B200, whole call: 226 -> 89 us. The sums keep
+// their order, so the results are those of the larger tiles bit for bit.
+constexpr int kTM = 32, kTN = 32;      // tile of C
+constexpr int kKC = 256;               // k staged at once
+constexpr int kRow = kKC + 8;          // staged row: fragment loads of a warp fall in distinct banks
+constexpr int kMmaThreads = 128;
 
 __device__ __forceinline__ std::uint32_t lds_pair(const __nv_bfloat16* p) {
     return *reinterpret_cast<const std::uint32_t*>(p);
-}
-
-__global__ void __launch_bounds__(kGemmThreads)
-    k_gemm_bf16(int M, int N, int K, const __nv_bfloat16* __restrict__ A, long long sam, long long sak,
-                const __nv_bfloat16* __restrict__ B, long long sbk, long long sbn, float* __restrict__ C,
-                long long ldc, const float* __restrict__ bias) {
-    __shared__ __align__(16) __nv_bfloat16 As[kBM][kPad];
-    __shared__ __align__(16) __nv_bfloat16 Bs[kBN][kPad];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-    const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
-    float acc[2][4][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0f;
-    const __nv_bfloat16 zero = __float2bfloat16(0.0f);
-    for (int k0 = 0; k0 < K; k0 += kBK) {
-        // stage: 64x16 elements of each operand, 8 per thread
-#pragma unroll
-        for (int r = 0; r < (kBM * kBK) / kGemmThreads; ++r) {
-            const int e = tid + r * kGemmThreads;
-            const int row = e / kBK, kk = e % kBK;
-            const int m = m0 + row, n = n0 + row, k = k0 + kk;
-            As[row][kk] = (m < M && k < K) ? A[m * sam + k * sak] : zero;
-            Bs[row][kk] = (n < N && k < K) ? B[k * sbk + n * sbn] : zero;
-        }
-        __syncthreads();
-        std::uint32_t af[2][4], bf[4][2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int r0 = wm + i * 16 + g;
-            af[i][0] = lds_pair(&As[r0][2 * t]);
-            af[i][1] = lds_pair(&As[r0 + 8][2 * t]);
-            af[i][2] = lds_pair(&As[r0][2 * t + 8]);
-            af[i][3] = lds_pair(&As[r0 + 8][2 * t + 8]);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c0 = wn + j * 8 + g;
-            bf[j][0] = lds_pair(&Bs[c0][2 * t]);
-            bf[j][1] = lds_pair(&Bs[c0][2 * t + 8]);
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                asm volatile(
-                    "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
-                    "{%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
-                    : "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3])
-                    : "r"(af[i][0]), "r"(af[i][1]), "r"(af[i][2]), "r"(af[i][3]), "r"(bf[j][0]), "r"(bf[j][1]));
-        __syncthreads();
-    }
-    // epilogue: c0, c1 at (g, 2t..2t+1), c2, c3 at (g+8, 2t..2t+1) of each 16x8 tile
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int m = m0 + wm + i * 16 + g + (r >= 2 ? 8 : 0);
-                const int n = n0 + wn + j * 8 + 2 * t + (r & 1);
-                if (m < M && n < N) C[m * ldc + n] = acc[i][j][r] + (bias ? bias[n] : 0.0f);
-            }
 }
 
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
@@ -105,36 +45,177 @@ __device__ __forceinline__ float gelu_grad(float x) {
     return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
-// activation of a layer's pre-activations z: a = gelu(z) (hidden) or z (output), stored BF16
-__global__ void k_act(int n, const float* __restrict__ z, __nv_bfloat16* __restrict__ a, int hidden) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = __float2bfloat16(hidden ? gelu(z[i]) : z[i]);
+// An operand as rows over k: element (r, k) at p[r * rs + k * ks]. FP32 inputs
+// are rounded to BF16 as they are staged.
+template <typename T>
+struct Operand {
+    const T* p;
+    long long rs, ks;
+};
+
+__device__ __forceinline__ __nv_bfloat16 as_bf16(__nv_bfloat16 v) { return v; }
+__device__ __forceinline__ __nv_bfloat16 as_bf16(float v) { return __float2bfloat16(v); }
+
+// Stages rows r0 .. r0 + 31 (of `rows`), k0 .. k0 + kc - 1 (of K; kc a multiple
+// of 16) into s[32][kRow], zeros outside. 16-byte loads where the operand is
+// BF16, contiguous along k or along the rows, and aligned; else one by one.
+template <typename T>
+__device__ __forceinline__ void stage(__nv_bfloat16 (*s)[kRow], const Operand<T>& o, int r0, int rows, int k0, int K,
+                                      int kc) {
+    const __nv_bfloat16 zero = __float2bfloat16(0.0f);
+    if constexpr (sizeof(T) == 2) {
+        const bool base16 = (reinterpret_cast<std::uintptr_t>(o.p) & 15u) == 0;
+        if (base16 && o.ks == 1 && (o.rs & 7) == 0 && (K & 7) == 0) {
+            const int per = kc / 8;
+            for (int e = threadIdx.x; e < 32 * per; e += kMmaThreads) {
+                const int r = e / per, k = (e - r * per) * 8;
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (r0 + r < rows && k0 + k < K)
+                    v = *reinterpret_cast<const uint4*>(o.p + (r0 + r) * o.rs + k0 + k);
+                *reinterpret_cast<uint4*>(&s[r][k]) = v;
+            }
+            return;
+        }
+        if (base16 && o.rs == 1 && (o.ks & 7) == 0 && (rows & 7) == 0) {
+            for (int e = threadIdx.x; e < 4 * kc; e += kMmaThreads) {
+                const int k = e >> 2, r = (e & 3) * 8;
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (r0 + r < rows && k0 + k < K)
+                    v = *reinterpret_cast<const uint4*>(o.p + (k0 + k) * o.ks + r0 + r);
+                const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) s[r + q][k] = w[q];
+            }
+            return;
+        }
+    }
+    const bool along_k = o.ks == 1;
+    for (int e = threadIdx.x; e < 32 * kc; e += kMmaThreads) {
+        const int r = along_k ? e / kc : (e & 31), k = along_k ? e - r * kc : (e >> 5);
+        s[r][k] = (r0 + r < rows && k0 + k < K) ? as_bf16(o.p[(r0 + r) * o.rs + (k0 + k) * o.ks]) : zero;
+    }
 }
 
-// output layer: loss terms and dL/dz = 2 (y - t) / (B * O), BF16
-__global__ void k_mse(int B, int O, const float* __restrict__ z, const float* __restrict__ t,
-                      const float* __restrict__ wt, __nv_bfloat16* __restrict__ dz, float* __restrict__ lterm) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * O) return;
-    const float w = wt ? wt[i % O] : 1.0f;
-    const float d = z[i] - t[i];
-    lterm[i] = w * d * d;
-    dz[i] = __float2bfloat16(2.0f * w * d / static_cast<float>(B * O));
+struct Tile {
+    __nv_bfloat16 a[kTM][kRow], b[kTN][kRow];
+};
+
+// The 32x32 tile at (m0, n0) of A (M x K) times B (K x N, given by columns);
+// out(m, n, c) for every element inside the matrix. Each of the four warps
+// holds 16x16 of it.
+template <typename TA, typename TB, typename Out>
+__device__ __forceinline__ void tile_product(Tile& t, const Operand<TA>& A, const Operand<TB>& B, int M, int N, int K,
+                                             int m0, int n0, Out&& out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, q = lane & 3;
+    const int wm = (warp >> 1) * 16, wn = (warp & 1) * 16;
+    float acc[2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[j][r] = 0.0f;
+    for (int k0 = 0; k0 < K; k0 += kKC) {
+        const int kc = min(kKC, (K - k0 + 15) & ~15);
+        if (k0) __syncthreads();
+        stage(t.a, A, m0, M, k0, K, kc);
+        stage(t.b, B, n0, N, k0, K, kc);
+        __syncthreads();
+#pragma unroll 4
+        for (int k = 0; k < kc; k += 16) {
+            std::uint32_t af[4], bf[2][2];
+            af[0] = lds_pair(&t.a[wm + g][k + 2 * q]);
+            af[1] = lds_pair(&t.a[wm + g + 8][k + 2 * q]);
+            af[2] = lds_pair(&t.a[wm + g][k + 2 * q + 8]);
+            af[3] = lds_pair(&t.a[wm + g + 8][k + 2 * q + 8]);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                bf[j][0] = lds_pair(&t.b[wn + j * 8 + g][k + 2 * q]);
+                bf[j][1] = lds_pair(&t.b[wn + j * 8 + g][k + 2 * q + 8]);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                asm volatile(
+                    "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
+                    "{%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
+                    : "+f"(acc[j][0]), "+f"(acc[j][1]), "+f"(acc[j][2]), "+f"(acc[j][3])
+                    : "r"(af[0]), "r"(af[1]), "r"(af[2]), "r"(af[3]), "r"(bf[j][0]), "r"(bf[j][1]));
+        }
+    }
+    // c0, c1 at (g, 2q..2q+1), c2, c3 at (g+8, 2q..2q+1) of each 16x8 tile
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int m = m0 + wm + g + (r >= 2 ? 8 : 0);
+            const int n = n0 + wn + j * 8 + 2 * q + (r & 1);
+            if (m < M && n < N) out(m, n, acc[j][r]);
+        }
 }
 
-// dz = da * gelu'(z), BF16
-__global__ void k_gelu_bwd(int n, const float* __restrict__ da, const float* __restrict__ z,
-                           __nv_bfloat16* __restrict__ dz) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dz[i] = __float2bfloat16(da[i] * gelu_grad(z[i]));
+// One layer forward: z = a W^T + bias; a hidden layer stores gelu(z) in BF16
+// (and z where the backward pass will need it), the output layer z, and with
+// `target` the loss terms and dL/dz = 2 w (z - t) / (batch * outputs) in BF16.
+template <typename TA>
+__global__ void __launch_bounds__(kMmaThreads)
+    k_forward(int M, int N, int K, const TA* __restrict__ a, const __nv_bfloat16* __restrict__ W,
+              const float* __restrict__ bias, float* __restrict__ z, __nv_bfloat16* __restrict__ act,
+              const float* __restrict__ target, const float* __restrict__ weight, __nv_bfloat16* __restrict__ dz,
+              float* __restrict__ lterm) {
+    __shared__ __align__(16) Tile t;
+    tile_product(t, Operand<TA>{a, K, 1}, Operand<__nv_bfloat16>{W, K, 1}, M, N, K, blockIdx.y * kTM, blockIdx.x * kTN,
+                 [&](int m, int n, float c) {
+                     const long long e = static_cast<long long>(m) * N + n;
+                     const float v = c + bias[n];
+                     if (z) z[e] = v;
+                     if (act) act[e] = __float2bfloat16(gelu(v));
+                     if (target) {
+                         const float w = weight ? weight[n] : 1.0f;
+                         const float d = v - target[e];
+                         lterm[e] = w * d * d;
+                         dz[e] = __float2bfloat16(2.0f * w * d / static_cast<float>(M * N));
+                     }
+                 });
 }
 
-// db[o] = sum_b dz[b, o] (FP32, b ascending)
-__global__ void k_bias_grad(int B, int O, const __nv_bfloat16* __restrict__ dz, float* __restrict__ db) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+// One layer backward from dz (B x O): blocks 0 .. nx-1 the tiles of dz_prev =
+// (dz W) gelu'(z_prev) (B x I, BF16; none for the first layer), then the tiles
+// of dW = dz^T a (O x I), then the bias sums db[o] = sum_b dz[b, o] (FP32, b
+// ascending; 128 outputs per block).
+template <typename TA>
+__global__ void __launch_bounds__(kMmaThreads)
+    k_backward(int B, int O, int I, const __nv_bfloat16* __restrict__ dz, const TA* __restrict__ a,
+               const __nv_bfloat16* __restrict__ W, const float* __restrict__ z_prev,
+               __nv_bfloat16* __restrict__ dz_prev, float* __restrict__ dW, float* __restrict__ db, int nx, int nw) {
+    __shared__ __align__(16) Tile t;
+    int b = blockIdx.x;
+    const int ti = (I + kTN - 1) / kTN;
+    if (b < nx) {
+        tile_product(t, Operand<__nv_bfloat16>{dz, O, 1}, Operand<__nv_bfloat16>{W, 1, I}, B, I, O, (b / ti) * kTM,
+                     (b % ti) * kTN, [&](int m, int n, float c) {
+                         const long long e = static_cast<long long>(m) * I + n;
+                         dz_prev[e] = __float2bfloat16(c * gelu_grad(z_prev[e]));
+                     });
+        return;
+    }
+    b -= nx;
+    if (b < nw) {
+        tile_product(t, Operand<__nv_bfloat16>{dz, 1, O}, Operand<TA>{a, 1, I}, O, I, B, (b / ti) * kTM, (b % ti) * kTN,
+                     [&](int m, int n, float c) { dW[static_cast<long long>(m) * I + n] = c; });
+        return;
+    }
+    b -= nw;
+    const int o = b * kMmaThreads + threadIdx.x;
     if (o >= O) return;
     float s = 0.0f;
-    for (int b = 0; b < B; ++b) s += __bfloat162float(dz[b * O + o]);
+    int r = 0;
+    for (; r + 16 <= B; r += 16) {  // sixteen loads in flight, added in order
+        float v[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = __bfloat162float(dz[static_cast<long long>(r + q) * O + o]);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) s += v[q];
+    }
+    for (; r < B; ++r) s += __bfloat162float(dz[static_cast<long long>(r) * O + o]);
     db[o] = s;
 }
 
@@ -159,12 +240,6 @@ __global__ void k_adam(int n, float* __restrict__ w, float* __restrict__ m, floa
     wb[i] = __float2bfloat16(wi);
 }
 
-void gemm(cudaStream_t st, int M, int N, int K, const __nv_bfloat16* A, long long sam, long long sak,
-          const __nv_bfloat16* B, long long sbk, long long sbn, float* C, long long ldc, const float* bias) {
-    dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM);
-    k_gemm_bf16<<<grid, kGemmThreads, 0, st>>>(M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, bias);
-}
-
 unsigned blocks(long long n) { return static_cast<unsigned>((n + 255) / 256); }
 
 std::size_t param_count(const int32_t* w, int L) {
@@ -175,9 +250,8 @@ std::size_t param_count(const int32_t* w, int L) {
 
 // Scratch of one forward/backward pass, carved from the caller's workspace.
 struct Work {
-    std::vector<__nv_bfloat16*> act;  // act[0] = input, act[l+1] = output of layer l (BF16)
+    std::vector<__nv_bfloat16*> act;  // act[l] = output of layer l - 1 (BF16), l >= 1
     std::vector<float*> z;            // pre-activations of layer l (FP32)
-    float* da;                        // FP32 gradient w.r.t. an activation
     __nv_bfloat16* dz;                // BF16 gradient w.r.t. a pre-activation
     __nv_bfloat16* dzp;               // the previous layer's
     float* lterm;
@@ -198,22 +272,31 @@ bool carve(void* ws, std::size_t ws_bytes, const int32_t* w, int L, int B, Work&
     wk.z.resize(L);
     for (int l = 0; l <= L; ++l) wk.act[l] = static_cast<__nv_bfloat16*>(take(static_cast<std::size_t>(B) * w[l] * 2));
     for (int l = 0; l < L; ++l) wk.z[l] = static_cast<float*>(take(static_cast<std::size_t>(B) * w[l + 1] * 4));
-    wk.da = static_cast<float*>(take(static_cast<std::size_t>(B) * wmax * 4));
+    take(static_cast<std::size_t>(B) * wmax * 4);
     wk.dz = static_cast<__nv_bfloat16*>(take(static_cast<std::size_t>(B) * wmax * 2));
     wk.dzp = static_cast<__nv_bfloat16*>(take(static_cast<std::size_t>(B) * wmax * 2));
     wk.lterm = static_cast<float*>(take(static_cast<std::size_t>(B) * w[L] * 4));
     return used <= ws_bytes;
 }
 
+// The layers' launches. y: where the output layer's z goes; with T the loss
+// terms go to lterm and the gradient to wk.dz, and the hidden z are kept.
 void forward(cudaStream_t st, const int32_t* w, int L, int B, const __nv_bfloat16* wb, const float* w32,
-             const float* X, Work& wk) {
-    k_to_bf16<<<blocks(static_cast<long long>(B) * w[0]), 256, 0, st>>>(B * w[0], X, wk.act[0]);
+             const float* X, Work& wk, float* y, const float* T, const float* weight, float* lterm) {
     std::size_t off = 0;
     for (int l = 0; l < L; ++l) {
         const int I = w[l], O = w[l + 1];
-        // z[b, o] = sum_i act[b, i] W[o, i] + bias[o]
-        gemm(st, B, O, I, wk.act[l], I, 1, wb + off, 1, I, wk.z[l], O, w32 + off + static_cast<std::size_t>(O) * I);
-        k_act<<<blocks(static_cast<long long>(B) * O), 256, 0, st>>>(B * O, wk.z[l], wk.act[l + 1], l + 1 < L);
+        const bool last = l + 1 == L;
+        const dim3 grid((O + kTN - 1) / kTN, (B + kTM - 1) / kTM);
+        const float* bias = w32 + off + static_cast<std::size_t>(O) * I;
+        float* z = last ? y : (T ? wk.z[l] : nullptr);
+        __nv_bfloat16* act = last ? nullptr : wk.act[l + 1];
+        const float* tgt = last ? T : nullptr;
+        if (l == 0)
+            k_forward<float><<<grid, kMmaThreads, 0, st>>>(B, O, I, X, wb + off, bias, z, act, tgt, weight, wk.dz, lterm);
+        else
+            k_forward<__nv_bfloat16><<<grid, kMmaThreads, 0, st>>>(B, O, I, wk.act[l], wb + off, bias, z, act, tgt, weight,
+                                                                   wk.dz, lterm);
         off += static_cast<std::size_t>(O) * I + O;
     }
 }
@@ -260,9 +343,8 @@ int32_t rcpg_mlp_forward(const int32_t* widths, int32_t layers, int32_t batch, c
     Work wk;
     if (!carve(workspace, workspace_bytes, widths, layers, batch, wk))
         return fail(err, errlen, RCPG_EINVAL, "rcpgenerator_b200: MLP workspace too small");
-    forward(st, widths, layers, batch, static_cast<const __nv_bfloat16*>(w_bf16), w_fp32, X, wk);
-    cudaMemcpyAsync(Y, wk.z[layers - 1], static_cast<std::size_t>(batch) * widths[layers] * 4,
-                    cudaMemcpyDeviceToDevice, st);
+    forward(st, widths, layers, batch, static_cast<const __nv_bfloat16*>(w_bf16), w_fp32, X, wk, Y, nullptr, nullptr,
+            nullptr);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(err, errlen, RCPG_ECUDA, cudaGetErrorString(e));
     return RCPG_OK;
@@ -282,10 +364,8 @@ int32_t rcpg_mlp_train_step(const int32_t* widths, int32_t layers, int32_t batch
     if (!carve(workspace, workspace_bytes, widths, layers, batch, wk))
         return fail(err, errlen, RCPG_EINVAL, "rcpgenerator_b200: MLP workspace too small");
     auto* wb = static_cast<__nv_bfloat16*>(w_bf16);
-    forward(st, widths, layers, batch, wb, w_fp32, X, wk);
-    const int O = widths[layers];
-    k_mse<<<blocks(static_cast<long long>(batch) * O), 256, 0, st>>>(batch, O, wk.z[layers - 1], T, out_weight,
-                                                                      wk.dz, wk.lterm);
+    forward(st, widths, layers, batch, wb, w_fp32, X, wk, wk.z[layers - 1], T, out_weight,
+            loss_terms ? loss_terms : wk.lterm);
     // offsets of the layers in the packed parameters
     std::vector<std::size_t> off(layers + 1, 0);
     for (int l = 0; l < layers; ++l) off[l + 1] = off[l] + static_cast<std::size_t>(widths[l + 1]) * widths[l] + widths[l + 1];
@@ -293,18 +373,18 @@ int32_t rcpg_mlp_train_step(const int32_t* widths, int32_t layers, int32_t batch
         const int I = widths[l], Ol = widths[l + 1];
         float* gW = grad + off[l];
         float* gb = gW + static_cast<std::size_t>(Ol) * I;
-        // dW[o, i] = sum_b dz[b, o] act[b, i]
-        gemm(st, Ol, I, batch, wk.dz, 1, Ol, wk.act[l], I, 1, gW, I, nullptr);
-        k_bias_grad<<<blocks(Ol), 256, 0, st>>>(batch, Ol, wk.dz, gb);
+        const int ti = (I + kTN - 1) / kTN, tb = (batch + kTM - 1) / kTM, to = (Ol + kTM - 1) / kTM;
+        const int nx = l > 0 ? tb * ti : 0, nw = to * ti, nb = (Ol + kMmaThreads - 1) / kMmaThreads;
+        const unsigned grid = static_cast<unsigned>(nx + nw + nb);
         if (l > 0) {
-            // da[b, i] = sum_o dz[b, o] W[o, i]; dz_prev = da * gelu'(z_prev)
-            gemm(st, batch, I, Ol, wk.dz, Ol, 1, wb + off[l], I, 1, wk.da, I, nullptr);
-            k_gelu_bwd<<<blocks(static_cast<long long>(batch) * I), 256, 0, st>>>(batch * I, wk.da, wk.z[l - 1], wk.dzp);
+            k_backward<__nv_bfloat16><<<grid, kMmaThreads, 0, st>>>(batch, Ol, I, wk.dz, wk.act[l], wb + off[l],
+                                                                    wk.z[l - 1], wk.dzp, gW, gb, nx, nw);
             std::swap(wk.dz, wk.dzp);
+        } else {
+            k_backward<float><<<grid, kMmaThreads, 0, st>>>(batch, Ol, I, wk.dz, X, wb + off[l], nullptr, nullptr, gW, gb,
+                                                            nx, nw);
         }
     }
-    if (loss_terms)
-        cudaMemcpyAsync(loss_terms, wk.lterm, static_cast<std::size_t>(batch) * O * 4, cudaMemcpyDeviceToDevice, st);
     if (adam_m && adam_v && lr > 0.0f) {
         const float b1 = 0.9f, b2 = 0.999f;
         const float c1 = 1.0f - std::pow(b1, static_cast<float>(step)), c2 = 1.0f - std::pow(b2, static_cast<float>(step));

@@ -139,3 +139,14 @@ def test_errors_are_loud(cuda_device):
     err = N.errbuf()
     rc = N.lib.rcpg_mlp_forward(w, 2, 4, None, None, None, None, None, 0, None, err, len(err))
     assert rc == N.RCPG_EINVAL and b"bad arguments" in err.value
+
+
+# tiles of 32 and staged chunks of 256 along k: aligned and unaligned rows, one chunk and a ragged second one
+@pytest.mark.parametrize("K,O,B", [(8, 8, 32), (264, 33, 64), (512, 24, 31), (300, 64, 33), (24, 40, 1)])
+def test_tile_edges_exact_on_small_integers(cuda_device, K, O, B):
+    test_tensor_core_gemm_exact_on_small_integers(cuda_device, K, O, B)
+
+
+@pytest.mark.parametrize("widths,B", [((8, 32, 16, 8), 32), ((12, 40, 24, 5), 257), ((16, 264, 9), 31), ((4, 7, 3), 513)])
+def test_gradient_matches_oracle_at_tile_edges(cuda_device, widths, B):
+    test_gradient_matches_oracle(cuda_device, widths, B)
