@@ -373,6 +373,14 @@ uint64_t rcpg_mlp_workspace_bytes(const int32_t* widths, int32_t layers, int32_t
 int32_t rcpg_mlp_forward(const int32_t* widths, int32_t layers, int32_t batch, const void* w_bf16,
                          const float* w_fp32, const float* X, float* Y, void* workspace,
                          uint64_t workspace_bytes, void* stream, char* err, size_t errlen);
+/* A warm start's prediction for raw FP64 descriptors X [batch x I], I =
+ * widths[0], O = widths[layers]: X is held inside [lo, hi], standardised ((x -
+ * mean) / std, FP64) and rounded to FP32 for the network, and Y [batch x O] =
+ * network * y_std + y_mean (FP64, no fused multiply-add). `norm` (device):
+ * lo[I], hi[I], mean[I], std[I], y_mean[O], y_std[O]. */
+int32_t rcpg_mlp_predict(const int32_t* widths, int32_t layers, int32_t batch, const void* w_bf16,
+                         const float* w_fp32, const double* X, const double* norm, double* Y,
+                         void* workspace, uint64_t workspace_bytes, void* stream, char* err, size_t errlen);
 /* One training step on the loss L = sum_{b,o} out_weight[o] (Y[b,o] - T[b,o])^2 / (batch * widths[layers])
  * (out_weight NULL = all ones): grad [param_count] = dL/dparams (FP32), and
  * loss_terms [batch x widths[layers]] (optional) the summands. With lr > 0 and

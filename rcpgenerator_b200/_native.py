@@ -53,6 +53,7 @@ EXPORTED_SYMBOLS = (
     "rcpg_mlp_param_count",
     "rcpg_mlp_workspace_bytes",
     "rcpg_mlp_forward",
+    "rcpg_mlp_predict",
     "rcpg_mlp_train_step",
     "rcpg_mlp_to_bf16",
 )
@@ -267,6 +268,10 @@ def _load() -> C.CDLL:
         "rcpg_mlp_forward": (
             C.c_int32,
             [_i32p, C.c_int32, C.c_int32, vp, vp, vp, vp, vp, C.c_uint64, vp, cp, sz],
+        ),
+        "rcpg_mlp_predict": (
+            C.c_int32,
+            [_i32p, C.c_int32, C.c_int32, vp, vp, vp, vp, vp, vp, C.c_uint64, vp, cp, sz],
         ),
         "rcpg_mlp_train_step": (
             C.c_int32,

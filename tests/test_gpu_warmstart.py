@@ -60,3 +60,21 @@ def test_training_pipeline_from_engine_packings(cuda_device):
     ws = W.WarmStart.fit(X, Y, epochs=150, batch=48, lr=2e-3)
     P = ws.predict(X)
     assert np.abs(P[:, 0] - Y[:, 0]).mean() < 0.3 * Y[:, 0].std()
+
+
+@pytest.mark.parametrize("rows", [1, 7, 33, 513])
+@pytest.mark.parametrize("held", [True, False])
+def test_prediction_scales_like_numpy(cuda_device, rows, held):
+    """predict() scales on the GPU: the same bits as NumPy around the network's
+    forward pass, also for rows outside the training range and NaN."""
+    from rcpgenerator_b200.warmstart import WarmStart
+    ws = WarmStart.load()
+    lo, hi = ws.x_lo, ws.x_hi
+    rng = np.random.default_rng(rows)
+    X = lo + (hi - lo + 0.1) * rng.uniform(-0.3, 1.3, (rows, lo.size))
+    X[0, 3] = np.nan
+    if not held:
+        ws.x_lo = ws.x_hi = None
+    Z = np.clip(X, lo, hi) if held else X
+    want = ws.net.forward((Z - ws.x_mean) / ws.x_std).astype(np.float64) * ws.y_std + ws.y_mean
+    np.testing.assert_array_equal(ws.predict(X), want)
