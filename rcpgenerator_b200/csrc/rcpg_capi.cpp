@@ -649,6 +649,7 @@ int32_t rcpg_pairs_forces_scan(uint64_t N, int32_t ndim, const double* x_dev, co
         }
         a.cell_count = u32(a.C_alloc + 1ull);
         a.cell_start = u32(a.C_alloc + 1ull);
+        cuda_ok(cudaMemsetAsync(a.cell_count, 0, (a.C_alloc + 1ull) * 4, st), "memset cell counts");
         a.scan_tmp = u32(2 * 4096 + 16);
         a.block_sums = static_cast<rcpg::ForceSums*>(
             sc.get(std::max<std::size_t>(rcpg::force_blocks(N), 4096) * sizeof(rcpg::ForceSums)));

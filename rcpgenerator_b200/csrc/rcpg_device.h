@@ -130,7 +130,7 @@ struct DevArrays {
     std::uint64_t* u64_tmp; // [N]
     std::uint32_t* cell_of;    // [N]
     std::uint32_t* cell_rank;  // [N]
-    std::uint32_t* cell_count; // [C_alloc + 1]
+    std::uint32_t* cell_count; // [C_alloc + 1]; with cell-order storage all zero between builds
     std::uint32_t* cell_start; // [C_alloc + 1]
     std::uint32_t* cell_list;  // [N] members of each cell in arrival order (k_build_scatter)
     std::uint32_t C_alloc;
@@ -195,7 +195,11 @@ RCPG_HD unsigned force_blocks(std::uint64_t N) {
 // ---- launchers (rcpg_kernels.cu) ------------------------------------------
 // All take the device arrays by value and enqueue on `st`.
 void launch_adam_refresh(const DevArrays& a, int do_adam, int do_refresh, cudaStream_t st);
-void launch_rebuild(const DevArrays& a, cudaStream_t st);
+// Whether a graph-mode build orders each cell's members first and then gathers
+// the particles (k_build_move says why the line lies there).
+inline bool gather_build(std::uint64_t N) { return N >= 200000; }
+// planned: the step gate of the same graph step has planned the build.
+void launch_rebuild(const DevArrays& a, cudaStream_t st, bool planned = false);
 // the same, with e0 / e1 recorded just before and after the search kernels
 // (the cell-unit or tiled search and the row or warp search; those that have nothing to do return)
 void launch_rebuild_timed(const DevArrays& a, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1);
@@ -203,7 +207,7 @@ void launch_forces(const DevArrays& a, int exact_terms, cudaStream_t st);
 // One variant of the pair kernel (mixed = 0: FP64 pair terms, 1: FP32 pair
 // terms), the body of a step graph's pair-kernel switch.
 void launch_forces_variant(const DevArrays& a, int mixed, cudaStream_t st);
-// The step gate of a captured step graph: opens the build (cond_build = 1
+// The step gate of a captured step graph: plans and opens the build (cond_build = 1
 // when the step rebuilds its rows) and sets the pair-kernel switch for a step
 // without a build.
 void launch_step_gate(const DevArrays& a, unsigned long long cond_build, cudaStream_t st);

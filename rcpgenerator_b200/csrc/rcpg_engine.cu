@@ -210,6 +210,7 @@ void Engine::alloc_device() {
     }
     a_.cell_count = static_cast<std::uint32_t*>(dalloc((a_.C_alloc + 1ull) * 4));
     a_.cell_start = static_cast<std::uint32_t*>(dalloc((a_.C_alloc + 1ull) * 4));
+    check(cudaMemsetAsync(a_.cell_count, 0, (a_.C_alloc + 1ull) * 4, st_), "memset cell counts");
     a_.scan_tmp = static_cast<std::uint32_t*>(dalloc(2 * 4096 * 4 + 64));
     // per-block partial sums: one per force block, or one per block of the
     // persistent tiled build when it computes the forces
@@ -744,15 +745,16 @@ void Engine::destroy_graph() {
     graph_ = nullptr;
 }
 
-// Kernels of one neighbour build (launch_rebuild): prepare, bin, the scan
-// (one kernel, or three for more than 4096 tiles of cells), scatter, cell
-// sort, the permutation of cell-order storage, the cell-unit search
-// (ndim <= 3, N >= 20,000; one kernel per pair precision the run may use) or
-// the tiled search, and the row search (graph mode) or the warp search.
+// Kernels of one neighbour build (launch_rebuild): prepare (in the step graph:
+// the gate's part), bin, the scan (one kernel, or two for more than 4096
+// cells), scatter, the move into cell order or the cell sort (large packings:
+// both; exact mode: the sort), the
+// cell-unit search (ndim <= 3, N >= 20,000; one kernel per pair precision the
+// run may use) or the tiled search, and the row search (graph mode) or the warp
+// search.
 std::uint64_t Engine::kernels_per_build() const {
-    const std::uint64_t cells = static_cast<std::uint64_t>(a_.C_alloc) + 1;
-    const std::uint64_t scans = cells <= 4096 ? 1 : 3;
-    std::uint64_t k = 4 + scans + (a_.permute ? 1 : 0) + 1;
+    const std::uint64_t scans = static_cast<std::uint64_t>(a_.C_alloc) + 1 <= 4096 ? 1 : 2;
+    std::uint64_t k = 4 + scans + (a_.permute && gather_build(N_) ? 2 : 1);
     if (ndim_ <= 3 && N_ >= 20000) {
         if (a_.permute) k += a_.mixed ? 2 : 1;
         else if (a_.sorted_rows) k += 1;
@@ -795,7 +797,7 @@ void Engine::capture_step() {
     DevArrays ag = a_;
     ag.cond_forces = forces;
     launch_step_gate(ag, build, st_);
-    add_conditional(cudaGraphCondTypeIf, build, 1, [&](cudaStream_t s, unsigned) { launch_rebuild(ag, s); });
+    add_conditional(cudaGraphCondTypeIf, build, 1, [&](cudaStream_t s, unsigned) { launch_rebuild(ag, s, true); });
     add_conditional(cudaGraphCondTypeSwitch, forces, mixed_ ? 2u : 1u,
                     [&](cudaStream_t s, unsigned variant) { launch_forces_variant(ag, static_cast<int>(variant), s); });
     launch_controller(ag, 0, st_);

@@ -157,46 +157,55 @@ __device__ __forceinline__ std::uint32_t unit_width(std::uint64_t N, double cell
     return static_cast<std::uint32_t>(w);
 }
 
-__global__ void k_build_prepare(DevArrays a) {
+// Parameters of a build, by one thread: the cell grids, the units and tiles of
+// the searches.
+__device__ void plan_build(const DevArrays& a) {
     DevCtl* ctl = a.ctl;
-    if (build_off(ctl)) return;
-    const std::uint32_t n = a.C_alloc + 1;
-    for (std::uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-        a.cell_count[k] = 0u;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const int nd = a.ndim;
-        double c0;  // cells of class 0's grid
-        plan_grid(ctl, nd, a.C_alloc, c0);
-        const std::uint32_t cells = ctl->ncells;
-        const int nc0 = ctl->cls_ncell[0][0];
-        // cell units of the cell-order kernels (one grid: class 0's)
-        if (nd == 2 || nd == 3) {
-            const std::uint32_t w = nd == 2 ? unit_width<2>(a.N, c0, nc0) : unit_width<3>(a.N, c0, nc0);
-            const std::uint32_t chunks = (static_cast<std::uint32_t>(nc0) + w - 1) / w;
-            std::uint32_t rows = static_cast<std::uint32_t>(ctl->cls_ncell[0][1]);
-            if (nd == 3) rows *= static_cast<std::uint32_t>(ctl->cls_ncell[0][2]);
-            ctl->unit_w = w;
-            ctl->unit_chunks = chunks;
-            ctl->unit_count = chunks * rows;
-        } else {
-            ctl->unit_w = ctl->unit_chunks = ctl->unit_count = 0u;
-        }
-        // 2-D tiles: kTileRowsPref cells high, lower where the halo's
-        // particles at the mean cell occupancy (with 30 % headroom) would not
-        // fit the staging area
-        if (nd == 2) {
-            const double ppc = static_cast<double>(a.N) / static_cast<double>(cells ? cells : 1u);
-            const double fit = floor(static_cast<double>(kTileStage2) / (18.0 * 1.3 * (ppc > 1e-3 ? ppc : 1e-3))) - 2.0;
-            double r = fit < static_cast<double>(kTileRowsPref) ? fit : static_cast<double>(kTileRowsPref);
-            if (!(r >= kTileRowsMin)) r = kTileRowsMin;
-            ctl->tile_rows = static_cast<int>(r);
-        } else {
-            ctl->tile_rows = 0;
-        }
-        // graph mode: the tiled build also computes this step's forces
-        // (only with unsorted rows: a sorted row is summed after its sort)
-        ctl->forces_done = a.sorted_rows ? 0u : ctl->fuse_forces;
+    const int nd = a.ndim;
+    double c0;  // cells of class 0's grid
+    plan_grid(ctl, nd, a.C_alloc, c0);
+    const std::uint32_t cells = ctl->ncells;
+    const int nc0 = ctl->cls_ncell[0][0];
+    // cell units of the cell-order kernels (one grid: class 0's)
+    if (nd == 2 || nd == 3) {
+        const std::uint32_t w = nd == 2 ? unit_width<2>(a.N, c0, nc0) : unit_width<3>(a.N, c0, nc0);
+        const std::uint32_t chunks = (static_cast<std::uint32_t>(nc0) + w - 1) / w;
+        std::uint32_t rows = static_cast<std::uint32_t>(ctl->cls_ncell[0][1]);
+        if (nd == 3) rows *= static_cast<std::uint32_t>(ctl->cls_ncell[0][2]);
+        ctl->unit_w = w;
+        ctl->unit_chunks = chunks;
+        ctl->unit_count = chunks * rows;
+    } else {
+        ctl->unit_w = ctl->unit_chunks = ctl->unit_count = 0u;
     }
+    // 2-D tiles: kTileRowsPref cells high, lower where the halo's
+    // particles at the mean cell occupancy (with 30 % headroom) would not
+    // fit the staging area
+    if (nd == 2) {
+        const double ppc = static_cast<double>(a.N) / static_cast<double>(cells ? cells : 1u);
+        const double fit = floor(static_cast<double>(kTileStage2) / (18.0 * 1.3 * (ppc > 1e-3 ? ppc : 1e-3))) - 2.0;
+        double r = fit < static_cast<double>(kTileRowsPref) ? fit : static_cast<double>(kTileRowsPref);
+        if (!(r >= kTileRowsMin)) r = kTileRowsMin;
+        ctl->tile_rows = static_cast<int>(r);
+    } else {
+        ctl->tile_rows = 0;
+    }
+    // graph mode: the tiled build also computes this step's forces
+    // (only with unsorted rows: a sorted row is summed after its sort)
+    ctl->forces_done = a.sorted_rows ? 0u : ctl->fuse_forces;
+}
+
+// First kernel of a build outside the step graph (there the step gate plans):
+// the plan and, without cell-order storage, the cell counts cleared (with it
+// k_build_move leaves them clear).
+__global__ void k_build_prepare(DevArrays a) {
+    if (build_off(a.ctl)) return;
+    if (!a.permute) {
+        const std::uint32_t n = a.C_alloc + 1;
+        for (std::uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+            a.cell_count[k] = 0u;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) plan_build(a);
 }
 
 template <int ND>
@@ -245,11 +254,21 @@ __global__ void __launch_bounds__(kScanThreads)
     if (threadIdx.x == 0 && block_sums) block_sums[blockIdx.x] = total;
 }
 
+// Adds to each tile the totals of the tiles before it, which every block sums
+// itself (at most kScanTile of them, four per thread): a launch less than
+// scanning the totals first.
 __global__ void __launch_bounds__(kScanThreads)
-    k_scan_add(std::uint32_t* out, std::uint32_t n, const std::uint32_t* block_offsets,
-               const DevCtl* gate) {
+    k_scan_add(std::uint32_t* out, std::uint32_t n, const std::uint32_t* tile_sums, const DevCtl* gate) {
     if (gate && build_off(gate)) return;
-    const std::uint32_t add = block_offsets[blockIdx.x];
+    __shared__ std::uint32_t smem[32];
+    std::uint32_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+        const std::uint32_t t = threadIdx.x + static_cast<std::uint32_t>(k) * kScanThreads;
+        if (t < blockIdx.x) sum += tile_sums[t];
+    }
+    std::uint32_t add;
+    block_exclusive_scan(sum, smem, add);
     const std::uint64_t base = static_cast<std::uint64_t>(blockIdx.x) * kScanTile + threadIdx.x * kScanItems;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k)
@@ -261,13 +280,8 @@ void scan_exclusive(const std::uint32_t* in, std::uint32_t* out, std::uint32_t n
                     std::uint32_t* tmp, const DevCtl* gate, cudaStream_t st) {
     const std::uint32_t tiles = (n + kScanTile - 1) / kScanTile;
     if (tiles > static_cast<std::uint32_t>(kScanTile)) throw std::length_error("rcpg scan: more than 4096^2 elements");
-    if (tiles <= 1) {
-        k_scan_tiles<<<1, kScanThreads, 0, st>>>(in, out, n, nullptr, gate);
-        return;
-    }
-    k_scan_tiles<<<tiles, kScanThreads, 0, st>>>(in, out, n, tmp, gate);
-    k_scan_tiles<<<1, kScanThreads, 0, st>>>(tmp, tmp + kScanTile, tiles, nullptr, gate);
-    k_scan_add<<<tiles, kScanThreads, 0, st>>>(out, n, tmp + kScanTile, gate);
+    k_scan_tiles<<<tiles, kScanThreads, 0, st>>>(in, out, n, tiles > 1 ? tmp : nullptr, gate);
+    if (tiles > 1) k_scan_add<<<tiles, kScanThreads, 0, st>>>(out, n, tmp, gate);
 }
 
 __global__ void __launch_bounds__(256) k_build_scatter(DevArrays a) {
@@ -305,8 +319,8 @@ __device__ __forceinline__ bool use_cells(const DevArrays& a) {
     return ok;
 }
 
-// Builds without the tiled search: the members of each cell in ascending
-// particle order in work (the atomic ranks of k_build_bin are arrival order;
+// Builds with sorted rows but without the tiled search, and large packings in
+// cell-order storage: the members of each cell in ascending particle order in work (the atomic ranks of k_build_bin are arrival order;
 // row slots and per-block force sums must not depend on it), and a copy of
 // their positions in that order (spos), so the search reads each cell's
 // candidates from contiguous memory. The tiled search orders its cells itself.
@@ -350,7 +364,7 @@ __global__ void __launch_bounds__(256) k_build_cell_sort(DevArrays a) {
             a.work[p] = v;
         }
     }
-    if (a.permute) return;  // cell-order storage: k_build_permute moves the particles themselves
+    if (a.permute) return;  // cell-order storage: k_build_move moves the particles themselves
     constexpr int P = pos_stride(ND);
     for (std::uint32_t q = q0; q < q1; ++q) {
         const double2* src = reinterpret_cast<const double2*>(a.pos + static_cast<std::uint64_t>(a.work[q]) * P);
@@ -360,14 +374,23 @@ __global__ void __launch_bounds__(256) k_build_cell_sort(DevArrays a) {
     }
 }
 
-// Cell-order storage (graph mode): particle q of the new order is particle
-// work[q] of the current one (cells in grid order, each cell's members in
-// their current order, written by k_build_cell_sort). Moves the per-particle
-// state into the other buffer set, anchors the refresh trigger there
-// (x_last = x, every build re-anchors every particle) and, once every block
-// has finished (all have read the current set), flips DevCtl::buf.
-template <int ND>
-__global__ void __launch_bounds__(256) k_build_permute(DevArrays a) {
+// Cell-order storage (graph mode): the particles in the order of their cells,
+// each cell's members in their present order. Their state moves to the other
+// buffer set, the refresh trigger is anchored (x_last = x, every build
+// re-anchors every particle), the cell counts are cleared for the next build
+// and, once every block has finished (all have read the current set),
+// DevCtl::buf flips. Two ways, the same result:
+//   GATHER = false: particle i finds its place from the present indices of its
+//     cell's members (a handful, in arrival order in cell_list) and is stored
+//     there: no kernel to order the cells first (9-18 us).
+//   GATHER = true: place q takes particle work[q] (k_build_cell_sort): stores
+//     coalesced. Large packings, whose particles pass several others between
+//     builds early in a run, so that scattered stores hit half sectors all over
+//     the second buffer set.
+// One B200, whole capped runs, moves against gathers: N = 12,001 4-D 77.4 / 86.2
+// ms, N = 100,000 3-D 122.4 / 125.3, N = 300,007 3-D equal, N = 1M 2-D 326 / 309.
+template <int ND, bool GATHER>
+__global__ void __launch_bounds__(256) k_build_move(DevArrays a) {
     DevCtl* ctl = a.ctl;
     if (build_off(ctl)) return;
     const std::uint32_t b = ctl->buf;
@@ -375,62 +398,69 @@ __global__ void __launch_bounds__(256) k_build_permute(DevArrays a) {
     constexpr int P = pos_stride(ND);
     const bool search = !use_cells<ND>(a);  // k_build_rows reads the FP32 search records
     const std::uint64_t N = a.N;
-    // two particles per thread, every load of both before any store
     const std::uint64_t stride = static_cast<std::uint64_t>(gridDim.x) * blockDim.x;
-    for (std::uint64_t q0 = blockIdx.x * static_cast<std::uint64_t>(blockDim.x) + threadIdx.x; q0 < N;
-         q0 += 2 * stride) {
+    const std::uint64_t first = blockIdx.x * static_cast<std::uint64_t>(blockDim.x) + threadIdx.x;
+    for (std::uint64_t c = first; c <= ctl->ncells; c += stride) a.cell_count[c] = 0u;
+    // two particles per thread, every load of both before any store
+    for (std::uint64_t e0 = first; e0 < N; e0 += 2 * stride) {
         constexpr int U = 2;
         double2 rec[U][P / 2];
         double mv[U][2 * ND];
-        std::uint64_t org[U];
-        std::uint32_t cap[U], rr[U];
+        std::uint64_t org[U], q[U];
+        std::uint32_t cap[U], rr[U], q0[U], q1[U];
         RCPG_UNROLL
         for (int u = 0; u < U; ++u) {
-            const std::uint64_t q = q0 + u * stride;
-            if (q >= N) continue;
-            const std::uint64_t o = a.work[q];
-            const double2* ps = reinterpret_cast<const double2*>(src.pos + o * P);
+            const std::uint64_t e = e0 + u * stride;
+            q0[u] = q1[u] = 0u;
+            if (e >= N) continue;
+            const std::uint64_t i = GATHER ? a.work[e] : e;
+            if constexpr (!GATHER) {
+                const std::uint32_t c = a.cell_of[i];
+                q0[u] = a.cell_start[c];
+                q1[u] = a.cell_start[c + 1];
+            }
+            const double2* ps = reinterpret_cast<const double2*>(src.pos + i * P);
             RCPG_UNROLL
             for (int h = 0; h < P / 2; ++h) rec[u][h] = ps[h];
             RCPG_UNROLL
             for (int d = 0; d < ND; ++d) {
-                mv[u][d] = src.m[o * ND + d];
-                mv[u][ND + d] = src.v[o * ND + d];
+                mv[u][d] = src.m[i * ND + d];
+                mv[u][ND + d] = src.v[i * ND + d];
             }
-            org[u] = src.origin[o];
-            cap[u] = src.caps[o];
-            rr[u] = src.ref_rank[o];
+            org[u] = src.origin[i];
+            cap[u] = src.caps[i];
+            rr[u] = src.ref_rank[i];
         }
         RCPG_UNROLL
         for (int u = 0; u < U; ++u) {
-            const std::uint64_t q = q0 + u * stride;
-            if (q >= N) continue;
-            double2* pd = reinterpret_cast<double2*>(dst.pos + q * P);
+            const std::uint64_t e = e0 + u * stride;
+            q[u] = GATHER ? e : q0[u];
+            if constexpr (!GATHER)
+                for (std::uint32_t k = q0[u]; k < q1[u]; ++k) q[u] += a.cell_list[k] < static_cast<std::uint32_t>(e);
+        }
+        RCPG_UNROLL
+        for (int u = 0; u < U; ++u) {
+            if (e0 + u * stride >= N) continue;
+            double2* pd = reinterpret_cast<double2*>(dst.pos + q[u] * P);
+            double xq[ND], D0q = 0.0;
             RCPG_UNROLL
             for (int h = 0; h < P / 2; ++h) {
                 pd[h] = rec[u][h];
-                if (2 * h < ND) a.x_last[q * ND + 2 * h] = rec[u][h].x;
-                if (2 * h + 1 < ND) a.x_last[q * ND + 2 * h + 1] = rec[u][h].y;
+                if (2 * h < ND) xq[2 * h] = rec[u][h].x;
+                else if (2 * h == ND) D0q = rec[u][h].x;
+                if (2 * h + 1 < ND) xq[2 * h + 1] = rec[u][h].y;
+                else if (2 * h + 1 == ND) D0q = rec[u][h].y;
             }
             RCPG_UNROLL
             for (int d = 0; d < ND; ++d) {
-                dst.m[q * ND + d] = mv[u][d];
-                dst.v[q * ND + d] = mv[u][ND + d];
+                a.x_last[q[u] * ND + d] = xq[d];
+                dst.m[q[u] * ND + d] = mv[u][d];
+                dst.v[q[u] * ND + d] = mv[u][ND + d];
             }
-            dst.origin[q] = org[u];
-            dst.caps[q] = cap[u];
-            dst.ref_rank[q] = rr[u];
-            if (search) {
-                double xq[ND], D0q = 0.0;
-                RCPG_UNROLL
-                for (int h = 0; h < P / 2; ++h) {
-                    if (2 * h < ND) xq[2 * h] = rec[u][h].x;
-                    else if (2 * h == ND) D0q = rec[u][h].x;
-                    if (2 * h + 1 < ND) xq[2 * h + 1] = rec[u][h].y;
-                    else if (2 * h + 1 == ND) D0q = rec[u][h].y;
-                }
-                store_search_record<ND>(a.fpos, ctl, &ctl->stray, q, xq, D0q);
-            }
+            dst.origin[q[u]] = org[u];
+            dst.caps[q[u]] = cap[u];
+            dst.ref_rank[q[u]] = rr[u];
+            if (search) store_search_record<ND>(a.fpos, ctl, &ctl->stray, q[u], xq, D0q);
         }
     }
     __syncthreads();
@@ -1955,14 +1985,15 @@ __global__ void __launch_bounds__(kCtlThreads) k_controller(DevArrays a, int ope
     if (threadIdx.x == 0 && s_publish) publish_step(ctl, cs, a.ndim);
 }
 
-// First node of a step in a captured step graph: opens the build when the
-// step rebuilds its rows, and sets the pair-kernel switch for a step without
+// First node of a step in a captured step graph: plans and opens the build
+// when the step rebuilds its rows, and sets the pair-kernel switch for a step without
 // a build (a build's last kernel sets it once the search has decided).
 __global__ void k_step_gate(DevArrays a, unsigned long long cond_build) {
     const DevCtl* ctl = a.ctl;
     const std::uint32_t st = ctl->stopped, ha = ctl->halted, rb = ctl->rebuild_flag, p32 = ctl->pair_fp32;
     const bool live = (st | ha) == 0u;
     const bool build = live && rb != 0u;
+    if (build) plan_build(a);
     cudaGraphSetConditional(cond_build, build ? 1u : 0u);
     cudaGraphSetConditional(a.cond_forces, forces_case(live && !build, p32, a.mixed));
 }
@@ -2374,21 +2405,28 @@ void launch_rows(const DevArrays& a, cudaStream_t st) {
     k_build_rows<ND><<<resident_grid<k_build_rows<ND>>(kRowThreads), kRowThreads, 0, st>>>(a, search_lanes<ND>(a.N));
 }
 
-// e0 / e1 (optional): events recorded around the search kernels only
+// persistent grid, two particles per thread and round
+template <int ND, bool GATHER>
+void move_nd(const DevArrays& a, cudaStream_t st) {
+    const unsigned need = (force_blocks(a.N) + 1) / 2, g = resident_grid<k_build_move<ND, GATHER>>(256);
+    k_build_move<ND, GATHER><<<need < g ? need : g, 256, 0, st>>>(a);
+}
+
+// planned: the step gate has planned the build. e0 / e1 (optional): events
+// recorded around the search kernels only
 template <int ND>
-void rebuild_impl(const DevArrays& a, cudaStream_t st, cudaEvent_t e0 = nullptr, cudaEvent_t e1 = nullptr) {
+void rebuild_impl(const DevArrays& a, cudaStream_t st, bool planned, cudaEvent_t e0 = nullptr,
+                  cudaEvent_t e1 = nullptr) {
     const unsigned nb = force_blocks(a.N);
     const unsigned cb = (a.C_alloc + 1 + 255) / 256;
-    k_build_prepare<<<cb < 1024 ? cb : 1024, 256, 0, st>>>(a);
+    if (!planned) k_build_prepare<<<a.permute ? 1 : (cb < 1024 ? cb : 1024), a.permute ? 32 : 256, 0, st>>>(a);
     k_build_bin<ND><<<nb, kForceBlock, 0, st>>>(a);
     scan_exclusive(a.cell_count, a.cell_start, a.C_alloc + 1, a.scan_tmp, a.ctl, st);
     k_build_scatter<<<nb, kForceBlock, 0, st>>>(a);
-    k_build_cell_sort<ND><<<(a.C_alloc + 255) / 256, 256, 0, st>>>(a);
-    if (a.permute) {
-        // persistent grid, two particles per thread and round
-        const unsigned need = (nb + 1) / 2, g = resident_grid<k_build_permute<ND>>(256);
-        k_build_permute<ND><<<need < g ? need : g, 256, 0, st>>>(a);
-    }
+    const bool gather = a.permute && gather_build(a.N);
+    if (!a.permute || gather) k_build_cell_sort<ND><<<(a.C_alloc + 255) / 256, 256, 0, st>>>(a);
+    if (gather) move_nd<ND, true>(a, st);
+    else if (a.permute) move_nd<ND, false>(a, st);
     if (e0) cudaEventRecord(e0, st);
     if (ND <= 3 && a.N >= kTiledMinN) {  // smaller packings take the row or the warp search
         if (a.permute) {
@@ -2420,12 +2458,12 @@ void launch_adam_refresh(const DevArrays& a, int do_adam, int do_refresh, cudaSt
     RCPG_DISPATCH_ND(a.ndim, (adam_nd<ND>(a, do_adam, do_refresh, st)));
 }
 
-void launch_rebuild(const DevArrays& a, cudaStream_t st) {
-    RCPG_DISPATCH_ND(a.ndim, (rebuild_impl<ND>(a, st)));
+void launch_rebuild(const DevArrays& a, cudaStream_t st, bool planned) {
+    RCPG_DISPATCH_ND(a.ndim, (rebuild_impl<ND>(a, st, planned)));
 }
 
 void launch_rebuild_timed(const DevArrays& a, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1) {
-    RCPG_DISPATCH_ND(a.ndim, (rebuild_impl<ND>(a, st, e0, e1)));
+    RCPG_DISPATCH_ND(a.ndim, (rebuild_impl<ND>(a, st, false, e0, e1)));
 }
 
 void launch_forces(const DevArrays& a, int exact_terms, cudaStream_t st) {

@@ -285,7 +285,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
     __syncthreads();
     if (lane == 0) prepare_ahead(ctl->c, a.hist, sh.ahead, warp);
     if (ctl->stopped | ctl->halted) return;  // the same in every block
-    bool counts_clear = false;  // cell_count is zero (kept so by this launch's builds)
     cluster.sync();             // every block has read the control block and cleared its flags
     for (std::uint32_t it = 0; it < steps; ++it) {
         DevArrays b = bound_arrays(a, ctl->buf);
@@ -303,12 +302,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
             }
             __syncthreads();
             const std::uint32_t ncells = ctl->ncells;
-            if (!counts_clear) {
-                for (std::uint32_t c = rank * kSmallThreads + tid; c < a.C_alloc + 1; c += C * kSmallThreads)
-                    a.cell_count[c] = 0u;
-                cluster.sync();
-                counts_clear = true;
-            }
             double x[ND], D0 = 0.0;
             std::uint32_t cell = 0, arrival = 0;
             if (mine) {
@@ -354,6 +347,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
                     dst.ref_rank[q] = ref;
                     store_search_record<ND>(a.fpos, ctl, &g->stray, q, x, D0);
                 }
+                // the counts clear again for the next build
                 for (std::uint32_t c = rank * kSmallThreads + tid; c <= ncells; c += C * kSmallThreads)
                     a.cell_count[c] = 0u;
             }
