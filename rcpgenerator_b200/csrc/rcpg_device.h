@@ -154,9 +154,8 @@ struct DevArrays {
     std::uint32_t* caps_alt;
     std::uint32_t* ref_rank;
     std::uint32_t* ref_rank_alt;
-    // [N*search_stride(ndim)] FP32 search records in cell order, written by the
-    // builds whose rows k_build_rows searches: position, then the diameter of
-    // the build
+    // [N*search_stride(ndim)] FP32 search records in cell order, written by each
+    // build for its search: position, then the diameter of the build
     float* fpos;
     // Captured step graphs with conditional nodes (graph mode): the handle of
     // the step's pair-kernel switch (0 = FP64 kernel, 1 = mixed kernel,

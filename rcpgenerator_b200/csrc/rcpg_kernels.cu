@@ -126,30 +126,31 @@ __global__ void __launch_bounds__(256) k_adam_refresh(DevArrays a, int do_adam, 
 constexpr int kTileRowsMin = 4, kTileRowsMax = 12, kTileRowsPref = 8;
 constexpr int kTileStage2 = 1024;  // staged particles per 2-D tile (TileShape<2>::stage)
 
-// Shape of the cell units of the cell-order search (k_cells, below).
+// Shape of the cell units of the cell-order search (k_cells, below). blocks is
+// the grid per SM whatever else would fit: with the units' width and the block
+// size it sets which terms each block sum holds.
 template <int ND>
 struct UnitShape {
     static constexpr int ndc = ND <= 3 ? ND : 3;
     static constexpr int rows = ndc == 2 ? 3 : 9;        // neighbour rows of a unit
     static constexpr int threads = ndc == 2 ? 128 : 64;  // block size
     static constexpr int target = ndc == 2 ? 112 : 56;   // particles per unit
-    static constexpr int stage = ndc == 2 ? 640 : 768;   // staged records (32 bytes each)
+    static constexpr int span = ndc == 2 ? 640 : 768;    // particles of a unit's neighbour rows (they share L1)
     static constexpr int maxw = ndc == 2 ? 256 : 128;    // cells per unit at most
-    static constexpr int slice = maxw + 3;               // cell_start entries per row (build)
-    static constexpr int windows = 3 * rows;             // main, wrapped x-1, wrapped x+1 per row
-    static constexpr int min_blocks = 6;                 // resident blocks per SM (register budget)
+    static constexpr int blocks = 6;                     // blocks per SM (register budget, grid)
+    static constexpr int list = ndc == 2 ? 24 : 40;      // listed candidates per thread
 };
 
 // Cells per unit for a build with `cells` cells in a grid of nc0 cells per row:
-// about `target` particles at the mean occupancy, windows that fit the stage
-// with 30 % headroom, at most maxw cells.
+// about `target` particles at the mean occupancy, at most `span` in its
+// neighbour rows with 30 % headroom, at most maxw cells.
 template <int ND>
 __device__ __forceinline__ std::uint32_t unit_width(std::uint64_t N, double cells, int nc0) {
     using US = UnitShape<ND>;
     const double ppc = static_cast<double>(N) / (cells > 1.0 ? cells : 1.0);
     const double occ = ppc > 1e-3 ? ppc : 1e-3;
     double w = floor(static_cast<double>(US::target) / occ);
-    const double ws = floor(static_cast<double>(US::stage) / (1.3 * US::rows * occ)) - 2.0;
+    const double ws = floor(static_cast<double>(US::span) / (1.3 * US::rows * occ)) - 2.0;
     if (ws < w) w = ws;
     if (w > static_cast<double>(US::maxw)) w = US::maxw;
     if (w > static_cast<double>(nc0)) w = nc0;
@@ -396,7 +397,6 @@ __global__ void __launch_bounds__(256) k_build_move(DevArrays a) {
     const std::uint32_t b = ctl->buf;
     const DevArrays src = bound_arrays(a, b), dst = bound_arrays(a, b ^ 1u);
     constexpr int P = pos_stride(ND);
-    const bool search = !use_cells<ND>(a);  // k_build_rows reads the FP32 search records
     const std::uint64_t N = a.N;
     const std::uint64_t stride = static_cast<std::uint64_t>(gridDim.x) * blockDim.x;
     const std::uint64_t first = blockIdx.x * static_cast<std::uint64_t>(blockDim.x) + threadIdx.x;
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(256) k_build_move(DevArrays a) {
             dst.origin[q[u]] = org[u];
             dst.caps[q[u]] = cap[u];
             dst.ref_rank[q[u]] = rr[u];
-            if (search) store_search_record<ND>(a.fpos, ctl, &ctl->stray, q[u], xq, D0q);
+            store_search_record<ND>(a.fpos, ctl, &ctl->stray, q[u], xq, D0q);
         }
     }
     __syncthreads();
@@ -1095,31 +1095,33 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_build_search_tiled(DevArray
 // With cell-order storage the members of consecutive cells of one grid row
 // are one contiguous range of particles. A unit is a chunk of unit_w
 // consecutive cells of one grid row (2-D: row y; 3-D: row (y, z)), sized by
-// each build so that it holds about UnitShape::target particles and its
-// windows fit the stage. A block takes one unit at a time:
-//   1. the cell_start entries of the unit's 3^(ndim-1) neighbour rows: cells
-//      cx0-1 .. cx1 of each (the main window), plus, where the unit touches
-//      the end of the grid row, the cell at the row's other end (the wrapped
-//      x-1 / x+1 cell);
-//   2. the FP64 records of those windows -- contiguous ranges of pos -- into
-//      shared memory, with coalesced 256-bit loads by the whole block (2-D:
-//      the record's spare slot takes the FP32 diameter of the mixed test);
-//   3. one thread per particle of the unit tests its candidates from shared
-//      memory (windows that do not fit the stage are read from pos instead:
-//      the same code instantiated for global records).
+// each build so that it holds about UnitShape::target particles; a block takes
+// one unit at a time, one thread per particle. A thread tests its candidates in
+// FP32 on the search records that the build's move wrote (as k_build_rows) and
+// lists the few that pass; the list is worked off on the FP64 records. The
+// records of a unit's 3^(ndim-1) neighbour rows are a few contiguous ranges
+// that its threads share in L1: staging them in shared memory first measured
+// the same in 3-D and slower in 2-D (five barriers per unit, of which none is
+// left).
 // A particle's candidates in scan order: the cells x-1, x, x+1 of each
 // neighbour row, rows in order (row offset r = (dy+1) + 3 (dz+1)), then the
 // wrapped cell of each row where the particle sits at the row's end (2-D: the
 // three rows' ranges are walked as one sequence, so the lanes of a warp run
-// about as many rounds as their longest candidate list, and each round probes
-// two candidates before committing them in order). Each goes through
-// the reference's predicate in FP64, or (MX) the mixed-precision shell test
-// (FP32 on FP64 differences, widened by kShellMarginF so that the rows hold
-// every pair of the FP64 shell); rows hold the partners in that order and the
-// step's forces are computed in the same pass, summed in row order with the
-// arithmetic of k_forces (which gives the same forces on these rows bit for
-// bit). MX: each variant returns at once when the step's pair precision is
-// the other one.
+// about as many rounds as their longest candidate list). Each listed candidate
+// goes through the reference's predicate in FP64, or (MX) the mixed-precision
+// shell test (FP32 on FP64 differences, widened by kShellMarginF so that the
+// rows hold every pair of the FP64 shell), two probed before they are committed
+// in order; rows hold the partners in that order and the step's forces are
+// computed in the same pass, summed in row order with the arithmetic of
+// k_forces (which gives the same forces on these rows bit for bit). MX: each
+// variant returns at once when the step's pair precision is the other one.
+//
+// Bound by instruction issue and, in 3-D, by the latency of few warps. Testing
+// every candidate in FP64 took 5,150 (2-D) and 21,000 (3-D) instructions per
+// warp of particles, nearly half of them FP64 in 3-D; the pre-test leaves a
+// third of the candidates to it. One B200: 3-D bidisperse FP64 N = 100,000 207
+// -> 111 us per build (a capped run of 400 steps 122.4 -> 89.0 ms); 2-D
+// bidisperse mixed N = 1M, run of 600 steps 309 -> 291 ms.
 
 // 32-byte particle record (ndim <= 3) from global memory, one 256-bit load
 __device__ __forceinline__ void ld_record(const double* p, double2& lo, double2& hi) {
@@ -1138,14 +1140,6 @@ __device__ __forceinline__ void unpack_record(const double2& lo, const double2& 
     } else {
         D0 = hi.x;
     }
-}
-
-// FP32 diameter kept in the spare slot of a staged 2-D record
-__device__ __forceinline__ double pack_f32(float f) {
-    return __longlong_as_double(static_cast<long long>(__float_as_uint(f)));
-}
-__device__ __forceinline__ float unpack_f32(double d) {
-    return __uint_as_float(static_cast<unsigned>(__double_as_longlong(d)));
 }
 
 // One particle's candidate tests and its pair sums in the arithmetic of
@@ -1232,17 +1226,6 @@ struct UnitPair {
             }
         }
     }
-    // One candidate probed and committed: whether it is a partner.
-    __device__ __forceinline__ bool candidate(bool upper, const double* xj, double D0j, float D0jf,
-                                              const double* bx, const double* ibx, const float* hbf,
-                                              double t_shell, float tf, bool fuse) {
-        Probe pr;
-        probe(pr, xj, D0j, D0jf, bx, ibx, hbf, t_shell, tf, fuse);
-        if (!pr.pass) return false;
-        commit(upper, pr);
-        return true;
-    }
-
     __device__ __forceinline__ void force(double* f) const {
         RCPG_UNROLL
         for (int d = 0; d < ND; ++d) f[d] = MX ? static_cast<double>(fif[d]) : fi[d];
@@ -1250,20 +1233,16 @@ struct UnitPair {
 };
 
 template <int ND, bool MX>
-__global__ void __launch_bounds__(UnitShape<ND>::threads, UnitShape<ND>::min_blocks) k_cells(DevArrays a) {
+__global__ void __launch_bounds__(UnitShape<ND>::threads, UnitShape<ND>::blocks) k_cells(DevArrays a) {
     using US = UnitShape<ND>;
-    constexpr int NDC = US::ndc, R = US::rows, T = US::threads, NW = US::windows;
+    constexpr int NDC = US::ndc, R = US::rows, T = US::threads;
     constexpr int CR = NDC == 2 ? 1 : 4;  // row offset of the unit's own row
     DevCtl* ctl = a.ctl;
     if (build_off(ctl) || !use_cells<ND>(a) || MX != (ctl->pair_fp32 != 0u)) return;
     bind_buffers(a);
-    extern __shared__ __align__(16) double u_stage[];  // [US::stage][4]: the staged records
-    std::uint32_t* s_cs = reinterpret_cast<std::uint32_t*>(u_stage + 4 * US::stage);  // [R][US::slice]
-    // windows, flat index w = 3 r + kind (0 main, 1 wrapped x-1, 2 wrapped x+1):
-    // first particle, length, index of the first record in the stage (or in
-    // pos, for a unit that is not staged)
-    __shared__ std::uint32_t s_wb[NW], s_wl[NW], s_ws[NW];
-    __shared__ std::uint32_t s_qa, s_qb, s_total, s_need;
+    __shared__ std::uint32_t s_list[T][US::list + 1];  // (odd stride: no bank conflicts)
+    std::uint32_t* const list = s_list[threadIdx.x];
+    __shared__ std::uint32_t s_need;
     __shared__ ForceSums s_red[T / 32];
     // the thread's column of the block sums (its particles in order), in
     // shared memory: they change once per particle
@@ -1283,6 +1262,16 @@ __global__ void __launch_bounds__(UnitShape<ND>::threads, UnitShape<ND>::min_blo
     int nc[NDC];
     RCPG_UNROLL
     for (int d = 0; d < NDC; ++d) nc[d] = ctl->ncell[d];
+    const float4* const frec = reinterpret_cast<const float4*>(a.fpos);
+    static_assert(search_stride(NDC) == 4, "one float4 per search record");
+    // the FP32 test's widening covers the mixed shell test's own (kShellMarginF on the square)
+    constexpr float kRel = MX ? 1.00002f : kSearchRel;
+    float side[NDC], widest = 0.0f;
+    RCPG_UNROLL
+    for (int d = 0; d < NDC; ++d) {
+        side[d] = static_cast<float>(bx[d]);
+        widest = fmaxf(widest, side[d]);
+    }
     const double scale0 = ctl->cell_scale[0];
     const std::uint32_t W = ctl->unit_w, chunks = ctl->unit_chunks, units = ctl->unit_count;
     const double kap = ctl->build_kappa;
@@ -1303,10 +1292,8 @@ __global__ void __launch_bounds__(UnitShape<ND>::threads, UnitShape<ND>::min_blo
         const int cx1 = min(cx0 + static_cast<int>(W), nc[0]);
         const int y0 = static_cast<int>(row0 % static_cast<std::uint32_t>(nc[1]));
         const int z0 = NDC == 3 ? static_cast<int>(row0 / static_cast<std::uint32_t>(nc[1])) : 0;
-        const int cl = max(cx0 - 1, 0), ch = min(cx1 + 1, nc[0]);
-        const int cnt = ch - cl + 1;  // cell_start entries of one row's slice
-        // first cell of the grid row at row offset r
-        auto rowbase = [&](int r) -> std::uint64_t {
+        // cell_start of the grid row at row offset r
+        auto row_cells = [&](int r) -> const std::uint32_t* {
             int y = y0 + (r % 3) - 1;
             y = y < 0 ? y + nc[1] : (y >= nc[1] ? y - nc[1] : y);
             std::uint64_t row = static_cast<std::uint64_t>(y);
@@ -1315,212 +1302,161 @@ __global__ void __launch_bounds__(UnitShape<ND>::threads, UnitShape<ND>::min_blo
                 z = z < 0 ? z + nc[2] : (z >= nc[2] ? z - nc[2] : z);
                 row += static_cast<std::uint64_t>(z) * static_cast<std::uint64_t>(nc[1]);
             }
-            return row * static_cast<std::uint64_t>(nc[0]);
+            return a.cell_start + row * static_cast<std::uint64_t>(nc[0]);
         };
-        __syncthreads();  // the previous unit is finished with the shared arrays
-        // 1. cell_start entries: the rows' slices and windows
-        for (int r = 0; r < R; ++r) {
-            const std::uint32_t* cs = a.cell_start + rowbase(r) + cl;
-            for (int c = threadIdx.x; c < cnt; c += T) s_cs[r * US::slice + c] = cs[c];
-        }
-        if (threadIdx.x < R) {
-            const int r = threadIdx.x;
-            const std::uint32_t* cs = a.cell_start + rowbase(r);
-            const std::uint32_t mb = cs[cl], me = cs[ch];
-            std::uint32_t lb = 0, le = 0, rb = 0, re = 0;
-            if (cx0 == 0) {
-                lb = cs[nc[0] - 1];
-                le = cs[nc[0]];
+        const std::uint32_t qb = __ldg(row_cells(CR) + cx1);
+        for (std::uint32_t q = __ldg(row_cells(CR) + cx0) + threadIdx.x; q < qb; q += T) {
+            double xq[ND], D0q;
+            {
+                double2 lo, hi;
+                ld_record(a.pos + 4 * static_cast<std::uint64_t>(q), lo, hi);
+                unpack_record<ND>(lo, hi, xq, D0q);
             }
-            if (cx1 == nc[0]) {
-                rb = cs[0];
-                re = cs[1];
-            }
-            s_wb[3 * r] = mb;
-            s_wl[3 * r] = me - mb;
-            s_wb[3 * r + 1] = lb;
-            s_wl[3 * r + 1] = le - lb;
-            s_wb[3 * r + 2] = rb;
-            s_wl[3 * r + 2] = re - rb;
-            if (r == CR) {
-                s_qa = cs[cx0];
-                s_qb = cs[cx1];
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            std::uint32_t tot = 0;
-            for (int w = 0; w < NW; ++w) {
-                s_ws[w] = tot;
-                tot += s_wl[w];
-            }
-            s_total = tot;
-            if (tot > static_cast<std::uint32_t>(US::stage))  // not staged: records read from pos
-                for (int w = 0; w < NW; ++w) s_ws[w] = s_wb[w];
-        }
-        __syncthreads();
-        const std::uint32_t total = s_total;
-        const bool staged = total <= static_cast<std::uint32_t>(US::stage);
-        // 2. stage the windows: each thread copies records tid, tid + T, ... of
-        // their concatenation, four loads in flight before the stores
-        if (staged) {
-            int wc = 0;
-            for (std::uint32_t e0 = threadIdx.x; e0 < total; e0 += 4u * T) {
-                double2 lo[4], hi[4];
+            UnitPair<ND, MX> up;
+            up.begin(xq, D0q, kap);
+            float xf[ND];
+            RCPG_UNROLL
+            for (int d = 0; d < ND; ++d) xf[d] = static_cast<float>(xq[d]);
+            const float half_q = __fmaf_rn(__fmaf_rn(static_cast<float>(up.Di), 0.5f, tf), kRel, kSearchAbs * widest);
+            std::uint32_t n = 0, listed = 0;
+            // FP32 test of a record: false only for a particle outside the shell
+            auto maybe = [&](const float4& r) {
+                float d2 = 0.0f;
+                const float rx[3] = {r.x, r.y, r.z};
                 RCPG_UNROLL
-                for (int k = 0; k < 4; ++k) {
-                    const std::uint32_t e = e0 + static_cast<std::uint32_t>(k * T);
-                    if (e < total) {
-                        while (e - s_ws[wc] >= s_wl[wc]) ++wc;
-                        const std::uint64_t p = s_wb[wc] + (e - s_ws[wc]);
-                        ld_record(a.pos + 4 * p, lo[k], hi[k]);
-                    }
+                for (int d = 0; d < NDC; ++d) {
+                    const float t = fabsf(rx[d] - xf[d]);
+                    const float m = fminf(t, side[d] - t);
+                    d2 = __fmaf_rn(m, m, d2);
                 }
-                RCPG_UNROLL
-                for (int k = 0; k < 4; ++k) {
-                    const std::uint32_t e = e0 + static_cast<std::uint32_t>(k * T);
-                    if (e < total) {
-                        if constexpr (NDC == 2) hi[k].y = pack_f32(static_cast<float>(hi[k].x));
-                        double2* dst = reinterpret_cast<double2*>(u_stage + 4 * static_cast<std::size_t>(e));
-                        dst[0] = lo[k];
-                        dst[1] = hi[k];
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        const std::uint32_t own_b = s_wb[3 * CR], own_s = s_ws[3 * CR];
-        // 3. the unit's particles; records from the stage or, for a unit whose
-        // windows did not fit, from pos
-        auto particles = [&](auto staged_tag) {
-            constexpr bool STG = decltype(staged_tag)::value;
-            const double* recs = STG ? static_cast<const double*>(u_stage) : a.pos;  // record s at recs + 4 s
-            for (std::uint32_t q = s_qa + threadIdx.x; q < s_qb; q += T) {
-                double xq[ND], D0q;
-                {
-                    const double2* r2 =
-                        reinterpret_cast<const double2*>(recs + 4 * static_cast<std::size_t>(own_s + (q - own_b)));
-                    unpack_record<ND>(r2[0], r2[1], xq, D0q);
-                }
-                UnitPair<ND, MX> up;
-                up.begin(xq, D0q, kap);
-                std::uint32_t n = 0;
-                // candidate p, record s of `recs`
-                auto test = [&](std::uint32_t p, std::uint32_t s) {
-                    const double2* r2 = reinterpret_cast<const double2*>(recs + 4 * static_cast<std::size_t>(s));
-                    const double2 lo = r2[0], hi = r2[1];
-                    double xj[ND], D0j;
-                    unpack_record<ND>(lo, hi, xj, D0j);
-                    float D0jf = 0.0f;
-                    if constexpr (MX) D0jf = (STG && NDC == 2) ? unpack_f32(hi.y) : static_cast<float>(D0j);
-                    if (up.candidate(p > q, xj, D0j, D0jf, bx, ibx, hbf, t_shell, tf, fuse)) {
-                        if (n < S) a.nbr[static_cast<std::uint64_t>(n) * N + q] = p;
-                        ++n;
-                    }
-                };
-                // the binning's cell (same arithmetic and positions), held
-                // inside the unit so that every slice index stays in range
-                const int cx = min(max(cell_coord(xq[0], scale0, nc[0]), cx0), cx1 - 1);
-                const int lo = cx == 0 ? 0 : cx - 1, hi = cx == nc[0] - 1 ? nc[0] : cx + 2;
-                // the main ranges: cells lo .. hi-1 of each row
-                if constexpr (NDC == 2) {
-                    std::uint32_t pb[3], ns[3], sb[3];
+                const float rc = __fmaf_rn(NDC == 2 ? r.z : r.w, 0.5f * kRel, half_q);
+                return !(d2 > rc * rc);
+            };
+            // the listed candidates, two probed side by side and committed in order
+            auto flush = [&]() {
+                for (std::uint32_t k = 0; k < listed; k += 2) {
+                    std::uint32_t pp[2];
+                    double2 rl[2], rh[2];
+                    typename UnitPair<ND, MX>::Probe pr[2];
                     RCPG_UNROLL
-                    for (int r = 0; r < 3; ++r) {
-                        const std::uint32_t* sl = s_cs + r * US::slice;
-                        pb[r] = sl[lo - cl];
-                        ns[r] = sl[hi - cl] - pb[r];
-                        sb[r] = s_ws[3 * r] + (pb[r] - s_wb[3 * r]);
+                    for (int v = 0; v < 2; ++v) {
+                        pp[v] = list[min(k + static_cast<std::uint32_t>(v), listed - 1)];
+                        ld_record(a.pos + 4 * static_cast<std::uint64_t>(pp[v]), rl[v], rh[v]);
                     }
-                    const std::uint32_t c1 = ns[0], c2 = ns[0] + ns[1], tot = c2 + ns[2];
-                    // two candidates per round: both probed (independent
-                    // work for the lane), then committed in scan order
-                    for (std::uint32_t k = 0; k < tot; k += 2) {
-                        std::uint32_t pp[2];
-                        typename UnitPair<ND, MX>::Probe pr[2];
-                        RCPG_UNROLL
-                        for (int v = 0; v < 2; ++v) {
-                            const std::uint32_t kk = min(k + static_cast<std::uint32_t>(v), tot - 1);
-                            const bool r0 = kk < c1, r1 = kk < c2;
-                            const std::uint32_t o = r0 ? kk : (r1 ? kk - c1 : kk - c2);
-                            pp[v] = (r0 ? pb[0] : (r1 ? pb[1] : pb[2])) + o;
-                            const std::uint32_t st = (r0 ? sb[0] : (r1 ? sb[1] : sb[2])) + o;
-                            const double2* r2 = reinterpret_cast<const double2*>(recs + 4 * static_cast<std::size_t>(st));
-                            const double2 rl = r2[0], rh = r2[1];
-                            double xj[ND], D0j;
-                            unpack_record<ND>(rl, rh, xj, D0j);
-                            float D0jf = 0.0f;
-                            if constexpr (MX) D0jf = STG ? unpack_f32(rh.y) : static_cast<float>(D0j);
-                            up.probe(pr[v], xj, D0j, D0jf, bx, ibx, hbf, t_shell, tf, fuse);
-                        }
-                        RCPG_UNROLL
-                        for (int v = 0; v < 2; ++v) {
-                            if (k + static_cast<std::uint32_t>(v) < tot && pp[v] != q && pr[v].pass) {
-                                if (n < S) a.nbr[static_cast<std::uint64_t>(n) * N + q] = pp[v];
-                                ++n;
-                                up.commit(pp[v] > q, pr[v]);
-                            }
+                    RCPG_UNROLL
+                    for (int v = 0; v < 2; ++v) {
+                        double xj[ND], D0j;
+                        unpack_record<ND>(rl[v], rh[v], xj, D0j);
+                        up.probe(pr[v], xj, D0j, static_cast<float>(D0j), bx, ibx, hbf, t_shell, tf, fuse);
+                    }
+                    RCPG_UNROLL
+                    for (int v = 0; v < 2; ++v) {
+                        if (k + static_cast<std::uint32_t>(v) < listed && pp[v] != q && pr[v].pass) {
+                            if (n < S) a.nbr[static_cast<std::uint64_t>(n) * N + q] = pp[v];
+                            ++n;
+                            up.commit(pp[v] > q, pr[v]);
                         }
                     }
-                } else {
-                    for (int r = 0; r < R; ++r) {
-                        const std::uint32_t* sl = s_cs + r * US::slice;
-                        const std::uint32_t pb = sl[lo - cl], pe = sl[hi - cl];
-                        const std::uint32_t sb = s_ws[3 * r] + (pb - s_wb[3 * r]);
-                        for (std::uint32_t p = pb; p < pe; ++p)
-                            if (p != q) test(p, sb + (p - pb));
-                    }
                 }
-                // the wrapped cells: the x-1 cell of a particle at x = 0, the
-                // x+1 cell of one at x = nc0-1
-                if (cx == 0 || cx == nc[0] - 1) {
-                    const int wk = cx == 0 ? 1 : 2;
-                    for (int r = 0; r < R; ++r) {
-                        const std::uint32_t wb = s_wb[3 * r + wk], wl = s_wl[3 * r + wk], ws = s_ws[3 * r + wk];
-                        for (std::uint32_t o = 0; o < wl; ++o)
-                            if (wb + o != q) test(wb + o, ws + o);
-                    }
+                listed = 0;
+            };
+            // candidates p .. pe - 1, four in flight
+            auto range = [&](std::uint32_t p, std::uint32_t pe) {
+                constexpr std::uint32_t U = 4;
+                for (; p < pe; p += U) {
+                    bool hit[U];
+                    RCPG_UNROLL
+                    for (std::uint32_t u = 0; u < U; ++u) hit[u] = maybe(__ldg(frec + min(p + u, pe - 1))) && p + u < pe;
+                    RCPG_UNROLL
+                    for (std::uint32_t u = 0; u < U; ++u)
+                        if (hit[u]) list[listed++] = p + u;
+                    if (listed > static_cast<std::uint32_t>(US::list) - U) flush();
                 }
-                // the reference's capacity check counts the partners after q in
-                // its own order; a row that fits the capacity in full needs no count
-                const std::uint32_t cap = a.caps[q];
-                if (n > cap && n <= S) {
-                    const std::uint32_t rq = a.ref_rank[q];
-                    std::uint32_t n_half = 0;
-                    for (std::uint32_t k = 0; k < n; ++k)
-                        n_half += a.ref_rank[a.nbr[static_cast<std::uint64_t>(k) * N + q]] > rq;
-                    if (n_half > cap) report_cap_error(ctl, rq, cap);
-                }
-                need = max(need, n);
-                if (n > S) {
-                    a.nbr_cnt[q] = 0u;  // overflow: empty row, rebuilt after the capacity grows
-                    overflow = true;
-                    continue;
-                }
-                a.nbr_cnt[q] = n;
-                if (!fuse) continue;
-                double f[ND];
-                up.force(f);
-                s_acc[0][col] = xadd(s_acc[0][col], static_cast<double>(up.sU));
-                s_acc[1][col] = xadd(s_acc[1][col], static_cast<double>(up.sLc));
-                s_acc[2][col] = xadd(s_acc[2][col], static_cast<double>(up.sdk));
-                s_acc[3][col] = xadd(s_acc[3][col], static_cast<double>(up.sFm));
-                s_acc[4][col] = fmax(s_acc[4][col], static_cast<double>(up.smax));
-                std::uint32_t wc = 0;
-                wall_forces<ND>(xq, up.Di, g, f, s_acc[0][col], s_acc[2][col], s_acc[3][col], wc);
-                s_accn[0][col] += up.scount + wc;
-                const double f2 = force_norm2<ND>(f);
-                if (f2 > 1.0E-16) {
-                    s_acc[5][col] = xadd(s_acc[5][col], xsqrt(f2));
-                    ++s_accn[1][col];
-                }
-                s_acc[6][col] = xadd(s_acc[6][col], up.Di);
+            };
+            // the binning's cell (same arithmetic and positions), held
+            // inside the unit
+            const int cx = min(max(cell_coord(xq[0], scale0, nc[0]), cx0), cx1 - 1);
+            const int lo = cx == 0 ? 0 : cx - 1, hi = cx == nc[0] - 1 ? nc[0] : cx + 2;
+            // the main ranges: cells lo .. hi-1 of each row
+            if constexpr (NDC == 2) {
+                // candidate k of the three rows' sequence is particle k + dp of its row
+                std::uint32_t dp[3], end[3], tot = 0;
                 RCPG_UNROLL
-                for (int d = 0; d < ND; ++d) a.F[static_cast<std::uint64_t>(q) * ND + d] = f[d];
+                for (int r = 0; r < 3; ++r) {
+                    const std::uint32_t* cs = row_cells(r);
+                    const std::uint32_t pb = __ldg(cs + lo);
+                    dp[r] = pb - tot;
+                    tot += __ldg(cs + hi) - pb;
+                    end[r] = tot;
+                }
+                constexpr std::uint32_t U = 4;
+                for (std::uint32_t k = 0; k < tot; k += U) {
+                    std::uint32_t p[U];
+                    bool hit[U];
+                    RCPG_UNROLL
+                    for (std::uint32_t u = 0; u < U; ++u) {
+                        const std::uint32_t kk = min(k + u, tot - 1);
+                        p[u] = kk + (kk < end[0] ? dp[0] : (kk < end[1] ? dp[1] : dp[2]));
+                        hit[u] = maybe(__ldg(frec + p[u])) && k + u < tot;
+                    }
+                    RCPG_UNROLL
+                    for (std::uint32_t u = 0; u < U; ++u)
+                        if (hit[u]) list[listed++] = p[u];
+                    if (listed > static_cast<std::uint32_t>(US::list) - U) flush();
+                }
+            } else {
+                for (int r = 0; r < R; ++r) {
+                    const std::uint32_t* cs = row_cells(r);
+                    range(__ldg(cs + lo), __ldg(cs + hi));
+                }
             }
-        };
-        if (staged) particles(std::true_type{});
-        else particles(std::false_type{});
+            // the wrapped cells: the x-1 cell of a particle at x = 0, the
+            // x+1 cell of one at x = nc0-1
+            if (cx == 0 || cx == nc[0] - 1) {
+                const int wc = cx == 0 ? nc[0] - 1 : 0;
+                for (int r = 0; r < R; ++r) {
+                    const std::uint32_t* cs = row_cells(r);
+                    range(__ldg(cs + wc), __ldg(cs + wc + 1));
+                }
+            }
+            flush();
+            // the reference's capacity check counts the partners after q in
+            // its own order; a row that fits the capacity in full needs no count
+            const std::uint32_t cap = a.caps[q];
+            if (n > cap && n <= S) {
+                const std::uint32_t rq = a.ref_rank[q];
+                std::uint32_t n_half = 0;
+                for (std::uint32_t k = 0; k < n; ++k)
+                    n_half += a.ref_rank[a.nbr[static_cast<std::uint64_t>(k) * N + q]] > rq;
+                if (n_half > cap) report_cap_error(ctl, rq, cap);
+            }
+            need = max(need, n);
+            if (n > S) {
+                a.nbr_cnt[q] = 0u;  // overflow: empty row, rebuilt after the capacity grows
+                overflow = true;
+                continue;
+            }
+            a.nbr_cnt[q] = n;
+            if (!fuse) continue;
+            double f[ND];
+            up.force(f);
+            s_acc[0][col] = xadd(s_acc[0][col], static_cast<double>(up.sU));
+            s_acc[1][col] = xadd(s_acc[1][col], static_cast<double>(up.sLc));
+            s_acc[2][col] = xadd(s_acc[2][col], static_cast<double>(up.sdk));
+            s_acc[3][col] = xadd(s_acc[3][col], static_cast<double>(up.sFm));
+            s_acc[4][col] = fmax(s_acc[4][col], static_cast<double>(up.smax));
+            std::uint32_t wc = 0;
+            wall_forces<ND>(xq, up.Di, g, f, s_acc[0][col], s_acc[2][col], s_acc[3][col], wc);
+            s_accn[0][col] += up.scount + wc;
+            const double f2 = force_norm2<ND>(f);
+            if (f2 > 1.0E-16) {
+                s_acc[5][col] = xadd(s_acc[5][col], xsqrt(f2));
+                ++s_accn[1][col];
+            }
+            s_acc[6][col] = xadd(s_acc[6][col], up.Di);
+            RCPG_UNROLL
+            for (int d = 0; d < ND; ++d) a.F[static_cast<std::uint64_t>(q) * ND + d] = f[d];
+        }
     }
     if (overflow && fuse) ctl->forces_done = 0u;
     // block maximum of the row lengths, one atomic per block
@@ -1546,14 +1482,6 @@ __global__ void __launch_bounds__(UnitShape<ND>::threads, UnitShape<ND>::min_blo
         __syncthreads();
     }
     if (threadIdx.x == 0 && s_need) atomicMax(&ctl->row_need, s_need);
-}
-
-// dynamic shared memory of k_cells<ND, *>: the stage and the rows' cell_start slices
-template <int ND>
-constexpr std::size_t cells_smem_bytes() {
-    using US = UnitShape<ND>;
-    return static_cast<std::size_t>(US::stage) * 4 * sizeof(double) +
-           static_cast<std::size_t>(US::rows) * US::slice * sizeof(std::uint32_t);
 }
 
 // ===========================================================================
@@ -2319,28 +2247,23 @@ void adam_nd(const DevArrays& a, int do_adam, int do_refresh, cudaStream_t st) {
     k_adam_refresh<ND><<<need < g ? need : g, kForceBlock, 0, st>>>(a, do_adam, do_refresh);
 }
 
-// persistent force grid: at most the blocks resident at once (the block-sum
-// buffers hold at least force_blocks(N) entries)
-// persistent grid of the cell-unit search: the blocks resident at once (at
-// most 4096, the engine's block-sum entries)
+// persistent grid of the cell-unit search: UnitShape::blocks per SM (at most
+// 4096, the engine's block-sum entries)
 template <int ND, bool MX>
 void launch_cells_variant(const DevArrays& a, cudaStream_t st) {
     if constexpr (ND <= 3) {
         int dev = 0;
         cudaGetDevice(&dev);
-        constexpr std::size_t smem = cells_smem_bytes<ND>();
         constexpr int T = UnitShape<ND>::threads;
         static int grid[64] = {};
         if (dev >= 0 && dev < 64 && grid[dev] == 0) {
-            cudaFuncSetAttribute(k_cells<ND, MX>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-            int sms = 148, per_sm = 1;
+            int sms = 148;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cells<ND, MX>, T, smem);
-            const int gr = sms * (per_sm > 0 ? per_sm : 1);
+            const int gr = sms * UnitShape<ND>::blocks;
             grid[dev] = gr < 4096 ? gr : 4096;
         }
         const unsigned g = (dev >= 0 && dev < 64) ? static_cast<unsigned>(grid[dev]) : 148u;
-        k_cells<ND, MX><<<g, T, smem, st>>>(a);
+        k_cells<ND, MX><<<g, T, 0, st>>>(a);
     }
 }
 
