@@ -128,6 +128,7 @@ class Engine {
     bool step_host();
     bool advance_graph(std::uint64_t max_new_steps);
     void capture_graph();
+    int captured_steps() const;  // steps of the captured graph, a divisor of graph_steps_
     // one step of the step graph: gate, conditional build, pair-kernel switch,
     // controller, ADAM (kernels run only where the step needs them)
     void capture_step();
