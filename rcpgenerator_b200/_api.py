@@ -19,6 +19,7 @@ controller, reductions in the reference's one-thread order), and
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 from typing import Any, Callable
 
 import numpy as np
@@ -26,6 +27,9 @@ import numpy as np
 from . import _native as N
 
 _dp = C.POINTER(C.c_double)
+# result arrays come from malloc (rcpg_result_free gives them to free)
+_free = C.CDLL(None).free
+_free.argtypes, _free.restype = [C.c_void_p], None
 _i8p = C.POINTER(C.c_int8)
 
 _num_threads = 1
@@ -175,10 +179,24 @@ def _arr(ptr, n: int, dtype) -> np.ndarray:
     return np.ctypeslib.as_array(ptr, shape=(n,)).astype(dtype, copy=True)
 
 
+def _take_positions(r: N.Result, n: int, nd: int) -> np.ndarray:
+    """The positions of a result as an [n, nd] array that owns the C buffer
+    (the result no longer does): they are the largest array of a result, and
+    filling a fresh copy costs a page fault per 4 KB."""
+    if n == 0 or not r.positions:
+        return np.zeros((n, nd))
+    addr = C.cast(r.positions, C.c_void_p).value
+    buf = (C.c_double * (n * nd)).from_address(addr)
+    fin = weakref.finalize(buf, _free, addr)
+    fin.atexit = False  # an array may outlive the interpreter's exit handlers
+    r.positions = _dp()
+    return np.frombuffer(buf, dtype=np.float64).reshape(n, nd)
+
+
 def result_to_dict(r: N.Result, as_arrays: bool = False) -> dict:
     """PackingResult -> the reference's result dict (module.cpp:154-184)."""
     n, nd, s = int(r.N), int(r.ndim), int(r.steps)
-    pos = _arr(r.positions, n * nd, np.float64).reshape(n, nd)
+    pos = _take_positions(r, n, nd)
     out: dict[str, Any] = {
         "positions": pos,
         "diameters": _arr(r.diameters, n, np.float64),

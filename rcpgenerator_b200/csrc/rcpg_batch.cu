@@ -963,7 +963,8 @@ std::vector<std::uint32_t> run_group(const std::vector<EngineInput>& ins, const 
             const double D0 = pos[(off + i) * P + nd];
             R.diameters[i] = c.runtime_fix_diameter ? D0 : D0 * kd;
         }
-        R.particle_origin.assign(origin.begin() + off, origin.begin() + off + N);
+        R.particle_origin.resize(N);
+        std::copy_n(origin.begin() + off, N, R.particle_origin.data());
         R.box.assign(c.box, c.box + nd);
         R.walls = r.walls;
         const std::size_t n = c.hist_filled, h0 = inst[q].hist_off;

@@ -102,7 +102,9 @@ T* dup(const std::vector<T>& v) {
     return p;
 }
 
-rcpg_result* make_result(const rcpg::EngineResult& r, std::uint64_t N, int ndim,
+// The result's arrays; the large ones (positions, diameters, particle_origin)
+// move over.
+rcpg_result* make_result(rcpg::EngineResult&& r, std::uint64_t N, int ndim,
                          const std::vector<rcpg::TraceSample>* trace, bool with_positions,
                          std::uint64_t launches) {
     rcpg_result* out = static_cast<rcpg_result*>(std::calloc(1, sizeof(rcpg_result)));
@@ -113,8 +115,8 @@ rcpg_result* make_result(const rcpg::EngineResult& r, std::uint64_t N, int ndim,
     out->phi = r.phi;
     out->max_min_dist = r.max_min_dist;
     out->force_magnitude = r.force_magnitude;
-    out->positions = dup(r.positions);
-    out->diameters = dup(r.diameters);
+    out->positions = r.positions.release();
+    out->diameters = r.diameters.release();
     out->box = dup(r.box);
     out->walls = dup(r.walls);
     out->phi_history = dup(r.phi_history);
@@ -124,7 +126,7 @@ rcpg_result* make_result(const rcpg::EngineResult& r, std::uint64_t N, int ndim,
     out->mu_history = dup(r.mu_history);
     out->alpha_history = dup(r.alpha_history);
     out->mu_flag_history = dup(r.mu_flag_history);
-    out->particle_origin = dup(r.particle_origin);
+    out->particle_origin = r.particle_origin.release();
     out->pair_builds = r.builds;
     out->row_capacity = r.row_capacity;
     out->kernel_launches = launches;
@@ -233,10 +235,10 @@ int32_t rcpg_run_packing(const rcpg_packing_input* in, const rcpg_run_options* o
     *out = nullptr;
     try {
         // argument errors first (they need no GPU), then the device
-        const rcpg::EngineInput ei = make_input(in, opt);
+        rcpg::EngineInput ei = make_input(in, opt);
         rcpg::check_run_input(ei);
         if (!have_device(err, errlen)) return RCPG_ECUDA;
-        rcpg::Engine eng(ei);
+        rcpg::Engine eng(std::move(ei));
         std::vector<rcpg::TraceSample> trace;
         rcpg::ObserverFn fn;
         if (observer) {
@@ -246,8 +248,8 @@ int32_t rcpg_run_packing(const rcpg_packing_input* in, const rcpg_run_options* o
             };
         }
         eng.run(progress_interval, capture_positions != 0, trajectory_interval, fn, &trace);
-        const rcpg::EngineResult r = eng.result();
-        *out = make_result(r, eng.N(), eng.ndim(), &trace, capture_positions != 0, eng.launches());
+        rcpg::EngineResult r = eng.result();
+        *out = make_result(std::move(r), eng.N(), eng.ndim(), &trace, capture_positions != 0, eng.launches());
         return RCPG_OK;
     } catch (const std::exception& e) {
         return fail(err, errlen, classify(e), e.what());
@@ -325,13 +327,13 @@ int32_t run_batch_impl(const rcpg_packing_input* inputs, uint64_t count, const r
                 std::vector<rcpg::EngineInput> ins;
                 ins.reserve(persistent.size());
                 for (uint64_t k : persistent) ins.push_back(input_of(k));
-                const std::vector<rcpg::BatchOutcome> res =
+                std::vector<rcpg::BatchOutcome> res =
                     rcpg::run_batch_persistent(ins, 2048u, on_streams.empty() ? 0 : 1);
                 for (std::size_t q = 0; q < persistent.size(); ++q) {
                     const uint64_t k = persistent[q];
-                    const rcpg::BatchOutcome& b = res[q];
+                    rcpg::BatchOutcome& b = res[q];
                     if (b.code == 0) {
-                        results[k] = make_result(b.result, b.N, b.ndim, nullptr, false, 0);
+                        results[k] = make_result(std::move(b.result), b.N, b.ndim, nullptr, false, 0);
                     } else {
                         record(k, b.code == -22 ? RCPG_EINVAL : (b.code == -2 ? RCPG_ECUDA : RCPG_ERUNTIME),
                                b.message);
@@ -363,8 +365,8 @@ int32_t run_batch_impl(const rcpg_packing_input* inputs, uint64_t count, const r
                 rcpg::Engine eng(input_of(k), st);
                 eng.set_blocking_sync(true);  // many host threads: sleep while the GPU works
                 eng.run(0, false, 0, rcpg::ObserverFn(), nullptr);
-                const rcpg::EngineResult r = eng.result();
-                results[k] = make_result(r, eng.N(), eng.ndim(), nullptr, false, eng.launches());
+                rcpg::EngineResult r = eng.result();
+                results[k] = make_result(std::move(r), eng.N(), eng.ndim(), nullptr, false, eng.launches());
             } catch (const std::exception& e) {
                 record(k, classify(e), e.what());
             }
@@ -459,8 +461,8 @@ uint64_t rcpg_engine_kernel_launches(const rcpg_engine* e) { return e ? e->eng->
 int32_t rcpg_engine_result(rcpg_engine* e, rcpg_result** out, char* err, size_t errlen) {
     if (!e || !out) return fail(err, errlen, RCPG_EINVAL, "rcpgenerator_b200: null argument");
     try {
-        const rcpg::EngineResult r = e->eng->result();
-        *out = make_result(r, e->eng->N(), e->eng->ndim(), nullptr, false, e->eng->launches());
+        rcpg::EngineResult r = e->eng->result();
+        *out = make_result(std::move(r), e->eng->N(), e->eng->ndim(), nullptr, false, e->eng->launches());
         return RCPG_OK;
     } catch (const std::exception& ex) {
         return fail(err, errlen, classify(ex), ex.what());

@@ -227,6 +227,12 @@ void launch_fix_height(const DevArrays& a, cudaStream_t st);
 
 void launch_pack(std::uint64_t N, int ndim, const double* x, const double* D, double* pos,
                  cudaStream_t st);
+// origin[i] = i and (optional) rank[i] = i
+void launch_identity(std::uint64_t N, std::uint64_t* origin, std::uint32_t* rank, cudaStream_t st);
+// The state in the reference's order: x [N*ndim], D = D0 * kd (D0 when fixed)
+// [N], origin [N].
+void launch_collect(const DevArrays& a, double kd, bool fixed, double* x, double* D, std::uint64_t* origin,
+                    cudaStream_t st);
 void launch_unpack(std::uint64_t N, int ndim, const double* pos, double* x, cudaStream_t st);
 void launch_refresh_arrays(std::uint64_t N, int ndim, const double* x, double* x_last,
                            const double* D, double* D_last, double* theta, double theta_new,

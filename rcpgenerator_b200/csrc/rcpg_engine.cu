@@ -124,7 +124,7 @@ void Engine::check(cudaError_t e, const char* what) {
 // ---------------------------------------------------------------------------
 // setup (ENG:4353-4990), shared with the host emulation (rcpg_setup.cpp)
 // ---------------------------------------------------------------------------
-void Engine::setup_host(const EngineInput& in) {
+void Engine::setup_host(EngineInput in) {
     // the target-phi lock rescales every diameter on the host, so runs that
     // can lock are host-controlled
     exact_ = in.exact || in.has_target_phi;
@@ -132,7 +132,7 @@ void Engine::setup_host(const EngineInput& in) {
     mixed_switch_ = in.mixed_switch;
     graph_steps_ = in.graph_steps > 0 ? in.graph_steps : 32;
     device_ = in.device;
-    RunSetup s = prepare_run(in);
+    RunSetup s = prepare_run(std::move(in));
     N_ = s.N;
     ndim_ = s.ndim;
     host_c_ = s.c;
@@ -350,22 +350,15 @@ void Engine::publish_step_params() {
 void Engine::upload_initial() {
     const std::uint64_t N = N_;
     const int nd = ndim_;
-    std::vector<double> pos(N * P_, 0.0);
-    for (std::uint64_t i = 0; i < N; ++i) {
-        for (int d = 0; d < nd; ++d) pos[i * P_ + d] = x0_[i * nd + d];
-        pos[i * P_ + nd] = D0_[i];
-    }
-    std::vector<std::uint64_t> origin(N);
-    std::iota(origin.begin(), origin.end(), 0ull);
-    check(cudaMemcpyAsync(a_.pos, pos.data(), pos.size() * 8, cudaMemcpyHostToDevice, st_), "H2D pos");
-    check(cudaMemcpyAsync(a_.origin, origin.data(), N * 8, cudaMemcpyHostToDevice, st_), "H2D origin");
+    // positions and diameters go up as they are, through scratch that only the
+    // reorder and its sort use; the records and the initial order are made there
+    double* D_up = reinterpret_cast<double*>(a_.sort_keys[0]);
+    check(cudaMemcpyAsync(a_.vec_tmp, x0_.data(), N * nd * 8, cudaMemcpyHostToDevice, st_), "H2D positions");
+    check(cudaMemcpyAsync(D_up, D0_.data(), N * 8, cudaMemcpyHostToDevice, st_), "H2D diameters");
     check(cudaMemcpyAsync(a_.caps, caps_.data(), N * 4, cudaMemcpyHostToDevice, st_), "H2D caps");
-    std::vector<std::uint32_t> rank;
-    if (a_.permute) {
-        rank.resize(N);
-        std::iota(rank.begin(), rank.end(), 0u);
-        check(cudaMemcpyAsync(a_.ref_rank, rank.data(), N * 4, cudaMemcpyHostToDevice, st_), "H2D rank");
-    }
+    launch_pack(N, nd, a_.vec_tmp, D_up, a_.pos, st_);
+    launch_identity(N, a_.origin, a_.permute ? a_.ref_rank : nullptr, st_);
+    launches_ += 2;
     check(cudaMemsetAsync(a_.m, 0, N * nd * 8, st_), "memset m");
     check(cudaMemsetAsync(a_.v, 0, N * nd * 8, st_), "memset v");
     check(cudaMemsetAsync(a_.F, 0, N * nd * 8, st_), "memset F");
@@ -434,9 +427,9 @@ void Engine::upload_initial() {
     push_ctl();
 }
 
-Engine::Engine(const EngineInput& in, cudaStream_t stream) {
-    setup_host(in);
-    check(cudaSetDevice(in.device), "cudaSetDevice");
+Engine::Engine(EngineInput in, cudaStream_t stream) {
+    setup_host(std::move(in));
+    check(cudaSetDevice(device_), "cudaSetDevice");
     if (stream) {
         st_ = stream;
     } else {
@@ -1023,33 +1016,19 @@ void Engine::download_histories() {
     }
 }
 
-void Engine::download_particles(std::vector<double>& pos, std::vector<std::uint64_t>* origin) {
+void Engine::download_particles(double kd, bool fixed, double* x, double* D, std::uint64_t* origin) {
+    // ordered and scaled on the GPU into scratch that only the reorder and its
+    // sort use, then three copies straight to their place: at N = 1e6 (2D) the
+    // scatter into the reference's order and the copies of it took 48 ms on the host
     const std::uint64_t N = N_;
-    pos.resize(N * P_);
-    if (origin) origin->resize(N);
-    if (!a_.permute) {
-        check(cudaMemcpyAsync(pos.data(), a_.pos, pos.size() * 8, cudaMemcpyDeviceToHost, st_), "D2H pos");
-        if (origin)
-            check(cudaMemcpyAsync(origin->data(), a_.origin, N * 8, cudaMemcpyDeviceToHost, st_), "D2H origin");
-        check(cudaStreamSynchronize(st_), "sync");
-        return;
-    }
-    // cell-order storage: the current buffer set, then particle q goes to its
-    // reference index ref_rank[q]
-    pull_ctl();
-    const DevArrays cur = bound_arrays(a_, hctl_.buf);
-    std::vector<double> cell(N * P_);
-    std::vector<std::uint64_t> org(origin ? N : 0);
-    std::vector<std::uint32_t> rank(N);
-    check(cudaMemcpyAsync(cell.data(), cur.pos, cell.size() * 8, cudaMemcpyDeviceToHost, st_), "D2H pos");
-    check(cudaMemcpyAsync(rank.data(), cur.ref_rank, N * 4, cudaMemcpyDeviceToHost, st_), "D2H rank");
-    if (origin) check(cudaMemcpyAsync(org.data(), cur.origin, N * 8, cudaMemcpyDeviceToHost, st_), "D2H origin");
+    double* D_out = reinterpret_cast<double*>(a_.sort_keys[0]);
+    launch_collect(a_, kd, fixed, a_.vec_tmp, D_out, a_.sort_keys[1], st_);
+    ++launches_;
+    check(cudaGetLastError(), "collect");
+    check(cudaMemcpyAsync(x, a_.vec_tmp, N * ndim_ * 8, cudaMemcpyDeviceToHost, st_), "D2H positions");
+    check(cudaMemcpyAsync(D, D_out, N * 8, cudaMemcpyDeviceToHost, st_), "D2H diameters");
+    if (origin) check(cudaMemcpyAsync(origin, a_.sort_keys[1], N * 8, cudaMemcpyDeviceToHost, st_), "D2H origin");
     check(cudaStreamSynchronize(st_), "sync");
-    for (std::uint64_t q = 0; q < N; ++q) {
-        const std::uint64_t r = rank[q];
-        for (int k = 0; k < P_; ++k) pos[r * P_ + k] = cell[q * P_ + k];
-        if (origin) (*origin)[r] = org[q];
-    }
 }
 
 EngineResult Engine::result() {
@@ -1070,16 +1049,12 @@ EngineResult Engine::result() {
     const std::uint64_t N = N_;
     const int nd = ndim_;
     EngineResult r;
-    std::vector<double> pos;
-    download_particles(pos, &r.particle_origin);
     r.positions.resize(N * nd);
     r.diameters.resize(N);
+    r.particle_origin.resize(N);
     // diameters of the last diameter update: D = D0*kappa (ENG:5733)
-    const double kd = c.runtime_fix_diameter ? 1.0 : c.kappa_D;
-    for (std::uint64_t i = 0; i < N; ++i) {
-        for (int d = 0; d < nd; ++d) r.positions[i * nd + d] = pos[i * P_ + d];
-        r.diameters[i] = c.runtime_fix_diameter ? pos[i * P_ + nd] : pos[i * P_ + nd] * kd;
-    }
+    download_particles(c.kappa_D, c.runtime_fix_diameter != 0, r.positions.data(), r.diameters.data(),
+                       r.particle_origin.data());
     r.box.assign(c.box, c.box + nd);
     r.walls = walls_;
     download_histories();
@@ -1181,8 +1156,6 @@ void Engine::observe(std::uint64_t step, bool capture, const ObserverFn& observe
             adam_pending_ = false;
             hctl_.adam_go = 0u;
         }
-        std::vector<double> pos;
-        download_particles(pos, nullptr);
         xs.resize(N_ * ndim_);
         TraceSample ts;
         ts.step = step;
@@ -1193,10 +1166,7 @@ void Engine::observe(std::uint64_t step, bool capture, const ObserverFn& observe
             kd = hctl_.c.kappa_D_prev;
         }
         if (host_c_.runtime_fix_diameter) kd = 1.0;
-        for (std::uint64_t i = 0; i < N_; ++i) {
-            for (int d = 0; d < ndim_; ++d) xs[i * ndim_ + d] = pos[i * P_ + d];
-            ts.diameters[i] = pos[i * P_ + ndim_] * kd;
-        }
+        download_particles(kd, false, xs.data(), ts.diameters.data(), nullptr);
         ts.positions = xs;
         ts.phi = ob.phi;
         ts.force = ob.force_magnitude;
@@ -1240,8 +1210,8 @@ void Engine::run(std::uint64_t progress_interval, bool capture_positions,
         if (trace && capture_positions) {
             TraceSample ts;
             ts.step = last;
-            ts.positions = r.positions;
-            ts.diameters = r.diameters;
+            ts.positions.assign(r.positions.begin(), r.positions.end());
+            ts.diameters.assign(r.diameters.begin(), r.diameters.end());
             ts.phi = r.phi;
             ts.force = r.force_magnitude;
             ts.energy = host_c_.U;
@@ -1250,7 +1220,8 @@ void Engine::run(std::uint64_t progress_interval, bool capture_positions,
         }
         if (observer) {
             Observation ob{last, r.phi, r.force_magnitude, host_c_.U, r.max_min_dist};
-            observer(ob, capture_positions ? &r.positions : nullptr);
+            const std::vector<double> xs(r.positions.begin(), capture_positions ? r.positions.end() : r.positions.begin());
+            observer(ob, capture_positions ? &xs : nullptr);
         }
     }
 }

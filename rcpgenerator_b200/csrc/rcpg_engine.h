@@ -4,9 +4,12 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstdlib>
 #include <functional>
+#include <new>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "rcpg_device.h"
@@ -19,10 +22,49 @@ struct Observation {
     double phi, force_magnitude, energy, max_min_dist;
 };
 
+// A malloc'd array that a result can hand over (release) instead of copying.
+template <typename T>
+class HostArray {
+public:
+    HostArray() = default;
+    HostArray(HostArray&& o) noexcept : p_(o.p_), n_(o.n_) { o.p_ = nullptr; o.n_ = 0; }
+    HostArray& operator=(HostArray&& o) noexcept {
+        std::swap(p_, o.p_);
+        std::swap(n_, o.n_);
+        return *this;
+    }
+    ~HostArray() { std::free(p_); }
+    // n elements, not initialised
+    void resize(std::size_t n) {
+        std::free(p_);
+        n_ = 0;
+        p_ = static_cast<T*>(std::malloc(n * sizeof(T) + 1));
+        if (!p_) throw std::bad_alloc();
+        n_ = n;
+    }
+    T* data() { return p_; }
+    const T* data() const { return p_; }
+    std::size_t size() const { return n_; }
+    T& operator[](std::size_t i) { return p_[i]; }
+    const T* begin() const { return p_; }
+    const T* end() const { return p_ + n_; }
+    // the array, to be freed with std::free()
+    T* release() {
+        T* p = p_;
+        p_ = nullptr;
+        n_ = 0;
+        return p;
+    }
+
+private:
+    T* p_ = nullptr;
+    std::size_t n_ = 0;
+};
+
 // PackingResult (rcp_generator.hpp:35-90) minus the research-only fields.
 struct EngineResult {
-    std::vector<double> positions;  // [N*ndim]
-    std::vector<double> diameters;
+    HostArray<double> positions;  // [N*ndim]
+    HostArray<double> diameters;
     std::vector<double> box;
     std::vector<std::int8_t> walls;
     std::vector<double> phi_history, force_history, energy_history, max_overlap_history,
@@ -30,7 +72,7 @@ struct EngineResult {
     std::vector<std::int8_t> mu_flag_history;
     std::uint64_t steps = 0;
     double phi = 0.0, max_min_dist = 0.0, force_magnitude = 0.0;
-    std::vector<std::uint64_t> particle_origin;
+    HostArray<std::uint64_t> particle_origin;
     // engine statistics
     std::uint64_t builds = 0;
     std::uint32_t row_capacity = 0;
@@ -73,7 +115,7 @@ class EngineError : public std::runtime_error {
 
 class Engine {
    public:
-    explicit Engine(const EngineInput& in, cudaStream_t stream = nullptr);
+    explicit Engine(EngineInput in, cudaStream_t stream = nullptr);
     ~Engine();
     Engine(const Engine&) = delete;
     Engine& operator=(const Engine&) = delete;
@@ -113,7 +155,7 @@ class Engine {
     void set_blocking_sync(bool on);
 
    private:
-    void setup_host(const EngineInput& in);
+    void setup_host(EngineInput in);
     void alloc_device();
     void free_device();
     void upload_initial();
@@ -141,9 +183,9 @@ class Engine {
     void observe(std::uint64_t step, bool capture, const ObserverFn& observer,
                  std::vector<TraceSample>* trace);
     void download_histories();
-    // particle records [N*P] and particle_origin (optional) of the current
-    // state in the reference's order (graph mode stores them in cell order)
-    void download_particles(std::vector<double>& pos, std::vector<std::uint64_t>* origin);
+    // the current state in the reference's order: x [N*ndim], diameters D0 * kd
+    // (D0 when fixed) [N], particle_origin [N] (optional)
+    void download_particles(double kd, bool fixed, double* x, double* D, std::uint64_t* origin);
     void check(cudaError_t e, const char* what);
 
     // configuration

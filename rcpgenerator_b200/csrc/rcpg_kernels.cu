@@ -2147,6 +2147,32 @@ __global__ void k_unpack(std::uint64_t N, const double* __restrict__ pos, double
     for (int d = 0; d < ND; ++d) x[i * ND + d] = xi[d];
 }
 
+// Initial order of a run: origin (and, with cell-order storage, the reference
+// rank) of particle i is i.
+__global__ void k_identity(std::uint64_t N, std::uint64_t* __restrict__ origin, std::uint32_t* __restrict__ rank) {
+    const std::uint64_t i = blockIdx.x * static_cast<std::uint64_t>(blockDim.x) + threadIdx.x;
+    if (i >= N) return;
+    origin[i] = i;
+    if (rank) rank[i] = static_cast<std::uint32_t>(i);
+}
+
+// The state in the reference's order, as a result returns it: positions,
+// diameters D0 * kd (D0 itself when the diameters are fixed), particle_origin.
+template <int ND>
+__global__ void k_collect(DevArrays a, double kd, int fixed, double* __restrict__ x_out, double* __restrict__ D_out,
+                          std::uint64_t* __restrict__ origin_out) {
+    const std::uint64_t q = blockIdx.x * static_cast<std::uint64_t>(blockDim.x) + threadIdx.x;
+    if (q >= a.N) return;
+    bind_buffers(a);
+    double x[ND], D0;
+    load_pos<ND>(a.pos, q, x, D0);
+    const std::uint64_t r = a.permute ? a.ref_rank[q] : q;
+    RCPG_UNROLL
+    for (int d = 0; d < ND; ++d) x_out[r * ND + d] = x[d];
+    D_out[r] = fixed ? D0 : xmul(D0, kd);
+    origin_out[r] = a.origin[q];
+}
+
 // Per-particle anchors, as the reference keeps them (ENG:6104-6145).
 template <int ND>
 __global__ void k_refresh_arrays(std::uint64_t N, const double* __restrict__ x, double* x_last,
@@ -2486,6 +2512,15 @@ void launch_pack(std::uint64_t N, int ndim, const double* x, const double* D, do
                  cudaStream_t st) {
     const unsigned nb = force_blocks(N);
     RCPG_DISPATCH_ND(ndim, (k_pack<ND><<<nb, kForceBlock, 0, st>>>(N, x, D, pos)));
+}
+
+void launch_identity(std::uint64_t N, std::uint64_t* origin, std::uint32_t* rank, cudaStream_t st) {
+    k_identity<<<force_blocks(N), kForceBlock, 0, st>>>(N, origin, rank);
+}
+
+void launch_collect(const DevArrays& a, double kd, bool fixed, double* x, double* D, std::uint64_t* origin,
+                    cudaStream_t st) {
+    RCPG_DISPATCH_ND(a.ndim, (k_collect<ND><<<force_blocks(a.N), kForceBlock, 0, st>>>(a, kd, fixed ? 1 : 0, x, D, origin)));
 }
 
 void launch_unpack(std::uint64_t N, int ndim, const double* pos, double* x, cudaStream_t st) {

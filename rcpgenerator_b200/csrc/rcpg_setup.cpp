@@ -101,7 +101,45 @@ void check_run_input(const EngineInput& in) {
         throw std::runtime_error("Error: --walls expects Ndim entries");
 }
 
-RunSetup prepare_run(const EngineInput& in) {
+namespace {
+
+// The element that std::nth_element puts at rank n/2, without its passes over
+// the whole array: two values of a sorted sample bracket the rank, one pass
+// counts what lies below them and keeps what lies between, and nth_element
+// runs on that. Too few elements, or a bracket that missed (or values that do
+// not order): nth_element on a copy. 1e6 diameters: 10 -> 2 ms.
+double median_of(const std::vector<double>& v) {
+    constexpr std::size_t kSample = 4096, kMargin = 160;  // 5 sigma of the sampled rank (sigma <= 32)
+    const std::size_t n = v.size(), rank = n / 2;
+    if (n >= 16 * kSample) {
+        std::vector<double> s(kSample);
+        for (std::size_t i = 0; i < kSample; ++i) s[i] = v[i * (n / kSample)];
+        std::sort(s.begin(), s.end());
+        const double lo = s[kSample / 2 - kMargin], hi = s[kSample / 2 + kMargin];
+        std::size_t below = 0, above = 0, inside = 0;
+        std::vector<double> mid;
+        mid.reserve(n / 8);
+        for (double x : v) {
+            below += x < lo;
+            above += x > hi;
+            if (!(x >= lo && x <= hi)) continue;
+            ++inside;
+            if (lo < hi) mid.push_back(x);
+        }
+        if (below <= rank && rank < below + inside && below + inside + above == n) {
+            if (lo == hi) return lo;
+            std::nth_element(mid.begin(), mid.begin() + (rank - below), mid.end());
+            return mid[rank - below];
+        }
+    }
+    std::vector<double> s = v;
+    std::nth_element(s.begin(), s.begin() + rank, s.end());
+    return s[rank];
+}
+
+}  // namespace
+
+RunSetup prepare_run(EngineInput in) {
     RunSetup out;
     if (in.N == 0) throw std::invalid_argument("rcpgenerator_b200: no particles");
     if (in.ndim < 2 || in.ndim > kMaxDim)
@@ -110,10 +148,9 @@ RunSetup prepare_run(const EngineInput& in) {
     const std::size_t N = in.N, nd = static_cast<std::size_t>(in.ndim);
     out.N = in.N;
     out.ndim = in.ndim;
-    std::vector<double> x = in.positions;
-    std::vector<double> D = in.diameters;
-    if (x.size() != N * nd || D.size() != N)
-        throw std::invalid_argument("rcpgenerator_b200: positions/diameters size mismatch");
+    check_run_input(in);
+    std::vector<double> x = std::move(in.positions);
+    std::vector<double> D = std::move(in.diameters);
 
     // refresh-trigger scale from the caller's diameters (ENG:4401-4430)
     double trigger_scale;
@@ -124,16 +161,13 @@ RunSetup prepare_run(const EngineInput& in) {
             if (dv > dmx) dmx = dv;
             if (dv < dmn) dmn = dv;
         }
-        std::vector<double> Ds = D;
-        std::nth_element(Ds.begin(), Ds.begin() + Ds.size() / 2, Ds.end());
-        const double med = Ds[Ds.size() / 2];
+        const double med = median_of(D);
         med_in = med;
         const double t_shell = std::min(std::max(med * 1.02, dmn * 2.25), dmx) * 0.5;
         const double rho = t_shell / dmn;
         trigger_scale = std::min(1.28 * rho, 1.9);
     }
 
-    check_run_input(in);
     std::vector<double> box = in.box;
     std::vector<std::int8_t> walls = in.walls;
     if (box.empty()) box.assign(nd, 1.0);
@@ -169,11 +203,21 @@ RunSetup prepare_run(const EngineInput& in) {
     const double coeff = std::pow(kPi, nd / 2.0) / std::tgamma(nd / 2.0 + 1.0);
     std::vector<double> terms(N);
     parallel_for(N, [&](std::size_t i) { terms[i] = coeff * std::pow(D[i] / 2.0, static_cast<double>(nd)); });
+    // D0 statistics (ENG:4800-4838) in the same pass: each sum in index order,
+    // the chains side by side
     double current_volume = 0.0;
-    for (double v : terms) current_volume += v;
+    double D0min = D[0], S = 0.0, D0max = 0.0;
+    for (std::size_t i = 0; i < N; ++i) {
+        current_volume += terms[i];
+        if (D[i] < D0min) D0min = D[i];
+        double r = D[i] * 0.5, rN = 1.0;
+        for (std::size_t k = 0; k < nd; ++k) rN *= r;
+        S += rN;
+        if (D[i] > D0max) D0max = D[i];
+    }
     double box_volume = std::accumulate(box.begin(), box.end(), 1.0, std::multiplies<double>());
     phi = current_volume / box_volume / phi_modifier;
-    const double Dmin = *std::min_element(D.begin(), D.end());
+    const double Dmin = D0min;
 
     std::uint32_t neighbor_max = in.neighbor_max;
     if (neighbor_max == 0) {
@@ -207,17 +251,7 @@ RunSetup prepare_run(const EngineInput& in) {
     if (nd == 4) alpha = alpha_max = 0.0035;
     if (nd >= 5) alpha = alpha_max = 0.0025;
 
-    // D0 statistics (ENG:4800-4838); D is not used after this point
     out.D0 = std::move(D);
-    const std::vector<double>& D0_ = out.D0;
-    double D0min = D0_[0], S = 0.0, D0max = 0.0;
-    for (std::size_t i = 0; i < N; ++i) {
-        if (D0_[i] < D0min) D0min = D0_[i];
-        double r = D0_[i] * 0.5, rN = 1.0;
-        for (std::size_t k = 0; k < nd; ++k) rN *= r;
-        S += rN;
-        if (D0_[i] > D0max) D0max = D0_[i];
-    }
     // the median of D0 = D * factor: a positive scale keeps every rank, and
     // the element at rank N/2 was scaled by the same rounded multiplication
     const double D0med = in.fix_diameter ? med_in : med_in * factor;
