@@ -579,7 +579,7 @@ __device__ void b_controller(const View& V, Shared& sh, const ForceSums& s, int 
             }
         }
         ctl->c = c;
-        if (sh.publish) publish_step(ctl, c, ndim);
+        if (sh.publish) publish_step(ctl, c, ndim, ctl->g.box, ctl->kappa_min);
     }
     __syncthreads();
 }
@@ -615,7 +615,7 @@ __device__ void b_after_stop(const View& V, Shared& sh) {
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        publish_step(ctl, ctl->c, ND);
+        publish_step(ctl, ctl->c, ND, ctl->g.box, ctl->kappa_min);
         ctl->adam_go = 0u;
         ctl->stopped = 0u;
         ctl->halted = 0u;

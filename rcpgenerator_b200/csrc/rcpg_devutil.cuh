@@ -176,10 +176,11 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T* smem, T& total) {
 }
 
 // Parameters of the kernels of the step that begin_step() just opened.
-__device__ __forceinline__ void publish_step(DevCtl* ctl, const Controller& c, int ndim) {
+__device__ __forceinline__ void publish_step(DevCtl* ctl, const Controller& c, int ndim, const double* box_now,
+                                             double kappa_min_now) {
     ctl->forces_done = 0u;
     for (int d = 0; d < ndim; ++d) {
-        if (ctl->g.box[d] != c.box[d]) {  // fix_height only: a division saved in every other step
+        if (box_now[d] != c.box[d]) {  // fix_height only: a division saved in every other step
             ctl->g.box[d] = c.box[d];
             ctl->g.inv_box[d] = 1.0 / c.box[d];
         }
@@ -195,7 +196,7 @@ __device__ __forceinline__ void publish_step(DevCtl* ctl, const Controller& c, i
         ctl->rebuild_flag = 1u;
     } else {
         ctl->rebuild_flag = 0u;
-        ctl->kappa_min = fmin(ctl->kappa_min, c.kappa_D);
+        ctl->kappa_min = fmin(kappa_min_now, c.kappa_D);
     }
 }
 

@@ -1814,56 +1814,84 @@ __global__ void __launch_bounds__(kCtlThreads) k_reduce_fast(DevArrays a) {
 // Graph-mode controller: reduce, finish step s (end_step), open step s+1
 // (begin_step) and publish the parameters of the kernels that follow. With
 // open_only it just opens the next step (the first step of a run).
-__global__ void __launch_bounds__(kCtlThreads) k_controller(DevArrays a, int open_only) {
+//
+// One block on the critical path of every step, bound by the latency of serial
+// FP64 (a pow is about 1,000 cycles in one thread, a division 129) and of the
+// loads ahead of it. So every load that needs no other one is issued at once;
+// warps 8-10 prepare the powers and the exponential of the schedule while
+// warps 0-7 reduce; warp 11 finishes the reported scalars beside thread 0.
+// A step of 25,003 particles (2-D, walls): 48.8 us with everything in thread
+// 0, 45.1 us so.
+constexpr int kCtlBlock = kCtlThreads + 128;
+constexpr int kCtlReport = kCtlThreads + 96;  // the thread of the reported scalars
+
+__global__ void __launch_bounds__(kCtlBlock) k_controller(DevArrays a, int open_only) {
     __shared__ ForceSums red[kCtlThreads / 32];
     __shared__ double s_hred[(kCtlThreads / 32) * 6];
     // the controller state is worked on in shared memory: one coalesced copy
     // in and out instead of a chain of dependent global loads in one thread
     __shared__ Controller cs;
     __shared__ HistStats s_stats;
+    __shared__ StepPre s_ahead;
+    __shared__ double s_box[kMaxDim];
     __shared__ int s_publish, s_go;
     DevCtl* ctl = a.ctl;
-    if (ctl_idle(ctl)) {
-        if (threadIdx.x == 0) ctl->adam_go = 0u;
-        return;
-    }
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     static_assert(sizeof(Controller) % 8 == 0, "controller copy by 8-byte words");
     constexpr int kWords = sizeof(Controller) / 8;
-    {
-        const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&ctl->c);
-        unsigned long long* dst = reinterpret_cast<unsigned long long*>(&cs);
-        for (int w = threadIdx.x; w < kWords; w += blockDim.x) dst[w] = src[w];
+    static_assert(kWords <= kCtlBlock, "one word per thread");
+    // one round trip for the flags, the state and the other control words
+    const unsigned long long word =
+        tid < kWords ? reinterpret_cast<const unsigned long long*>(&ctl->c)[tid] : 0ull;
+    const unsigned nb = open_only ? 0u : ctl->nsum_blocks;
+    const double box = tid < a.ndim ? ctl->g.box[tid] : 0.0;
+    const std::uint32_t row_need = ctl->row_need, cap_error = ctl->cap_error, pair_fp32 = ctl->pair_fp32;
+    const std::uint64_t steps = ctl->c.steps;
+    const double t_open = ctl->c.t;
+    const double force_mu = ctl->force_mu, mixed_switch = ctl->mixed_switch, kappa_min = ctl->kappa_min;
+    if (ctl_idle(ctl)) {
+        if (tid == 0) ctl->adam_go = 0u;
+        return;
     }
-    // the control words thread 0 needs, loaded before the reduction so that
-    // their latency overlaps it
-    std::uint32_t row_need = 0, cap_error = 0, pair_fp32 = 0;
-    double force_mu = 0.0, mixed_switch = 0.0;
-    if (threadIdx.x == 0) {
-        row_need = ctl->row_need;
-        cap_error = ctl->cap_error;
-        pair_fp32 = ctl->pair_fp32;
-        force_mu = ctl->force_mu;
-        mixed_switch = ctl->mixed_switch;
+    if (tid < kWords) reinterpret_cast<unsigned long long*>(&cs)[tid] = word;
+    if (tid < a.ndim) s_box[tid] = box;
+    if (tid < kCtlThreads) {
+        if (!open_only) {
+            ForceSums s;
+            sums_zero(s);
+            for (unsigned b = tid; b < nb; b += kCtlThreads) sums_add(s, a.block_sums[b]);
+            warp_reduce_sums(s);
+            if (lane == 0) red[warp] = s;
+        }
+    } else if (lane == 0) {
+        prepare_ahead(t_open, steps, a.hist, s_ahead, warp - kCtlThreads / 32);
     }
     __syncthreads();
+    // capacity problems of the last build stop the run before its results are used
+    const bool halt = !open_only && (row_need > a.S || cap_error);
     ForceSums s;
-    if (!open_only) reduce_blocks(a, red, s);
-    // 1. end of the finished step (thread 0)
-    if (threadIdx.x == 0) {
+    if (!open_only && (tid == 0 || tid == kCtlReport)) {
+        s = red[0];
+        RCPG_UNROLL
+        for (int w = 1; w < kCtlThreads / 32; ++w) sums_add(s, red[w]);
+    }
+    // 1. end of the finished step
+    if (tid == 0) {
         Controller& c = cs;
         s_publish = 0;
         bool go = true;
         if (!open_only) {
             ctl->sums = s;
-            // capacity problems of the last build stop the run before its results are used
-            if (row_need > a.S || cap_error) {
+            if (halt) {
                 ctl->halted = 1u;
                 ctl->adam_go = 0u;
                 go = false;
             } else {
-                const StepScalars sc = finalize_sums(s, force_mu, a.ndim);
-                ctl->scal = sc;
-                end_step(c, a.hist, sc);
+                StepScalars sc;
+                finalize_schedule(s, force_mu, sc);
+                ctl->scal.max_overlap = sc.max_overlap;
+                ctl->scal.dkappa = sc.dkappa;
+                end_step(c, a.hist, sc, &s_ahead);
                 // mixed precision: FP64 pair terms from the first step whose
                 // (nonzero) max overlap is below the switch, for the rest of the run
                 if (pair_fp32 && sc.max_overlap > 0.0 && sc.max_overlap < mixed_switch) {
@@ -1888,29 +1916,34 @@ __global__ void __launch_bounds__(kCtlThreads) k_controller(DevArrays a, int ope
             }
         }
         s_go = go ? 1 : 0;
+    } else if (tid == kCtlReport && !open_only && !halt) {
+        StepScalars sc;
+        finalize_report(s, a.ndim, sc);
+        ctl->scal.U = sc.U;
+        ctl->scal.Lc = sc.Lc;
+        ctl->scal.Fmean = sc.Fmean;
+        ctl->scal.mean_force = sc.mean_force;
+        ctl->scal.count = sc.count;
+        end_step_report(cs, a.hist, sc);
     }
     __syncthreads();
     // 2. the history windows the next step's schedule may read (the block)
     const std::uint64_t next = cs.steps + 1;
-    const bool stats = s_go && need_hist_stats(cs, a.hist, next);
+    const bool stats = s_go && need_hist_stats(cs, a.hist, next, &s_ahead);
     if (stats) hist_stats_block<kCtlThreads>(a.hist, next, s_stats, s_hred);
-    __syncthreads();
+    __syncthreads();  // also: every thread has read the state that begin_step changes
     // 3. top of the next step (thread 0)
-    if (threadIdx.x == 0 && s_go) {
+    if (tid == 0 && s_go) {
         Controller& c = cs;
-        begin_step(c, a.hist, next, stats ? &s_stats : nullptr);
+        begin_step(c, a.hist, next, stats ? &s_stats : nullptr, &s_ahead);
         // the stretch of a reorder step waits until after the reorder (ENG:5661 < :5758)
         ctl->fix_height_scale = c.reorder ? 1.0 : c.fix_height_scale;
         if (c.done || c.reorder || c.lock_now) ctl->stopped = 1u;
         else s_publish = 1;
     }
     __syncthreads();
-    {
-        const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&cs);
-        unsigned long long* dst = reinterpret_cast<unsigned long long*>(&ctl->c);
-        for (int w = threadIdx.x; w < kWords; w += blockDim.x) dst[w] = src[w];
-    }
-    if (threadIdx.x == 0 && s_publish) publish_step(ctl, cs, a.ndim);
+    if (tid < kWords) reinterpret_cast<unsigned long long*>(&ctl->c)[tid] = reinterpret_cast<const unsigned long long*>(&cs)[tid];
+    if (tid == 0 && s_publish) publish_step(ctl, cs, a.ndim, s_box, kappa_min);
 }
 
 // First node of a step in a captured step graph: plans and opens the build
@@ -2496,7 +2529,7 @@ void launch_reduce_fast(const DevArrays& a, cudaStream_t st) {
 }
 
 void launch_controller(const DevArrays& a, int open_only, cudaStream_t st) {
-    k_controller<<<1, kCtlThreads, 0, st>>>(a, open_only);
+    k_controller<<<1, kCtlBlock, 0, st>>>(a, open_only);
 }
 
 void launch_reorder(const DevArrays& a, cudaStream_t st) {

@@ -99,21 +99,6 @@ __device__ __forceinline__ unsigned long long bits_of(double v) {
     return static_cast<unsigned long long>(__double_as_longlong(v));
 }
 
-// StepPre of the step that is open now, each part by another warp (one lane).
-__device__ __forceinline__ void prepare_ahead(const Controller& c, const Histories& h, StepPre& p, int warp) {
-    if (warp == kSmallWarps - 1) {
-        p.pb1 = pow(0.9, c.t);
-        p.inv_b1 = xdiv(1.0, xsub(1.0, p.pb1));
-    } else if (warp == kSmallWarps - 2) {
-        p.pb2 = pow(0.999, c.t);
-        p.inv_b2 = xdiv(1.0, xsub(1.0, p.pb2));
-    } else if (warp == kSmallWarps - 3) {
-        const std::uint64_t step = c.steps + 1;
-        p.boost = exp(xdiv(-static_cast<double>(step), 350.0));
-        p.phi_250 = step > 251 ? h.phi[step - 250] : 0.0;
-    }
-}
-
 // The pair sums of this block's particles (row_pairs, with `lanes` threads per
 // particle and the same order of every sum): the force components, U, Lc, dk
 // and Fm in sh.terms, sh.maxov, sh.npair at [warp of the particle][field][lane].
@@ -283,7 +268,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
         sums_zero(sh.total);  // the wall terms join the pair sums: their own stay zero
     }
     __syncthreads();
-    if (lane == 0) prepare_ahead(ctl->c, a.hist, sh.ahead, warp);
+    if (lane == 0) prepare_ahead(ctl->c.t, ctl->c.steps, a.hist, sh.ahead, kSmallWarps - 1 - warp);
     if (ctl->stopped | ctl->halted) return;  // the same in every block
     cluster.sync();             // every block has read the control block and cleared its flags
     for (std::uint32_t it = 0; it < steps; ++it) {
@@ -547,7 +532,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
             begin_step(c, a.hist, c.steps + 1, sh.have_stats ? &sh.stats : nullptr, &sh.ahead);
             ctl->fix_height_scale = c.reorder ? 1.0 : c.fix_height_scale;
             if (c.done || c.reorder || c.lock_now) ctl->stopped = 1u;
-            else publish_step(ctl, c, ND);
+            else publish_step(ctl, c, ND, ctl->g.box, ctl->kappa_min);
         };
         const bool stretch = ctl->c.fix_height != 0;
         if (stretch) {
@@ -580,7 +565,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(DevArrays a, s
             trig = refresh_trigger(d2, xmul(D0i, ctl->refresh_kappa), xmul(D0i, ctl->kappa_min), ctl->theta);
         }
         // meanwhile, the parts of the next step's schedule that are known now
-        if (lane == 0) prepare_ahead(ctl->c, a.hist, sh.ahead, warp);
+        if (lane == 0) prepare_ahead(ctl->c.t, ctl->c.steps, a.hist, sh.ahead, kSmallWarps - 1 - warp);
         const std::uint32_t par = it & 1u;
         if (__syncthreads_or(trig) && static_cast<std::uint32_t>(tid) < C)
             *cluster.map_shared_rank(&sh.trigger[par], tid) = 1u;

@@ -727,6 +727,21 @@ __device__ __forceinline__ void row_pairs(const DevArrays& a, std::uint64_t t, s
 // whole block: sums in a fixed tree (graph mode; the host sums in order).
 constexpr int kCtlThreads = 256;
 
+// StepPre of the open step (time t, number steps), parts 0..2 by one thread each.
+__device__ __forceinline__ void prepare_ahead(double t, std::uint64_t steps, const Histories& h, StepPre& p, int part) {
+    if (part == 0) {
+        p.pb1 = pow(0.9, t);
+        p.inv_b1 = xdiv(1.0, xsub(1.0, p.pb1));
+    } else if (part == 1) {
+        p.pb2 = pow(0.999, t);
+        p.inv_b2 = xdiv(1.0, xsub(1.0, p.pb2));
+    } else if (part == 2) {
+        const std::uint64_t step = steps + 1;
+        p.boost = exp(xdiv(-static_cast<double>(step), 350.0));
+        p.phi_250 = step > 251 ? h.phi[step - 250] : 0.0;
+    }
+}
+
 // Whether begin_step(step) may read window statistics: the phi range while mu
 // decays or the final oscillation phase waits for its tick, the force means
 // where the learning-rate rule's other conditions hold (they read no windows).
