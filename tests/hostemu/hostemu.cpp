@@ -312,3 +312,15 @@ extern "C" int hostemu_noalloc_plan(std::uint64_t N, int ndim, std::uint32_t row
     out[16] = kNoAllocScratchBytes;
     return p.ok ? 1 : 0;
 }
+
+// The median of the caller's diameters as the run set-up takes it (2-D, fixed diameters).
+extern "C" double hostemu_setup_median(std::uint64_t N, const double* diameters) {
+    EngineInput in;
+    in.N = N;
+    in.ndim = 2;
+    in.positions.assign(2 * N, 0.5);
+    in.diameters.assign(diameters, diameters + N);
+    in.fix_diameter = true;
+    in.max_steps = 1;
+    return prepare_run(std::move(in)).c.D0_med;
+}
