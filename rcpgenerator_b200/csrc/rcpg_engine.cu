@@ -1022,9 +1022,16 @@ void Engine::download_particles(double kd, bool fixed, double* x, double* D, std
     // scatter into the reference's order and the copies of it took 48 ms on the host
     const std::uint64_t N = N_;
     double* D_out = reinterpret_cast<double*>(a_.sort_keys[0]);
+    // a launch, unlike the copies, needs the engine's device current; a result
+    // may be read from any thread
+    int current = device_;
+    check(cudaGetDevice(&current), "cudaGetDevice");
+    if (current != device_) check(cudaSetDevice(device_), "cudaSetDevice");
     launch_collect(a_, kd, fixed, a_.vec_tmp, D_out, a_.sort_keys[1], st_);
+    const cudaError_t launched = cudaGetLastError();
+    if (current != device_) check(cudaSetDevice(current), "cudaSetDevice");
     ++launches_;
-    check(cudaGetLastError(), "collect");
+    check(launched, "collect");
     check(cudaMemcpyAsync(x, a_.vec_tmp, N * ndim_ * 8, cudaMemcpyDeviceToHost, st_), "D2H positions");
     check(cudaMemcpyAsync(D, D_out, N * 8, cudaMemcpyDeviceToHost, st_), "D2H diameters");
     if (origin) check(cudaMemcpyAsync(origin, a_.sort_keys[1], N * 8, cudaMemcpyDeviceToHost, st_), "D2H origin");
