@@ -40,12 +40,15 @@ struct OvGrid {
     int periodic;
     int ncell[kOvMaxDim];
     double lo[kOvMaxDim], width[kOvMaxDim], box[kOvMaxDim];
-    double rq;  // candidate radius 2 R_max
+    double near[kOvMaxDim];  // up to this difference a pair needs no image; -1: every pair takes the quotient
+    double rq;               // candidate radius 2 R_max
 };
 
 // |x_i - x_j|^2 with the image removed, in the operation order of the
 // reference's NumPy expression (no fused multiply-adds). Below 0.49 box
-// lengths the rounded quotient is zero: no division (129 cycles in FP64).
+// lengths the rounded quotient is zero: no division (129 cycles in FP64). A
+// zero or infinite side has no such range: 0 / 0 and 0 * inf are not numbers,
+// which drops the pair.
 template <int ND>
 __device__ __forceinline__ double pair_dist2(const double* xi, const double* __restrict__ x, std::uint64_t q,
                                              const OvGrid& g) {
@@ -53,7 +56,7 @@ __device__ __forceinline__ double pair_dist2(const double* xi, const double* __r
     RCPG_UNROLL
     for (int d = 0; d < ND; ++d) {
         double dd = xsub(xi[d], x[q * ND + d]);
-        if (g.periodic && !(fabs(dd) <= 0.49 * g.box[d])) dd = xsub(dd, xmul(nearbyint(dd / g.box[d]), g.box[d]));
+        if (g.periodic && !(fabs(dd) <= g.near[d])) dd = xsub(dd, xmul(nearbyint(dd / g.box[d]), g.box[d]));
         s = xadd(s, xmul(dd, dd));
     }
     return s;
@@ -368,6 +371,7 @@ extern "C" int32_t rcpg_overlap_report(uint64_t N, int32_t ndim, const double* p
             if (n > 1048576.0) n = 1048576.0;
             g.lo[d] = lo;
             g.box[d] = box ? box[d] : L;
+            g.near[d] = g.box[d] > 0.0 && std::isfinite(g.box[d]) ? 0.49 * g.box[d] : -1.0;
             g.ncell[d] = static_cast<int>(n);
             cells *= n;
         }
