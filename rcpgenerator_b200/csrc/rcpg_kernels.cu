@@ -1314,9 +1314,15 @@ __global__ void __launch_bounds__(UnitShape<ND>::threads, UnitShape<ND>::blocks)
             }
             UnitPair<ND, MX> up;
             up.begin(xq, D0q, kap);
-            float xf[ND];
-            RCPG_UNROLL
-            for (int d = 0; d < ND; ++d) xf[d] = static_cast<float>(xq[d]);
+            // its own search record: not a number on an axis where it lies outside the box (store_search_record),
+            // where min(t, L - t) below would be no minimum image
+            float xf[NDC];
+            {
+                const float4 r = __ldg(frec + q);
+                xf[0] = r.x;
+                xf[1] = r.y;
+                if constexpr (NDC == 3) xf[2] = r.z;
+            }
             const float half_q = __fmaf_rn(__fmaf_rn(static_cast<float>(up.Di), 0.5f, tf), kRel, kSearchAbs * widest);
             std::uint32_t n = 0, listed = 0;
             // FP32 test of a record: false only for a particle outside the shell
