@@ -1272,6 +1272,7 @@ __global__ void __launch_bounds__(UnitShape<ND>::threads, UnitShape<ND>::blocks)
         side[d] = static_cast<float>(bx[d]);
         widest = fmaxf(widest, side[d]);
     }
+    if (widest < kSearchMinSide) widest = HUGE_VALF;
     const double scale0 = ctl->cell_scale[0];
     const std::uint32_t W = ctl->unit_w, chunks = ctl->unit_chunks, units = ctl->unit_count;
     const double kap = ctl->build_kappa;

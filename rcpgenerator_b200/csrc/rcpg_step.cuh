@@ -160,6 +160,11 @@ constexpr int kSliceLanes = 8;        // groups up to this size deal out ranges,
 // 1.2e-7 per axis (3.4e-7 in 8 dimensions), and positions may lie 1e-6 outside
 // the box; relative: the sum of squares and the cutoff round by less than 1e-6.
 constexpr float kSearchAbs = 3e-6f, kSearchRel = 1.000004f;
+// In a box whose longest side is below this the FP32 squares may leave FP32's
+// normal range: the absolute widening is worth at least 9e-12 of the squared
+// side, 9e-42 here, and the squares' subnormal steps are 1.4e-45. An infinite
+// side in the widening then lets every candidate and every range through.
+constexpr float kSearchMinSide = 1e-15f;
 
 template <int ND>
 struct SearchRecord {
@@ -387,7 +392,7 @@ struct SearchParams {
     double kap, t_shell;
     int K;       // size classes
     bool prune;  // no particle lies outside the box
-    float side[ND], widest;
+    float side[ND], widest;  // box sides; the longest, for the widening
 
     __device__ __forceinline__ void read(const DevCtl* ctl, bool in_box) {
         kap = ctl->build_kappa;
@@ -400,6 +405,7 @@ struct SearchParams {
             side[d] = static_cast<float>(ctl->g.box[d]);
             widest = fmaxf(widest, side[d]);
         }
+        if (widest < kSearchMinSide) widest = HUGE_VALF;
     }
 };
 

@@ -1,6 +1,7 @@
 """The FP32 tests ahead of the graph engine's neighbour searches (k_cells and
 k_build_rows, through rcpg_pairs_forces_scan) over the coordinates that the
-FP64 predicate takes: particles whole box sides outside the box."""
+FP64 predicate takes: particles whole box sides outside the box, and boxes
+whose squared lengths leave the range of FP32."""
 
 from __future__ import annotations
 
@@ -63,3 +64,19 @@ def test_cell_units_keep_partners_of_particles_whole_sides_outside(cuda_device, 
     assert cells
     assert sum(len(want[i]) for i in out) > 600  # they have partners
     assert [tuple(sorted(r)) for r in got] == want
+
+
+# cell units (2-D, 3-D), and the row search by one lane per particle with size classes
+@pytest.mark.parametrize("n,nd,ratio,cells", [(20011, 2, 1.3, True), (20011, 3, 1.3, True), (32771, 3, 10.0, False),
+                                              (70001, 2, 8.0, False)])
+@pytest.mark.parametrize("power", [-300, -70, -60, -50, 60, 120, 300])
+def test_rows_do_not_depend_on_the_unit_of_length(cuda_device, native, n, nd, ratio, cells, power):
+    """Lengths scaled by a power of two: every FP64 operation scales exactly, so the rows are the same."""
+    from tests import gpu_util as G
+    x, D = _state(n, nd, ratio, 0.4 if nd == 2 else 0.3)
+    t = native.lib.rcpg_t_shell(G.hp(D), n)
+    want, c0 = _scan(native, x, D, np.ones(nd), t, 192)
+    s = 2.0 ** power
+    got, c1 = _scan(native, x * s, D * s, np.full(nd, s), t * s, 192)
+    assert c0 == c1 == cells
+    assert got == want
