@@ -651,6 +651,7 @@ __device__ __forceinline__ std::uint32_t search_row_group(const DevArrays& a, co
             search_class_group<ND, NC>(a, ctl, sp, cell_start, sc, rs, G, s_list, s_q, s_end);
         }
     }
+    __syncwarp();  // the group's first lane reads the row that all its lanes have stored (close_row)
     return rs.n;
 }
 
