@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kMmaThreads)
               const float* __restrict__ target, const float* __restrict__ weight, __nv_bfloat16* __restrict__ dz,
               float* __restrict__ lterm, const double* __restrict__ scale, double* __restrict__ y64) {
     __shared__ __align__(16) Tile t;
-    tile_product(t, Operand<TA>{a, K, 1}, Operand<__nv_bfloat16>{W, K, 1}, M, N, K, blockIdx.y * kTM, blockIdx.x * kTN,
+    tile_product(t, Operand<TA>{a, K, 1}, Operand<__nv_bfloat16>{W, K, 1}, M, N, K, blockIdx.x * kTM, blockIdx.y * kTN,
                  [&](int m, int n, float c) {
                      const long long e = static_cast<long long>(m) * N + n;
                      const float v = c + bias[n];
@@ -308,7 +308,7 @@ void forward(cudaStream_t st, const int32_t* w, int L, int B, const __nv_bfloat1
     for (int l = 0; l < L; ++l) {
         const int I = w[l], O = w[l + 1];
         const bool last = l + 1 == L;
-        const dim3 grid((O + kTN - 1) / kTN, (B + kTM - 1) / kTM);
+        const dim3 grid((B + kTM - 1) / kTM, (O + kTN - 1) / kTN);  // rows along x: y ends at 65,535 tiles
         const float* bias = w32 + off + static_cast<std::size_t>(O) * I;
         float* z = last ? y : (T ? wk.z[l] : nullptr);
         __nv_bfloat16* act = last ? nullptr : wk.act[l + 1];
