@@ -922,7 +922,9 @@ bool Engine::advance_graph(std::uint64_t max_new_steps) {
             launches_ += 3 * static_cast<std::uint64_t>(graph_steps_) +
                          (hctl_.nbuilds - b0) * kernels_per_build() + (hctl_.pair_kernel_runs - f0);
         }
-        if (hctl_.halted) {
+        // a row overflow: the redone step counts like the others of this slice,
+        // and what it ends with (another overflow, a stop) is handled like theirs
+        while (hctl_.halted) {
             if (hctl_.cap_error) {
                 throw EngineError(-ENOSPC, std::string("rcpgenerator: particle ") +
                                                std::to_string(cap_error_particle(hctl_)) +
@@ -933,7 +935,8 @@ bool Engine::advance_graph(std::uint64_t max_new_steps) {
                                                "Recommendation: pass a larger neighbor_max (the per-particle base; e.g. neighbor_max=1500 -- capacity scales as 50*(D_i/D_min)^omega + neighbor_max), or reduce the size ratio.");
             }
             handle_overflow_and_resume();
-            continue;
+            pull_ctl();
+            c = hctl_.c;
         }
         if (hctl_.stopped) {
             if (c.done || c.steps + 1 > c.step_cap || c.hist_filled >= c.step_cap) {

@@ -1,0 +1,66 @@
+"""The engine's host code (rcpg_engine.cu) on a stand-in for the CUDA runtime
+and the kernels (tests/hostfake): no GPU."""
+
+from __future__ import annotations
+
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import pytest
+
+HERE = Path(__file__).resolve().parent / "hostfake"
+
+
+@pytest.fixture(scope="module")
+def lib():
+    subprocess.run(["make", "-s", "-C", str(HERE)], check=True)
+    lib = C.CDLL(str(HERE / "libhostfake.so"))
+    u64, vp = C.c_uint64, C.c_void_p
+    lib.hf_overflow.argtypes = [u64, C.c_uint32]
+    lib.hf_counts.argtypes = [C.POINTER(u64)]
+    lib.hf_engine.restype, lib.hf_engine.argtypes = vp, [u64, C.c_int, C.c_int, C.c_int, u64, C.c_int]
+    lib.hf_free.argtypes = [vp]
+    lib.hf_advance.argtypes = [vp, u64]
+    lib.hf_steps.restype, lib.hf_steps.argtypes = u64, [vp]
+    lib.hf_run.restype, lib.hf_run.argtypes = u64, [vp, u64, C.POINTER(u64), u64]
+    lib.hf_result.argtypes = [vp, C.POINTER(C.c_double)]
+    yield lib
+    lib.hf_set_device(0)
+
+
+def _engine(lib, small, graph_steps=32, max_steps=100, overflows=(), exact=0, mixed=0, device=0):
+    lib.hf_reset(small)
+    lib.hf_set_device(device)
+    for step, need in overflows:
+        lib.hf_overflow(step, need)
+    e = lib.hf_engine(50, exact, mixed, graph_steps, max_steps, device)
+    assert e
+    return e
+
+
+# overflows in the middle of a slice, at its first and its last step, twice in a step's slice, at the last step of
+# the run; by the small-packing kernel and by the step graph (replays of 32 and single steps)
+OVERFLOWS = [[], [(7, 40)], [(1, 40)], [(5, 40)], [(6, 40)], [(40, 30), (41, 50)], [(100, 40)], [(33, 40), (64, 50)]]
+
+
+@pytest.mark.parametrize("small", [1, 0])
+@pytest.mark.parametrize("overflows", OVERFLOWS)
+def test_advance_takes_the_steps_it_is_asked_for(lib, small, overflows):
+    e = _engine(lib, small, overflows=overflows)
+    steps = 0
+    for k in (5, 1, 1, 33, 2, 40, 7, 32):
+        done = lib.hf_advance(e, k)
+        steps = min(steps + k, 100)
+        assert (lib.hf_steps(e), done) == (steps, int(steps == 100))
+    lib.hf_free(e)
+
+
+@pytest.mark.parametrize("small", [1, 0])
+@pytest.mark.parametrize("overflows", OVERFLOWS)
+def test_every_observation_of_a_run_arrives(lib, small, overflows):
+    e = _engine(lib, small, overflows=overflows)
+    out = (C.c_uint64 * 64)()
+    n = lib.hf_run(e, 5, out, 64)
+    assert list(out[:n]) == list(range(0, 101, 5))
+    lib.hf_free(e)
