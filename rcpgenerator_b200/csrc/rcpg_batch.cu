@@ -689,7 +689,8 @@ __device__ void run_instance(const View& V, Shared& sh, std::uint32_t chunk, int
         }
         if (ctl->stopped) {
             const Controller& c = ctl->c;
-            if (c.done || c.steps + 1 > c.step_cap || c.hist_filled >= c.step_cap) {
+            // (a step that opens with a reorder has still to run, the last one too)
+            if (c.done || c.hist_filled >= c.step_cap) {
                 b_finish(V, 2u);
                 return;
             }

@@ -939,10 +939,8 @@ bool Engine::advance_graph(std::uint64_t max_new_steps) {
             c = hctl_.c;
         }
         if (hctl_.stopped) {
-            if (c.done || c.steps + 1 > c.step_cap || c.hist_filled >= c.step_cap) {
-                if (!c.done && c.hist_filled < c.step_cap) {
-                    // stopped before opening the next step: nothing pending
-                }
+            // (a step that opens with a reorder has still to run, the last one too)
+            if (c.done || c.hist_filled >= c.step_cap) {
                 finished_ = true;
                 break;
             }

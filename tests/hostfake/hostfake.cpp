@@ -28,6 +28,7 @@ struct Fake {
     cudaError_t small_error = cudaSuccess;     // what its launch returns
     std::vector<std::uint64_t> overflow_steps; // steps whose build finds a row beyond the capacity
     std::vector<std::uint32_t> overflow_need;
+    std::uint64_t reorder_every = 0;           // steps that open with a reorder stop the loop
     // records
     std::uint64_t wrong_device = 0;            // launches and allocations on a device that is not the engine's
     std::uint64_t graph_launches = 0, small_launches = 0;
@@ -66,8 +67,13 @@ void controller(const rcpg::DevArrays& a) {
         return;
     }
     k.c.hist_filled = k.c.steps;
-    if (k.c.steps + 1 > k.c.step_cap) k.stopped = 1u;
-    else k.c.steps += 1;
+    k.c.reorder = 0;
+    if (k.c.steps + 1 > k.c.step_cap) {
+        k.stopped = 1u;
+        return;
+    }
+    k.c.steps += 1;
+    if (fk.reorder_every && k.c.steps % fk.reorder_every == 0) k.c.reorder = k.stopped = 1u;
 }
 
 void step(const rcpg::DevArrays& a) {
@@ -228,6 +234,7 @@ void hf_overflow(std::uint64_t step, std::uint32_t need) {
     fk.overflow_steps.push_back(step);
     fk.overflow_need.push_back(need);
 }
+void hf_reorder_every(std::uint64_t steps) { fk.reorder_every = steps; }
 void hf_set_device(int d) { current_device = d; }
 int hf_get_device() { return current_device; }
 // wrong-device launches and allocations, graph launches, steps of the graph, small-packing launches

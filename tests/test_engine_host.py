@@ -18,6 +18,7 @@ def lib():
     lib = C.CDLL(str(HERE / "libhostfake.so"))
     u64, vp = C.c_uint64, C.c_void_p
     lib.hf_overflow.argtypes = [u64, C.c_uint32]
+    lib.hf_reorder_every.argtypes = [u64]
     lib.hf_counts.argtypes = [C.POINTER(u64)]
     lib.hf_engine.restype, lib.hf_engine.argtypes = vp, [u64, C.c_int, C.c_int, C.c_int, u64, C.c_int]
     lib.hf_free.argtypes = [vp]
@@ -63,4 +64,13 @@ def test_every_observation_of_a_run_arrives(lib, small, overflows):
     out = (C.c_uint64 * 64)()
     n = lib.hf_run(e, 5, out, 64)
     assert list(out[:n]) == list(range(0, 101, 5))
+    lib.hf_free(e)
+
+
+@pytest.mark.parametrize("small", [1, 0])
+@pytest.mark.parametrize("every", [100, 50, 20, 99])
+def test_a_reorder_at_the_last_step_does_not_end_the_run_before_it(lib, small, every):
+    e = _engine(lib, small)
+    lib.hf_reorder_every(every)
+    assert lib.hf_advance(e, 0) == 1 and lib.hf_steps(e) == 100
     lib.hf_free(e)
