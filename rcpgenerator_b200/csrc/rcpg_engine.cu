@@ -314,6 +314,7 @@ void Engine::pull_ctl() {
 }
 
 void Engine::set_blocking_sync(bool on) {
+    const DeviceGuard current(device_);
     if (on && !sync_ev_) {
         check(cudaEventCreateWithFlags(&sync_ev_, cudaEventBlockingSync | cudaEventDisableTiming), "event");
     } else if (!on && sync_ev_) {
@@ -455,11 +456,13 @@ Engine::~Engine() {
 }
 
 std::uint64_t Engine::builds() {
+    const DeviceGuard on(device_);
     pull_ctl();
     return hctl_.nbuilds;
 }
 
 void Engine::profile_build_kernel(std::uint32_t reps, double* avg_ms, double* alg_bytes) {
+    const DeviceGuard on(device_);
     pull_ctl();
     const DevCtl saved = hctl_;
     const std::size_t flush_bytes = std::size_t{256} << 20;
@@ -512,6 +515,7 @@ void Engine::profile_build_kernel(std::uint32_t reps, double* avg_ms, double* al
 
 void Engine::profile_pair_kernel(std::uint32_t reps, double* avg_ms, double* alg_bytes,
                                  double* mean_row) {
+    const DeviceGuard on(device_);
     pull_ctl();
     const DevCtl saved = hctl_;
     hctl_.stopped = 0u;
@@ -665,6 +669,7 @@ bool Engine::step_host() {
         hctl_.halted = 0u;
         push_ctl();
         launch_adam_refresh(a_, 1, 0, st_);
+        check(cudaGetLastError(), "ADAM pass");
         ++launches_;
         adam_pending_ = false;
         hctl_.adam_go = 0u;
@@ -912,6 +917,7 @@ bool Engine::advance_graph(std::uint64_t max_new_steps) {
                 launch_adam_refresh(a_, 1, 1, st_);
                 launches_ += kernels_per_build() + (mixed_ ? 4 : 3);
             }
+            check(cudaGetLastError(), "step kernels");  // without them the loop would wait for its steps for ever
         }
         pull_ctl();
         c = hctl_.c;
@@ -967,11 +973,25 @@ void Engine::handle_overflow_and_resume() {
     launch_forces(a_, 0, st_);
     launch_controller(a_, 0, st_);
     launch_adam_refresh(a_, 1, 1, st_);
+    check(cudaGetLastError(), "step after a row overflow");
     launches_ += kernels_per_build() + (mixed_ ? 4 : 3);
+}
+
+void Engine::apply_pending_adam() {
+    if (!adam_pending_) return;
+    hctl_.adam_go = 1u;
+    hctl_.fix_height_scale = 1.0;
+    push_ctl();
+    launch_adam_refresh(a_, 1, 0, st_);
+    check(cudaGetLastError(), "ADAM pass");
+    ++launches_;
+    adam_pending_ = false;
+    hctl_.adam_go = 0u;
 }
 
 bool Engine::advance(std::uint64_t max_new_steps) {
     if (finished_) return true;
+    const DeviceGuard on(device_);
     if (exact_) {
         std::uint64_t n = 0;
         while (!max_new_steps || n < max_new_steps) {
@@ -981,15 +1001,7 @@ bool Engine::advance(std::uint64_t max_new_steps) {
             }
             ++n;
         }
-        if (finished_ && adam_pending_) {
-            hctl_.adam_go = 1u;
-            hctl_.fix_height_scale = 1.0;
-            push_ctl();
-            launch_adam_refresh(a_, 1, 0, st_);
-            ++launches_;
-            adam_pending_ = false;
-            hctl_.adam_go = 0u;
-        }
+        if (finished_) apply_pending_adam();
         return finished_;
     }
     return advance_graph(max_new_steps);
@@ -1023,16 +1035,9 @@ void Engine::download_particles(double kd, bool fixed, double* x, double* D, std
     // scatter into the reference's order and the copies of it took 48 ms on the host
     const std::uint64_t N = N_;
     double* D_out = reinterpret_cast<double*>(a_.sort_keys[0]);
-    // a launch, unlike the copies, needs the engine's device current; a result
-    // may be read from any thread
-    int current = device_;
-    check(cudaGetDevice(&current), "cudaGetDevice");
-    if (current != device_) check(cudaSetDevice(device_), "cudaSetDevice");
     launch_collect(a_, kd, fixed, a_.vec_tmp, D_out, a_.sort_keys[1], st_);
-    const cudaError_t launched = cudaGetLastError();
-    if (current != device_) check(cudaSetDevice(current), "cudaSetDevice");
+    check(cudaGetLastError(), "collect");
     ++launches_;
-    check(launched, "collect");
     check(cudaMemcpyAsync(x, a_.vec_tmp, N * ndim_ * 8, cudaMemcpyDeviceToHost, st_), "D2H positions");
     check(cudaMemcpyAsync(D, D_out, N * 8, cudaMemcpyDeviceToHost, st_), "D2H diameters");
     if (origin) check(cudaMemcpyAsync(origin, a_.sort_keys[1], N * 8, cudaMemcpyDeviceToHost, st_), "D2H origin");
@@ -1040,15 +1045,8 @@ void Engine::download_particles(double kd, bool fixed, double* x, double* D, std
 }
 
 EngineResult Engine::result() {
-    if (exact_ && adam_pending_) {
-        hctl_.adam_go = 1u;
-        hctl_.fix_height_scale = 1.0;
-        push_ctl();
-        launch_adam_refresh(a_, 1, 0, st_);
-        ++launches_;
-        adam_pending_ = false;
-        hctl_.adam_go = 0u;
-    }
+    const DeviceGuard on(device_);
+    if (exact_) apply_pending_adam();
     if (!exact_) {
         pull_ctl();
         host_c_ = hctl_.c;
@@ -1088,6 +1086,7 @@ EngineResult Engine::result() {
 }
 
 void Engine::pair_precision_error(double* energy_rel, double* force_rel) {
+    const DeviceGuard on(device_);
     pull_ctl();
     const DevCtl saved = hctl_;
     const std::uint64_t n = N_ * static_cast<std::uint64_t>(ndim_);
@@ -1108,11 +1107,13 @@ void Engine::pair_precision_error(double* energy_rel, double* force_rel) {
         push_ctl();
         launch_forces(a_, 0, st_);
         launch_reduce_fast(a_, st_);
+        check(cudaGetLastError(), "precision check");
         launches_ += 2;
         if (prec == 0) {
             check(cudaMemcpyAsync(F64, a_.F, n * 8, cudaMemcpyDeviceToDevice, st_), "copy F");
         } else {
             launch_diff_max(F64, a_.F, n, mx, st_);
+            check(cudaGetLastError(), "precision check");
             ++launches_;
         }
         pull_ctl();
@@ -1134,6 +1135,17 @@ void Engine::pair_precision_error(double* energy_rel, double* force_rel) {
 
 void Engine::observe(std::uint64_t step, bool capture, const ObserverFn& observer,
                      std::vector<TraceSample>* trace) {
+    Observation ob{step, 0.0, 0.0, 0.0, 0.0};
+    std::vector<double> xs;
+    sample(ob, capture, xs, trace);
+    if (observer) observer(ob, capture ? &xs : nullptr);
+}
+
+// The data of an observation (and its trajectory sample). The observer is
+// called outside, with the caller's device current.
+void Engine::sample(Observation& ob, bool capture, std::vector<double>& xs, std::vector<TraceSample>* trace) {
+    const DeviceGuard on(device_);
+    const std::uint64_t step = ob.step;
     double vals[4] = {0, 0, 0, 0};
     if (step == 0) {
         vals[0] = host_c_.phi;  // setup phi (already divided by phi_modifier, ENG:4505)
@@ -1152,18 +1164,9 @@ void Engine::observe(std::uint64_t step, bool capture, const ObserverFn& observe
         vals[2] = h_energy_[step - 1];
         vals[3] = h_maxov_[step - 1];
     }
-    Observation ob{step, vals[0], vals[1], vals[2], vals[3]};
-    std::vector<double> xs;
+    ob = Observation{step, vals[0], vals[1], vals[2], vals[3]};
     if (capture) {
-        if (exact_ && adam_pending_) {
-            hctl_.adam_go = 1u;
-            hctl_.fix_height_scale = 1.0;
-            push_ctl();
-            launch_adam_refresh(a_, 1, 0, st_);
-            ++launches_;
-            adam_pending_ = false;
-            hctl_.adam_go = 0u;
-        }
+        if (exact_) apply_pending_adam();
         xs.resize(N_ * ndim_);
         TraceSample ts;
         ts.step = step;
@@ -1182,7 +1185,6 @@ void Engine::observe(std::uint64_t step, bool capture, const ObserverFn& observe
         ts.max_min_dist = ob.max_min_dist;
         if (trace) trace->push_back(std::move(ts));
     }
-    if (observer) observer(ob, capture ? &xs : nullptr);
 }
 
 void Engine::run(std::uint64_t progress_interval, bool capture_positions,

@@ -113,6 +113,33 @@ class EngineError : public std::runtime_error {
     int code_;
 };
 
+// Makes a device current for its scope. Launches, allocations and events go to
+// the current device, whatever the stream; an engine may be used from any
+// thread, and its caller may have selected another device since.
+class DeviceGuard {
+   public:
+    explicit DeviceGuard(int device) {
+        cudaGetLastError();  // what the caller's own calls left is not the engine's error
+        cudaError_t e = cudaGetDevice(&before_);
+        if (e == cudaSuccess && before_ != device) {
+            e = cudaSetDevice(device);
+            switched_ = e == cudaSuccess;
+        }
+        if (e != cudaSuccess)
+            throw EngineError(-2, std::string("rcpgenerator_b200: cannot select the engine's device: ") +
+                                      cudaGetErrorString(e));
+    }
+    ~DeviceGuard() {
+        if (switched_) cudaSetDevice(before_);
+    }
+    DeviceGuard(const DeviceGuard&) = delete;
+    DeviceGuard& operator=(const DeviceGuard&) = delete;
+
+   private:
+    int before_ = 0;
+    bool switched_ = false;
+};
+
 class Engine {
    public:
     explicit Engine(EngineInput in, cudaStream_t stream = nullptr);
@@ -179,9 +206,12 @@ class Engine {
     std::uint64_t kernels_per_build() const;
     void destroy_graph();
     void handle_overflow_and_resume();
+    // exact mode: the ADAM pass of the last finished step, if it is still due
+    void apply_pending_adam();
     void after_stop();
     void observe(std::uint64_t step, bool capture, const ObserverFn& observer,
                  std::vector<TraceSample>* trace);
+    void sample(Observation& ob, bool capture, std::vector<double>& xs, std::vector<TraceSample>* trace);
     void download_histories();
     // the current state in the reference's order: x [N*ndim], diameters D0 * kd
     // (D0 when fixed) [N], particle_origin [N] (optional)

@@ -12,6 +12,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <stdexcept>
 #include <vector>
 
 #include "rcpg_engine.h"
@@ -30,6 +31,7 @@ struct Fake {
     std::vector<std::uint32_t> overflow_need;
     std::uint64_t reorder_every = 0;           // steps that open with a reorder stop the loop
     // records
+    int observer_device = -1;                  // device that was current in every observer call (-2: several)
     std::uint64_t wrong_device = 0;            // launches and allocations on a device that is not the engine's
     std::uint64_t graph_launches = 0, small_launches = 0;
     int captured = 0;                          // steps of the graph captured last
@@ -46,7 +48,7 @@ int device_of(cudaStream_t st) { return st ? reinterpret_cast<Stream*>(st)->devi
 // Whether a launch on st takes place.
 bool launched(cudaStream_t st) {
     if (current_device == device_of(st)) return true;
-    ++fk.wrong_device;
+    if (++fk.wrong_device > 1000) throw std::runtime_error("a loop whose launches all fail");
     last_error = cudaErrorInvalidResourceHandle;
     return false;
 }
@@ -236,7 +238,9 @@ void hf_overflow(std::uint64_t step, std::uint32_t need) {
 }
 void hf_reorder_every(std::uint64_t steps) { fk.reorder_every = steps; }
 void hf_set_device(int d) { current_device = d; }
+void hf_leave_error() { last_error = cudaErrorInvalidValue; }
 int hf_get_device() { return current_device; }
+int hf_observer_device() { return fk.observer_device; }
 // wrong-device launches and allocations, graph launches, steps of the graph, small-packing launches
 void hf_counts(std::uint64_t* out) {
     out[0] = fk.wrong_device;
@@ -275,13 +279,20 @@ std::uint64_t hf_steps(void* e) { return static_cast<rcpg::Engine*>(e)->steps_do
 // the steps that a run's observer sees; their number
 std::uint64_t hf_run(void* e, std::uint64_t interval, std::uint64_t* steps, std::uint64_t cap) {
     std::uint64_t n = 0;
-    static_cast<rcpg::Engine*>(e)->run(
-        interval, false, 0,
-        [&](const rcpg::Observation& o, const std::vector<double>*) {
-            if (n < cap) steps[n] = o.step;
-            ++n;
-        },
-        nullptr);
+    std::vector<rcpg::TraceSample> trace;
+    try {
+        static_cast<rcpg::Engine*>(e)->run(
+            interval, true, interval,
+            [&](const rcpg::Observation& o, const std::vector<double>*) {
+                if (n < cap) steps[n] = o.step;
+                ++n;
+                fk.observer_device = fk.observer_device == -1 || fk.observer_device == current_device ? current_device : -2;
+            },
+            &trace);
+    } catch (const std::exception&) {
+        return 0;
+    }
+    if (trace.size() != n) return 0;
     return n;
 }
 int hf_result(void* e, double* x0) {

@@ -74,3 +74,28 @@ def test_a_reorder_at_the_last_step_does_not_end_the_run_before_it(lib, small, e
     lib.hf_reorder_every(every)
     assert lib.hf_advance(e, 0) == 1 and lib.hf_steps(e) == 100
     lib.hf_free(e)
+
+
+@pytest.mark.parametrize("exact,mixed,small", [(1, 0, 0), (0, 0, 0), (0, 0, 1), (0, 1, 0), (0, 1, 1)])
+@pytest.mark.parametrize("device", [0, 1])
+def test_work_goes_to_the_engines_device_whatever_is_current(lib, exact, mixed, small, device):
+    """Steps, observations and results with the other device current: everything is launched and allocated on the
+    engine's device, the pending ADAM pass of the exact engine among it, and the caller's device stays current."""
+    e = _engine(lib, small, exact=exact, mixed=mixed, overflows=[(9, 40)], device=device)
+    other = 1 - device
+    lib.hf_set_device(other)
+    passes = C.c_double()
+    lib.hf_leave_error()  # by a call of the caller's own
+    assert lib.hf_advance(e, 12) == 0 and lib.hf_get_device() == other
+    assert lib.hf_result(e, C.byref(passes)) == 0 and lib.hf_get_device() == other
+    if exact:
+        assert passes.value == 0.5 + 12  # the stand-in ADAM pass adds one
+    out = (C.c_uint64 * 64)()
+    n = lib.hf_run(e, 5, out, 64)
+    # step 0 is reported at the start of the call
+    assert list(out[:n]) == [0] + list(range(15, 101, 5)) and lib.hf_get_device() == other
+    assert lib.hf_observer_device() == other
+    counts = (C.c_uint64 * 4)()
+    lib.hf_counts(counts)
+    assert counts[0] == 0
+    lib.hf_free(e)
