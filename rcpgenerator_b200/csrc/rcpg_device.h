@@ -219,10 +219,11 @@ void launch_diff_max(const double* ref, const double* cmp, std::uint64_t n, unsi
 void launch_controller(const DevArrays& a, int open_only, cudaStream_t st);
 void launch_reorder(const DevArrays& a, cudaStream_t st);
 // Up to `steps` steps of a small packing in one launch (rcpg_small.cu), from
-// the same state and to the same state as the step graph; small_steps_ok: the
-// packing and its cell grid are small enough.
+// the same state and to the same state as the step graph. small_steps_ok: the
+// packing and its cell grid are small enough and the current device can place
+// the kernel's cluster (asked of the driver: once per engine).
 bool small_steps_ok(const DevArrays& a);
-void launch_small_steps(const DevArrays& a, std::uint32_t steps, cudaStream_t st);
+cudaError_t launch_small_steps(const DevArrays& a, std::uint32_t steps, cudaStream_t st);
 void launch_fix_height(const DevArrays& a, cudaStream_t st);
 
 void launch_pack(std::uint64_t N, int ndim, const double* x, const double* D, double* pos,

@@ -257,6 +257,7 @@ void Engine::alloc_device() {
                         h_mu_.data(), h_alpha_.data(), h_muflag_.data()};
     }
     hctl_pinned_ = pinned_ctl_acquire();
+    small_ = small_steps_ok(a_);
 }
 
 void Engine::ensure_row_capacity(std::uint32_t need) {
@@ -896,15 +897,14 @@ bool Engine::advance_graph(std::uint64_t max_new_steps) {
         const std::uint64_t done_steps = c.hist_filled - start;
         if (max_new_steps && done_steps >= max_new_steps) break;
         const std::uint64_t want = max_new_steps ? max_new_steps - done_steps : ~0ull;
-        const bool small = small_steps_ok(a_);
-        if (!small && !graph_exec_) capture_graph();
+        if (!small_ && !graph_exec_) capture_graph();
         const std::uint64_t b0 = hctl_.nbuilds, f0 = hctl_.pair_kernel_runs;
         bool replay = false;
-        if (small) {
+        if (small_) {
             // the steps of a small packing as one cluster kernel, short enough
             // (a few ms) that other engines' work interleaves
-            launch_small_steps(a_, static_cast<std::uint32_t>(std::min<std::uint64_t>(want, kSmallSlice)), st_);
-            check(cudaGetLastError(), "small steps");
+            check(launch_small_steps(a_, static_cast<std::uint32_t>(std::min<std::uint64_t>(want, kSmallSlice)), st_),
+                  "small steps");
             ++launches_;
         } else if (want >= static_cast<std::uint64_t>(graph_steps_)) {
             for (int k = 0; k < graph_steps_; k += captured_steps()) check(cudaGraphLaunch(graph_exec_, st_), "graph launch");

@@ -254,6 +254,7 @@ class Engine {
     std::vector<void*> allocs_;
     cudaGraphExec_t graph_exec_ = nullptr;
     cudaGraph_t graph_ = nullptr;
+    bool small_ = false;  // graph mode: the steps run in the cluster kernel (small_steps_ok)
     std::uint64_t graph_nodes_per_step_ = 0;
     cudaStream_t body_st_ = nullptr;  // captures the bodies of the step graph's conditional nodes
     std::uint32_t* pinned_ = nullptr;

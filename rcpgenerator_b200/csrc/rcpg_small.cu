@@ -600,14 +600,19 @@ int small_blocks(std::uint64_t N) {
     return C;
 }
 
+// Clusters of this packing's kernel that the device can hold at once (none
+// where it has no room for one: a partitioned GPU, fewer multiprocessors or
+// less shared memory); without `clusters`, up to `steps` steps launched.
 template <int ND>
-void small_nd(const DevArrays& a, std::uint32_t steps, cudaStream_t st) {
+cudaError_t small_nd(const DevArrays& a, std::uint32_t steps, cudaStream_t st, int* clusters) {
     const int C = small_blocks(a.N);
     const std::uint64_t own = ((a.N + 31) / 32 + C - 1) / C * 32;  // particles per block
     int lanes = 1;
     while (lanes < 32 && own * static_cast<std::uint64_t>(lanes) * 2 <= kSmallThreads) lanes *= 2;
-    cudaFuncSetAttribute(k_small_steps<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(SmallShared)));
-    cudaFuncSetAttribute(k_small_steps<ND>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaError_t e = cudaFuncSetAttribute(k_small_steps<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(sizeof(SmallShared)));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_steps<ND>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(C));
     cfg.blockDim = dim3(kSmallThreads);
@@ -619,26 +624,36 @@ void small_nd(const DevArrays& a, std::uint32_t steps, cudaStream_t st) {
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_small_steps<ND>, a, steps, lanes);
+    if (clusters) return cudaOccupancyMaxActiveClusters(clusters, k_small_steps<ND>, &cfg);
+    return cudaLaunchKernelEx(&cfg, k_small_steps<ND>, a, steps, lanes);
+}
+
+cudaError_t small_any(const DevArrays& a, std::uint32_t steps, cudaStream_t st, int* clusters) {
+    switch (a.ndim) {
+        case 2: return small_nd<2>(a, steps, st, clusters);
+        case 3: return small_nd<3>(a, steps, st, clusters);
+        case 4: return small_nd<4>(a, steps, st, clusters);
+        case 5: return small_nd<5>(a, steps, st, clusters);
+        case 6: return small_nd<6>(a, steps, st, clusters);
+        case 7: return small_nd<7>(a, steps, st, clusters);
+        case 8: return small_nd<8>(a, steps, st, clusters);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace
 
 bool small_steps_ok(const DevArrays& a) {
-    return a.permute && !a.sorted_rows && a.N <= static_cast<std::uint64_t>(kSmallN) && a.C_alloc + 1 <= kSmallCells;
+    if (!a.permute || a.sorted_rows || a.N > static_cast<std::uint64_t>(kSmallN) || a.C_alloc + 1 > kSmallCells)
+        return false;
+    int clusters = 0;
+    const cudaError_t e = small_any(a, 0, nullptr, &clusters);
+    if (e != cudaSuccess) cudaGetLastError();  // the step graph runs instead
+    return e == cudaSuccess && clusters > 0;
 }
 
-void launch_small_steps(const DevArrays& a, std::uint32_t steps, cudaStream_t st) {
-    switch (a.ndim) {
-        case 2: small_nd<2>(a, steps, st); break;
-        case 3: small_nd<3>(a, steps, st); break;
-        case 4: small_nd<4>(a, steps, st); break;
-        case 5: small_nd<5>(a, steps, st); break;
-        case 6: small_nd<6>(a, steps, st); break;
-        case 7: small_nd<7>(a, steps, st); break;
-        case 8: small_nd<8>(a, steps, st); break;
-        default: break;
-    }
+cudaError_t launch_small_steps(const DevArrays& a, std::uint32_t steps, cudaStream_t st) {
+    return small_any(a, steps, st, nullptr);
 }
 
 }  // namespace rcpg

@@ -26,7 +26,6 @@ struct Stream {
 struct Fake {
     // scenario
     int small_clusters = 0;                    // clusters of the small-packing kernel that fit the device
-    cudaError_t small_error = cudaSuccess;     // what its launch returns
     std::vector<std::uint64_t> overflow_steps; // steps whose build finds a row beyond the capacity
     std::vector<std::uint32_t> overflow_need;
     std::uint64_t reorder_every = 0;           // steps that open with a reorder stop the loop
@@ -217,10 +216,11 @@ void launch_collect(const DevArrays& a, double kd, bool fixed, double* x, double
     }
 }
 bool small_steps_ok(const DevArrays&) { return fk.small_clusters > 0; }
-void launch_small_steps(const DevArrays& a, std::uint32_t steps, cudaStream_t st) {
-    if (!launched(st)) return;
+cudaError_t launch_small_steps(const DevArrays& a, std::uint32_t steps, cudaStream_t st) {
+    if (!launched(st)) return cudaErrorInvalidResourceHandle;
     ++fk.small_launches;
     for (std::uint32_t k = 0; k < steps; ++k) step(a);
+    return cudaSuccess;
 }
 
 }  // namespace rcpg

@@ -99,3 +99,39 @@ def test_work_goes_to_the_engines_device_whatever_is_current(lib, exact, mixed, 
     lib.hf_counts(counts)
     assert counts[0] == 0
     lib.hf_free(e)
+
+
+@pytest.fixture(scope="module")
+def small():
+    subprocess.run(["make", "-s", "-C", str(HERE), "libsmallfit.so"], check=True)
+    lib = C.CDLL(str(HERE / "libsmallfit.so"))
+    lib.sf_ok.argtypes = [C.c_uint64, C.c_int, C.c_uint32, C.c_int, C.c_int, C.c_int]
+    return lib
+
+
+@pytest.mark.parametrize("nd", range(2, 9))
+def test_cluster_kernel_only_where_its_cluster_fits(small, nd):
+    """A device without room for the cluster (or a refusal of its shared memory or size) leaves small packings to the
+    step graph, without an error; larger packings and grids never ask."""
+    for n, blocks in ((64, 1), (2000, 16), (8192, 16)):
+        assert small.sf_ok(n, nd, 500, 1, 0, 0) == 1 and small.sf_cluster() == blocks
+        assert small.sf_ok(n, nd, 500, 0, 0, 0) == 0
+        assert small.sf_ok(n, nd, 500, 1, 1, 0) == 0  # cudaFuncSetAttribute refuses
+        assert small.sf_ok(n, nd, 500, 1, 0, 1) == 0  # the query fails
+    assert small.sf_ok(8193, nd, 500, 1, 0, 0) == 0 and small.sf_ok(8192, nd, 12288, 1, 0, 0) == 0
+    assert small.sf_ok(8192, nd, 12287, 1, 0, 0) == 1
+
+
+def test_cluster_kernel_reports_its_launch(small):
+    assert small.sf_run(3, 0, 0) == 0
+    assert small.sf_run(3, 1, 0) == 1 and small.sf_run(3, 0, 701) == 701 and small.sf_run(9, 0, 0) != 0
+
+
+def test_engine_takes_the_step_graph_where_the_cluster_kernel_does_not_fit(lib):
+    for fits in (0, 1):
+        e = _engine(lib, fits)
+        counts = (C.c_uint64 * 4)()
+        assert lib.hf_advance(e, 0) == 1 and lib.hf_steps(e) == 100
+        lib.hf_counts(counts)
+        assert (counts[1] > 0, counts[3] > 0) == (not fits, bool(fits))
+        lib.hf_free(e)
