@@ -803,20 +803,24 @@ void Engine::capture_step() {
     launch_adam_refresh(ag, 1, 1, st_);
 }
 
+// Capturing, instantiating and destroying 32 steps with their conditional
+// nodes costs 8 ms per engine, a quarter of that with 8 steps; below four steps
+// the launches would cost more than they save (up to 31 of them for 31 steps).
 int Engine::captured_steps() const {
-    constexpr int kCaptureSteps = 8;
-    int k = graph_steps_ < kCaptureSteps ? graph_steps_ : kCaptureSteps;
-    while (graph_steps_ % k != 0) --k;
+    for (int k = 8; k >= 4; --k)
+        if (graph_steps_ % k == 0) return k;
+    if (graph_steps_ <= 8) return graph_steps_;
+    int k = 9;
+    while (graph_steps_ % k != 0) ++k;
     return k;
 }
 
-// The step loop as one CUDA graph of a divisor of graph_steps_ steps (at most
-// kCaptureSteps), launched several times between two looks at the control
-// block: capturing, instantiating and destroying 32 steps with their
-// conditional nodes cost 8 ms per engine, a quarter of that now. Each step opens with
-// a one-thread gate kernel; the build and the pair kernel sit in conditional
-// nodes that the gate and the build set on the device, so a step without a
-// rebuild launches four kernels (gate, pair kernel, controller, ADAM).
+// The step loop as one CUDA graph of a divisor of graph_steps_ steps
+// (captured_steps), launched as often as that takes between two looks at the
+// control block. Each step opens with a one-thread gate kernel; the build and
+// the pair kernel sit in conditional nodes that the gate and the build set on
+// the device, so a step without a rebuild launches four kernels (gate, pair
+// kernel, controller, ADAM).
 void Engine::capture_graph() {
     destroy_graph();
     if (!body_st_) check(cudaStreamCreateWithFlags(&body_st_, cudaStreamNonBlocking), "cudaStreamCreate");

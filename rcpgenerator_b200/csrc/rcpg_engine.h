@@ -197,7 +197,9 @@ class Engine {
     bool step_host();
     bool advance_graph(std::uint64_t max_new_steps);
     void capture_graph();
-    int captured_steps() const;  // steps of the captured graph, a divisor of graph_steps_
+    // steps of the captured graph: the largest divisor of graph_steps_ from 8 down
+    // to 4, else the smallest one above 8 (fewer than 4 steps: all of them)
+    int captured_steps() const;
     // one step of the step graph: gate, conditional build, pair-kernel switch,
     // controller, ADAM (kernels run only where the step needs them)
     void capture_step();

@@ -135,3 +135,19 @@ def test_engine_takes_the_step_graph_where_the_cluster_kernel_does_not_fit(lib):
         lib.hf_counts(counts)
         assert (counts[1] > 0, counts[3] > 0) == (not fits, bool(fits))
         lib.hf_free(e)
+
+
+def test_graph_of_any_length_takes_few_launches(lib):
+    """graph_steps steps between two looks, whatever divides them: no graph of fewer than four steps unless there are
+    no more, no more launches than one per four steps, and no larger graph than the steps themselves."""
+    for graph_steps in list(range(1, 70)) + [97, 128, 1009]:
+        e = _engine(lib, 0, graph_steps=graph_steps, max_steps=2 * graph_steps)
+        counts = (C.c_uint64 * 4)()
+        assert lib.hf_advance(e, graph_steps) == (0 if graph_steps else 1) and lib.hf_steps(e) == graph_steps
+        lib.hf_counts(counts)
+        launches, captured = counts[1], counts[2]
+        assert launches * captured == graph_steps
+        assert captured >= min(4, graph_steps)
+        assert captured <= max(8, min(d for d in range(4, graph_steps + 1) if graph_steps % d == 0)
+                               if graph_steps >= 4 else 3)
+        lib.hf_free(e)
