@@ -80,8 +80,9 @@ def overlap_report(packing, frac_def="sum", verbose=False, device: int = 0):
         boxp = box.ctypes.data_as(N._dp)
     ncand, nov = C.c_uint64(0), C.c_uint64(0)
     # room for a jammed packing's contacts (2 d pairs of neighbours, d per particle) and as many rattling
-    # overlaps; a state with more is reported by a second call with the exact size
-    cap = 2 * ndim * n
+    # overlaps; a state with more is reported by a second call with the exact size. Beyond 2^23 pairs (200 MB) that
+    # room would be several times the state's own memory: the first call only counts
+    cap = 2 * ndim * n if 2 * ndim * n <= 1 << 23 else 0
     for _ in range(2):
         pairs = np.empty((max(cap, 1), 2), np.uint32)
         fs = np.empty(max(cap, 1))
