@@ -283,6 +283,7 @@ class WarmStart:
         X = np.atleast_2d(np.asarray(X, dtype=np.float64))
         if hasattr(self.net, "predict"):
             lo, hi = (-np.inf, np.inf) if self.x_lo is None else (self.x_lo, self.x_hi)
+            X = np.broadcast_to(X, np.broadcast_shapes(X.shape, self.x_mean.shape))
             return self.net.predict(X, lo, hi, self.x_mean, self.x_std, self.y_mean, self.y_std)
         # a stand-in network that only has forward()
         if self.x_lo is not None:
