@@ -204,6 +204,10 @@ int32_t rcpg_engine_advance(rcpg_engine* e, uint64_t max_new_steps, int32_t* fin
 uint64_t rcpg_engine_steps(const rcpg_engine* e);
 uint64_t rcpg_engine_kernel_launches(const rcpg_engine* e);
 int32_t rcpg_engine_result(rcpg_engine* e, rcpg_result** out, char* err, size_t errlen);
+/* Diagnostic: with on != 0 the engine's later steps run in the step graph also
+ * where the cluster kernel of small packings applies. Both give the same
+ * results bit for bit. */
+void rcpg_engine_step_graph(rcpg_engine* e, int32_t on);
 void rcpg_engine_destroy(rcpg_engine* e);
 /* Engine diagnostics (no reference counterpart): times `reps` launches of the
  * pair-force kernel on the engine's current state with CUDA events on its

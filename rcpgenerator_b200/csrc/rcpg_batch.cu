@@ -369,7 +369,7 @@ __device__ ForceSums b_forces(const View& V, Shared& sh, bool mixed) {
             if (mixed) {
                 float dxf[ND];
                 const float d2f = mixed_disp<ND>(xi, xj, bx, hbf, dxf);
-                const float rsum = 0.5f * (Dif + static_cast<float>(D0j) * kapf);
+                const float rsum = mixed_rij(Dif, static_cast<float>(D0j), kapf);
                 if (!(d2f < rsum * rsum)) continue;
                 pair_terms_mixed<ND>(dxf, d2f, rsum, fif, pt);
             } else {

@@ -494,6 +494,10 @@ int32_t rcpg_engine_profile_build_kernel(rcpg_engine* e, uint32_t reps, double* 
     }
 }
 
+void rcpg_engine_step_graph(rcpg_engine* e, int32_t on) {
+    if (e) e->eng->prefer_step_graph(on != 0);
+}
+
 void rcpg_engine_destroy(rcpg_engine* e) {
     if (!e) return;
     delete e->eng;

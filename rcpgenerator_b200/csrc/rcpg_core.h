@@ -211,33 +211,40 @@ RCPG_UNROLL
     return d2;
 }
 
-// Force and scalar terms of an overlapping pair (d2 < rsum^2, rsum = r_ij) in
-// FP32 (ENG:4105-4139 with FP32 operands); the force is added to the FP32
-// per-particle sum fi, the scalar terms go to the FP64 accumulators. The
-// overlap-dependent terms carry a relative error of about 1e-7 / overlap.
-// The scalar terms of the FP32 pair path, kept in FP32: the per-particle sums
-// of that path are FP32, so the terms never need an FP64 round trip.
+// The FP32 pair path. Its multiplications and additions are written out
+// (no contraction left to the compiler): a run mixes kernels -- the cluster
+// kernel or the step graph, a build's fused forces or the pair kernel -- and
+// each of them must give the same terms and sums.
+//
+// The scalar terms of a pair, kept in FP32: the per-particle sums of this path
+// are FP32, so the terms never need an FP64 round trip.
 struct PairTermsF {
-    float U, Lc, dk, Fm;
+    float U, Lc, gap, Fm;  // gap = dist - r_ij: the dkappa term is r_ij * gap (mixed_add_dk)
 };
 
-// dist - r of an overlapping pair. Where a kernel adds the dkappa term r (dist
-// - r) to an FP32 sum, the product and the sum are one fused multiply-add.
-__device__ __forceinline__ float mixed_gap(float d2, float rsum) {
-    return __fsub_rn(__fmul_rn(d2, rsqrtf(d2)), rsum);
+// r_ij of particle i (Di = its FP32 diameter) and partner j (D0j, times kap).
+__device__ __forceinline__ float mixed_rij(float Di, float D0j, float kap) {
+    return __fmul_rn(0.5f, __fmaf_rn(D0j, kap, Di));
 }
 
+// s + the dkappa term of a pair, one rounding
+__device__ __forceinline__ float mixed_add_dk(float s, float r_ij, float gap) { return __fmaf_rn(r_ij, gap, s); }
+
+// Force and scalar terms of an overlapping pair (d2 < rsum^2, rsum = r_ij) in
+// FP32 (ENG:4105-4139 with FP32 operands); the force is added to the FP32
+// per-particle sum fi. The overlap-dependent terms carry a relative error of
+// about 1e-7 / overlap.
 template <int ND>
 __device__ __forceinline__ void pair_terms_mixed_f(const float* dxf, float d2, float rsum, float* fi,
                                                    PairTermsF& pt) {
     const float inv_dist = rsqrtf(d2);
-    const float dist = d2 * inv_dist;
+    const float dist = __fmul_rn(d2, inv_dist);
     const float F_mag = __fmaf_rn(-rsum, inv_dist, 1.0f);  // -(r/dist - 1)
 RCPG_UNROLL
     for (int d = 0; d < ND; ++d) fi[d] = __fmaf_rn(F_mag, dxf[d], fi[d]);
-    pt.U = 1.0f - __fdividef(dist, rsum);
+    pt.U = __fmaf_rn(-dist, __fdividef(1.0f, rsum), 1.0f);  // 1 - dist / r_ij
     pt.Lc = rsum;
-    pt.dk = rsum * (dist - rsum);
+    pt.gap = __fsub_rn(dist, rsum);
     pt.Fm = F_mag;
 }
 
@@ -248,7 +255,7 @@ __device__ __forceinline__ void pair_terms_mixed(const float* dxf, float d2, flo
     pair_terms_mixed_f<ND>(dxf, d2, rsum, fi, f);
     pt.U = static_cast<double>(f.U);
     pt.Lc = static_cast<double>(f.Lc);
-    pt.dk = static_cast<double>(f.dk);
+    pt.dk = static_cast<double>(__fmul_rn(f.Lc, f.gap));
     pt.Fm = static_cast<double>(f.Fm);
 }
 #endif

@@ -901,10 +901,11 @@ bool Engine::advance_graph(std::uint64_t max_new_steps) {
         const std::uint64_t done_steps = c.hist_filled - start;
         if (max_new_steps && done_steps >= max_new_steps) break;
         const std::uint64_t want = max_new_steps ? max_new_steps - done_steps : ~0ull;
-        if (!small_ && !graph_exec_) capture_graph();
+        const bool small = small_ && !step_graph_;
+        if (!small && !graph_exec_) capture_graph();
         const std::uint64_t b0 = hctl_.nbuilds, f0 = hctl_.pair_kernel_runs;
         bool replay = false;
-        if (small_) {
+        if (small) {
             // the steps of a small packing as one cluster kernel, short enough
             // (a few ms) that other engines' work interleaves
             check(launch_small_steps(a_, static_cast<std::uint32_t>(std::min<std::uint64_t>(want, kSmallSlice)), st_),

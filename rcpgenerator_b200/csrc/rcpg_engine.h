@@ -180,6 +180,9 @@ class Engine {
     // Waits for the device by sleeping on a blocking event instead of spinning
     // (for many engines driven by more host threads than cores: a batch).
     void set_blocking_sync(bool on);
+    // Later steps by the step graph also where the cluster kernel applies
+    // (diagnostic: both give the same results bit for bit).
+    void prefer_step_graph(bool on) { step_graph_ = on; }
 
    private:
     void setup_host(EngineInput in);
@@ -256,7 +259,8 @@ class Engine {
     std::vector<void*> allocs_;
     cudaGraphExec_t graph_exec_ = nullptr;
     cudaGraph_t graph_ = nullptr;
-    bool small_ = false;  // graph mode: the steps run in the cluster kernel (small_steps_ok)
+    bool small_ = false;       // graph mode: the cluster kernel can run the steps (small_steps_ok)
+    bool step_graph_ = false;  // ... but is not asked to
     std::uint64_t graph_nodes_per_step_ = 0;
     cudaStream_t body_st_ = nullptr;  // captures the bodies of the step graph's conditional nodes
     std::uint32_t* pinned_ = nullptr;

@@ -1185,7 +1185,7 @@ struct UnitPair {
                                           bool fuse) const {
         if constexpr (MX) {
             pr.d2 = mixed_disp<ND>(xi, xj, bx, hbf, pr.dx);
-            pr.r = 0.5f * (Dif + D0jf * kapf);
+            pr.r = mixed_rij(Dif, D0jf, kapf);
             const float rc = pr.r + tf;
             pr.pass = pr.d2 < rc * rc * kShellMarginF;
             pr.ov = fuse && pr.d2 < pr.r * pr.r;
@@ -1208,7 +1208,7 @@ struct UnitPair {
             if (upper) {
                 sU += pf.U;
                 sLc += pf.Lc;
-                sdk += pf.dk;
+                sdk = mixed_add_dk(sdk, pf.Lc, pf.gap);
                 sFm += pf.Fm;
                 smax = fmaxf(smax, pf.U);
                 ++scount;
@@ -1552,7 +1552,7 @@ __global__ void __launch_bounds__(kForceBlock, EXACT ? 1 : ((MIXED && ND == 2) ?
                 // FP32 terms summed in FP32 (EXACT never takes FP32 terms)
                 sU += pt.U;
                 sLc += pt.Lc;
-                sdk += pt.dk;
+                sdk = mixed_add_dk(sdk, pt.Lc, pt.gap);
                 sFm += pt.Fm;
                 smax = fmaxf(smax, pt.U);
                 ++scount;

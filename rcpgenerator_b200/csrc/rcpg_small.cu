@@ -160,7 +160,7 @@ __device__ __forceinline__ void pair_sums(const DevArrays& b, const DevCtl* ctl,
         T dx[ND], d2, r;
         if constexpr (MX) {
             d2 = mixed_disp<ND>(xi, xj, bx, hbf, dx);
-            r = 0.5f * (Dif + static_cast<float>(D0j) * kapf);
+            r = mixed_rij(Dif, static_cast<float>(D0j), kapf);
         } else {
             r = xmul(0.5, xadd(Di, xmul(D0j, kap)));
             d2 = pair_disp<ND>(xi, xj, bx, ibx, dx);
@@ -183,7 +183,7 @@ __device__ __forceinline__ void pair_sums(const DevArrays& b, const DevCtl* ctl,
                 for (int d = 0; d < ND; ++d) out[33 * d + lane] = dx[d];
                 out[33 * ND + lane] = pf.U;
                 out[33 * (ND + 1) + lane] = pf.Lc;
-                out[33 * (ND + 2) + lane] = mixed_gap(d2, r);
+                out[33 * (ND + 2) + lane] = pf.gap;
                 out[33 * (ND + 3) + lane] = pf.Fm;
             } else {
                 PairTerms pt;
@@ -209,7 +209,7 @@ __device__ __forceinline__ void pair_sums(const DevArrays& b, const DevCtl* ctl,
                 const T v = out[33 * f + q];
                 if constexpr (MX) {
                     if (f < ND) sum[f] = __fmaf_rn(out[33 * (ND + 3) + q], v, sum[f]);
-                    else if (f == ND + 2) sum[f] = __fmaf_rn(out[33 * (ND + 1) + q], v, sum[f]);  // += r (dist - r)
+                    else if (f == ND + 2) sum[f] = mixed_add_dk(sum[f], out[33 * (ND + 1) + q], v);
                     else sum[f] += v;
                 } else {
                     sum[f] = xadd(sum[f], v);

@@ -702,7 +702,7 @@ __device__ __forceinline__ void row_pairs(const DevArrays& a, std::uint64_t t, s
             }
             if constexpr (MX) {
                 pd2[u] = mixed_disp<ND>(xi, xj[u], bx, hbf, pdx[u]);
-                pr[u] = 0.5f * (Dif + static_cast<float>(D0j[u]) * kapf);
+                pr[u] = mixed_rij(Dif, static_cast<float>(D0j[u]), kapf);
                 pov[u] = live && pd2[u] < pr[u] * pr[u];
             } else {
                 pr[u] = xmul(0.5, xadd(Di, xmul(D0j[u], kap)));
