@@ -208,6 +208,10 @@ int32_t rcpg_engine_result(rcpg_engine* e, rcpg_result** out, char* err, size_t 
  * where the cluster kernel of small packings applies. Both give the same
  * results bit for bit. */
 void rcpg_engine_step_graph(rcpg_engine* e, int32_t on);
+/* Diagnostic: the later builds of the step graph bring the particles into cell
+ * order by gathers (on != 0) or by scattered moves; an engine chooses by N. The
+ * state is the same bit for bit. */
+void rcpg_engine_gather_builds(rcpg_engine* e, int32_t on);
 void rcpg_engine_destroy(rcpg_engine* e);
 /* Engine diagnostics (no reference counterpart): times `reps` launches of the
  * pair-force kernel on the engine's current state with CUDA events on its

@@ -37,6 +37,7 @@ EXPORTED_SYMBOLS = (
     "rcpg_engine_kernel_launches",
     "rcpg_engine_result",
     "rcpg_engine_step_graph",
+    "rcpg_engine_gather_builds",
     "rcpg_engine_destroy",
     "rcpg_engine_profile_pair_kernel",
     "rcpg_engine_profile_build_kernel",
@@ -217,6 +218,7 @@ def _load() -> C.CDLL:
         "rcpg_engine_kernel_launches": (C.c_uint64, [vp]),
         "rcpg_engine_result": (C.c_int32, [vp, C.POINTER(C.POINTER(Result)), cp, sz]),
         "rcpg_engine_step_graph": (None, [vp, C.c_int32]),
+        "rcpg_engine_gather_builds": (None, [vp, C.c_int32]),
         "rcpg_engine_destroy": (None, [vp]),
         "rcpg_engine_profile_build_kernel": (C.c_int32, [vp, C.c_uint32, _dp, _dp, cp, sz]),
         "rcpg_engine_profile_pair_kernel": (

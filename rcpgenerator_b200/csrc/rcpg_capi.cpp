@@ -498,6 +498,10 @@ void rcpg_engine_step_graph(rcpg_engine* e, int32_t on) {
     if (e) e->eng->prefer_step_graph(on != 0);
 }
 
+void rcpg_engine_gather_builds(rcpg_engine* e, int32_t on) {
+    if (e) e->eng->gather_builds(on != 0);
+}
+
 void rcpg_engine_destroy(rcpg_engine* e) {
     if (!e) return;
     delete e->eng;
@@ -610,6 +614,7 @@ int32_t rcpg_pairs_forces_scan(uint64_t N, int32_t ndim, const double* x_dev, co
         a.P = P;
         // the graph engine's layout: cell-order storage in two buffer sets
         a.permute = 1;
+        a.gather = rcpg::gather_build(N) ? 1 : 0;
         auto dbl = [&](std::size_t n) { return static_cast<double*>(sc.get(n * 8)); };
         auto u32 = [&](std::size_t n) { return static_cast<std::uint32_t*>(sc.get(n * 4)); };
         auto u64 = [&](std::size_t n) { return static_cast<std::uint64_t*>(sc.get(n * 8)); };

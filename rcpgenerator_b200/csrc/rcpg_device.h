@@ -102,6 +102,7 @@ struct DevArrays {
     std::uint64_t N;
     int ndim;
     int P;                  // pos stride
+    int gather;             // cell-order storage: builds gather the particles (gather_build)
     double* pos;            // [N*P] x_0..x_{d-1}, D0 (32-byte aligned records for the force kernel)
     double* pos_tmp;        // [N*P] reorder gather target
     double* spos;           // [N*P] positions in cell order (build scratch; may alias pos_tmp)

@@ -161,6 +161,7 @@ void Engine::alloc_device() {
     // graph mode stores the particles in cell order (every build permutes them
     // into the second buffer set); exact mode keeps the reference's order
     a_.permute = exact_ ? 0 : 1;
+    a_.gather = gather_build(N) ? 1 : 0;
     a_.pos = static_cast<double*>(dalloc(N * P_ * sizeof(double)));
     a_.F = static_cast<double*>(dalloc(N * nd * sizeof(double)));
     a_.m = static_cast<double*>(dalloc(N * nd * sizeof(double)));
@@ -753,7 +754,7 @@ void Engine::destroy_graph() {
 // search.
 std::uint64_t Engine::kernels_per_build() const {
     const std::uint64_t scans = static_cast<std::uint64_t>(a_.C_alloc) + 1 <= 4096 ? 1 : 2;
-    std::uint64_t k = 4 + scans + (a_.permute && gather_build(N_) ? 2 : 1);
+    std::uint64_t k = 4 + scans + (a_.permute && a_.gather ? 2 : 1);
     if (ndim_ <= 3 && N_ >= 20000) {
         if (a_.permute) k += a_.mixed ? 2 : 1;
         else if (a_.sorted_rows) k += 1;

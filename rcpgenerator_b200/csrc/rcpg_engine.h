@@ -183,6 +183,12 @@ class Engine {
     // Later steps by the step graph also where the cluster kernel applies
     // (diagnostic: both give the same results bit for bit).
     void prefer_step_graph(bool on) { step_graph_ = on; }
+    // Which way the step graph's later builds bring the particles into cell
+    // order (diagnostic: the same state either way).
+    void gather_builds(bool on) {
+        a_.gather = on ? 1 : 0;
+        destroy_graph();
+    }
 
    private:
     void setup_host(EngineInput in);

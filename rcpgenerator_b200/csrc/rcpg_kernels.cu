@@ -2424,7 +2424,7 @@ void rebuild_impl(const DevArrays& a, cudaStream_t st, bool planned, cudaEvent_t
     k_build_bin<ND><<<nb, kForceBlock, 0, st>>>(a);
     scan_exclusive(a.cell_count, a.cell_start, a.C_alloc + 1, a.scan_tmp, a.ctl, st);
     k_build_scatter<<<nb, kForceBlock, 0, st>>>(a);
-    const bool gather = a.permute && gather_build(a.N);
+    const bool gather = a.permute && a.gather;
     if (!a.permute || gather) k_build_cell_sort<ND><<<(a.C_alloc + 255) / 256, 256, 0, st>>>(a);
     if (gather) move_nd<ND, true>(a, st);
     else if (a.permute) move_nd<ND, false>(a, st);
