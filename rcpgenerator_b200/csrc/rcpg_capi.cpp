@@ -364,6 +364,7 @@ int32_t run_batch_impl(const rcpg_packing_input* inputs, uint64_t count, const r
             try {
                 rcpg::Engine eng(input_of(k), st);
                 eng.set_blocking_sync(true);  // many host threads: sleep while the GPU works
+                eng.set_engines(nthreads);
                 eng.run(0, false, 0, rcpg::ObserverFn(), nullptr);
                 rcpg::EngineResult r = eng.result();
                 results[k] = make_result(std::move(r), eng.N(), eng.ndim(), nullptr, false, eng.launches());

@@ -225,6 +225,11 @@ void launch_reorder(const DevArrays& a, cudaStream_t st);
 // the kernel's cluster (asked of the driver: once per engine).
 bool small_steps_ok(const DevArrays& a);
 cudaError_t launch_small_steps(const DevArrays& a, std::uint32_t steps, cudaStream_t st);
+// Particles up to which the cluster kernel is the faster way however many steps
+// rebuild; above, only where few of them do (Engine::by_cluster): its 16
+// multiprocessors share a search that the step graph spreads over 148, and a
+// particle has several times the candidates for each dimension more.
+std::uint64_t small_always(int ndim, int nclass, bool many_engines);
 void launch_fix_height(const DevArrays& a, cudaStream_t st);
 
 void launch_pack(std::uint64_t N, int ndim, const double* x, const double* D, double* pos,

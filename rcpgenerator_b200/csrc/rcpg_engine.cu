@@ -869,7 +869,52 @@ void Engine::after_stop() {
 }
 
 namespace {
-constexpr std::uint64_t kSmallSlice = 512;  // steps per launch of the small-packing kernel
+// Steps per launch of the cluster kernel: 5 to 50 ms, after which the host looks
+// at the control block (and another engine's work gets its turn); fewer, and a
+// new choice of the path, where the share of rebuilding steps decides it.
+constexpr std::uint64_t kSmallSlice = 512, kChoiceSteps = 64;
+// Engines at the same time from which the share of the GPU that a step takes
+// counts for more than its time.
+constexpr std::uint64_t kManyEngines = 8;
+}  // namespace
+
+std::uint64_t small_always(int ndim, int nclass, bool many_engines) {
+    // Whole runs from random positions in the unit box, where nearly every step
+    // rebuilds, on one B200, cluster kernel / step graph. d <= 3, N = 8,000:
+    // 13.8 / 19.2 ms (3-D, 200 steps). 4-D, 200 steps, one size class: N = 3,000
+    // 14.9 / 16.9, N = 4,000 19.0 / 17.7, N = 8,000 38.2 / 21.5; several: N =
+    // 1,000 11.0 / 16.7, N = 2,000 22.9 / 20.2, N = 4,000 59.2 / 23.3. 5-D: N =
+    // 1,000 15.9 / 19.6 (several), N = 2,000 20.5 / 17.3, N = 4,000 102 / 21. 6-D,
+    // 60 steps: N = 1,000 9.4 / 9.9 (several), N = 2,000 14.3 / 9.6. 7-D: N =
+    // 1,000 8.8 / 9.2. 8-D: N = 500 7.2 / 10.2, N = 1,000 14.0 / 11.8.
+    // 32 engines at once: 4-D N = 3,000 148 / 202, N = 8,000 117 / 206; 5-D N =
+    // 2,000 139 / 204, N = 4,000 322 / 203; 6-D N = 2,000 98 / 155, N = 4,000 272 /
+    // 178; 8-D N = 1,000 77 / 168; 8 engines: as fast either way or better.
+    if (ndim <= 3) return ~0ull;
+    if (ndim == 4) return many_engines ? ~0ull : (nclass > 1 ? 1500 : 3500);
+    if (many_engines) return ndim <= 6 ? 2500 : 1200;
+    return ndim == 5 ? 1200 : (ndim <= 7 ? 1000 : 700);
+}
+
+// Which way the next steps of a small packing go. Up to small_always() particles
+// the cluster kernel takes all of them. Above, a step without a build is still
+// cheaper there (4-D, N = 8,000: about 15 us against 49) while a build costs
+// more (180 against 50), so the share s of rebuilding steps decides. The two
+// met at s = 0.68 and 0.27 (4-D, one class, N = 4,000 and 8,000), 0.19 (4-D,
+// several, 3,000), 0.33 and 0.07 (5-D, 2,000 and 4,000), 0.25 and 0.04 (6-D,
+// 2,000 and 4,000): at 0.9 (always / N)^2. A run's first steps nearly all
+// rebuild; the cluster kernel takes them where they cost less than capturing the
+// step graph (4 to 5 ms).
+bool Engine::by_cluster(std::uint64_t always) {
+    if (!small_ || step_graph_) return false;
+    if (N_ <= always) return true;
+    const double r = static_cast<double>(always) / static_cast<double>(N_);
+    if (steps_seen_ >= kChoiceSteps) {
+        few_builds_ = static_cast<double>(builds_seen_) <= 0.9 * r * r * static_cast<double>(steps_seen_);
+        steps_seen_ = builds_seen_ = 0;
+        chosen_ = true;
+    }
+    return chosen_ ? few_builds_ : 1.5 * r >= 1.0;
 }
 
 bool Engine::advance_graph(std::uint64_t max_new_steps) {
@@ -902,15 +947,14 @@ bool Engine::advance_graph(std::uint64_t max_new_steps) {
         const std::uint64_t done_steps = c.hist_filled - start;
         if (max_new_steps && done_steps >= max_new_steps) break;
         const std::uint64_t want = max_new_steps ? max_new_steps - done_steps : ~0ull;
-        const bool small = small_ && !step_graph_;
+        const std::uint64_t always = small_always(ndim_, hctl_.nclass, engines_ >= kManyEngines);
+        const bool small = by_cluster(always);
         if (!small && !graph_exec_) capture_graph();
-        const std::uint64_t b0 = hctl_.nbuilds, f0 = hctl_.pair_kernel_runs;
+        const std::uint64_t b0 = hctl_.nbuilds, f0 = hctl_.pair_kernel_runs, s0 = c.hist_filled;
         bool replay = false;
         if (small) {
-            // the steps of a small packing as one cluster kernel, short enough
-            // (a few ms) that other engines' work interleaves
-            check(launch_small_steps(a_, static_cast<std::uint32_t>(std::min<std::uint64_t>(want, kSmallSlice)), st_),
-                  "small steps");
+            const std::uint64_t slice = std::min(want, N_ <= always ? kSmallSlice : kChoiceSteps);
+            check(launch_small_steps(a_, static_cast<std::uint32_t>(slice), st_), "small steps");
             ++launches_;
         } else if (want >= static_cast<std::uint64_t>(graph_steps_)) {
             for (int k = 0; k < graph_steps_; k += captured_steps()) check(cudaGraphLaunch(graph_exec_, st_), "graph launch");
@@ -927,6 +971,8 @@ bool Engine::advance_graph(std::uint64_t max_new_steps) {
         }
         pull_ctl();
         c = hctl_.c;
+        steps_seen_ += c.hist_filled - s0;
+        builds_seen_ += hctl_.nbuilds - b0;
         if (replay) {
             // kernels the replay ran: gate, controller and ADAM of each of its
             // steps (they return at once after a stop), and the builds and pair

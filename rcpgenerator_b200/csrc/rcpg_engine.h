@@ -180,6 +180,9 @@ class Engine {
     // Waits for the device by sleeping on a blocking event instead of spinning
     // (for many engines driven by more host threads than cores: a batch).
     void set_blocking_sync(bool on);
+    // How many engines run at the same time (a batch): among many, what counts
+    // is the share of the GPU that a step takes.
+    void set_engines(std::uint64_t n) { engines_ = n; }
     // Later steps by the step graph also where the cluster kernel applies
     // (diagnostic: both give the same results bit for bit).
     void prefer_step_graph(bool on) { step_graph_ = on; }
@@ -205,6 +208,7 @@ class Engine {
     void finish_step_host();
     bool step_host();
     bool advance_graph(std::uint64_t max_new_steps);
+    bool by_cluster(std::uint64_t always);
     void capture_graph();
     // steps of the captured graph: the largest divisor of graph_steps_ from 8 down
     // to 4, else the smallest one above 8 (fewer than 4 steps: all of them)
@@ -267,6 +271,9 @@ class Engine {
     cudaGraph_t graph_ = nullptr;
     bool small_ = false;       // graph mode: the cluster kernel can run the steps (small_steps_ok)
     bool step_graph_ = false;  // ... but is not asked to
+    // by_cluster(): steps and builds since the last choice, and that choice
+    std::uint64_t engines_ = 1, steps_seen_ = 0, builds_seen_ = 0;
+    bool chosen_ = false, few_builds_ = false;
     std::uint64_t graph_nodes_per_step_ = 0;
     cudaStream_t body_st_ = nullptr;  // captures the bodies of the step graph's conditional nodes
     std::uint32_t* pinned_ = nullptr;

@@ -28,6 +28,7 @@ struct Fake {
     int small_clusters = 0;                    // clusters of the small-packing kernel that fit the device
     std::vector<std::uint64_t> overflow_steps; // steps whose build finds a row beyond the capacity
     std::vector<std::uint32_t> overflow_need;
+    std::uint64_t build_every = 1;             // steps that rebuild
     std::uint64_t reorder_every = 0;           // steps that open with a reorder stop the loop
     // records
     int observer_device = -1;                  // device that was current in every observer call (-2: several)
@@ -78,7 +79,10 @@ void controller(const rcpg::DevArrays& a) {
 }
 
 void step(const rcpg::DevArrays& a) {
-    if (!(a.ctl->stopped | a.ctl->halted)) a.ctl->row_need = need_of(*a.ctl);
+    if (!(a.ctl->stopped | a.ctl->halted)) {
+        a.ctl->row_need = need_of(*a.ctl);
+        if (a.ctl->c.steps % fk.build_every == 0) a.ctl->nbuilds += 1;
+    }
     controller(a);
 }
 
@@ -174,7 +178,7 @@ namespace rcpg {
 void launch_rebuild(const DevArrays& a, cudaStream_t st, bool) {
     if (fk.capturing || !launched(st) || (a.ctl->stopped | a.ctl->halted)) return;
     a.ctl->row_need = need_of(*a.ctl);
-    a.ctl->nbuilds += 1;
+    if (a.ctl->c.steps % fk.build_every == 0) a.ctl->nbuilds += 1;
 }
 void launch_rebuild_timed(const DevArrays& a, cudaStream_t st, cudaEvent_t, cudaEvent_t) { launch_rebuild(a, st, false); }
 void launch_forces(const DevArrays&, int, cudaStream_t st) { launched(st); }
@@ -236,6 +240,8 @@ void hf_overflow(std::uint64_t step, std::uint32_t need) {
     fk.overflow_steps.push_back(step);
     fk.overflow_need.push_back(need);
 }
+void hf_build_every(std::uint64_t steps) { fk.build_every = steps; }
+void hf_engines(void* e, std::uint64_t n) { static_cast<rcpg::Engine*>(e)->set_engines(n); }
 void hf_reorder_every(std::uint64_t steps) { fk.reorder_every = steps; }
 void hf_set_device(int d) { current_device = d; }
 void hf_leave_error() { last_error = cudaErrorInvalidValue; }
@@ -248,12 +254,14 @@ void hf_counts(std::uint64_t* out) {
     out[2] = static_cast<std::uint64_t>(fk.captured);
     out[3] = fk.small_launches;
 }
-void* hf_engine(std::uint64_t N, int exact, int mixed, int graph_steps, std::uint64_t max_steps, int device) {
+void* hf_engine(std::uint64_t N, int ndim, double wide, int exact, int mixed, int graph_steps, std::uint64_t max_steps,
+                int device) {
     rcpg::EngineInput in;
     in.N = N;
-    in.ndim = 2;
-    in.positions.assign(2 * N, 0.5);
+    in.ndim = ndim;
+    in.positions.assign(ndim * N, 0.5);
     in.diameters.assign(N, 0.01);
+    in.diameters[0] *= wide;
     in.fix_diameter = true;
     in.max_steps = max_steps;
     in.reorder_interval = 0;

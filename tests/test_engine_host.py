@@ -18,9 +18,10 @@ def lib():
     lib = C.CDLL(str(HERE / "libhostfake.so"))
     u64, vp = C.c_uint64, C.c_void_p
     lib.hf_overflow.argtypes = [u64, C.c_uint32]
-    lib.hf_reorder_every.argtypes = [u64]
+    lib.hf_reorder_every.argtypes = lib.hf_build_every.argtypes = [u64]
+    lib.hf_engines.argtypes = [vp, u64]
     lib.hf_counts.argtypes = [C.POINTER(u64)]
-    lib.hf_engine.restype, lib.hf_engine.argtypes = vp, [u64, C.c_int, C.c_int, C.c_int, u64, C.c_int]
+    lib.hf_engine.restype, lib.hf_engine.argtypes = vp, [u64, C.c_int, C.c_double, C.c_int, C.c_int, C.c_int, u64, C.c_int]
     lib.hf_free.argtypes = [vp]
     lib.hf_advance.argtypes = [vp, u64]
     lib.hf_steps.restype, lib.hf_steps.argtypes = u64, [vp]
@@ -30,12 +31,12 @@ def lib():
     lib.hf_set_device(0)
 
 
-def _engine(lib, small, graph_steps=32, max_steps=100, overflows=(), exact=0, mixed=0, device=0):
+def _engine(lib, small, graph_steps=32, max_steps=100, overflows=(), exact=0, mixed=0, device=0, n=50, ndim=2, wide=1.0):
     lib.hf_reset(small)
     lib.hf_set_device(device)
     for step, need in overflows:
         lib.hf_overflow(step, need)
-    e = lib.hf_engine(50, exact, mixed, graph_steps, max_steps, device)
+    e = lib.hf_engine(n, ndim, wide, exact, mixed, graph_steps, max_steps, device)
     assert e
     return e
 
@@ -151,3 +152,29 @@ def test_graph_of_any_length_takes_few_launches(lib):
         assert captured <= max(8, min(d for d in range(4, graph_steps + 1) if graph_steps % d == 0)
                                if graph_steps >= 4 else 3)
         lib.hf_free(e)
+
+
+# (ndim, width of the size distribution, engines at once): particles up to which the cluster kernel takes every step
+@pytest.mark.parametrize("ndim,wide,engines,limit", [
+    (2, 1.0, 1, 8192), (3, 9.0, 1, 8192), (4, 1.0, 1, 3500), (4, 9.0, 1, 1500), (4, 9.0, 8, 8192), (5, 1.0, 7, 1200),
+    (5, 1.0, 32, 2500), (6, 9.0, 1, 1000), (6, 1.0, 32, 2500), (7, 1.0, 1, 1000), (8, 1.0, 1, 700), (8, 1.0, 32, 1200),
+])
+def test_path_of_small_packings(lib, ndim, wide, engines, limit):
+    """Above the limit the share of rebuilding steps decides: at most 0.9 (limit / N)^2 of the last 64 or more. The first
+    64 steps are the step graph's above 1.5 times the limit."""
+    for n in (m for m in (limit - 1, limit, limit + 1, 2 * limit) if m <= 8192):  # more never ask for it
+        for every in (1, 8, 2, 64):
+            e = _engine(lib, 1, max_steps=384, n=n, ndim=ndim, wide=wide)
+            lib.hf_engines(e, engines)
+            lib.hf_build_every(every)
+            assert lib.hf_advance(e, 0) == 1 and lib.hf_steps(e) == 384
+            counts = (C.c_uint64 * 4)()
+            lib.hf_counts(counts)
+            steps_of_graph = counts[1] * counts[2]
+            if n <= limit:
+                assert (steps_of_graph, counts[3]) == (0, 1)
+            elif n == limit + 1:  # by the cluster kernel at once
+                assert (steps_of_graph, counts[3]) == ((320, 1) if every == 1 else (0, 6))
+            else:  # by the step graph at once
+                assert (steps_of_graph, counts[3]) == ((384, 0) if every <= 2 else (64, 5))
+            lib.hf_free(e)

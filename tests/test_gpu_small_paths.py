@@ -62,3 +62,21 @@ def test_a_run_may_change_between_the_paths(cuda_device, native):
     eng.close()
     for key in ("positions", "diameters", "phi_history", "force_history", "energy_history", "max_overlap_history"):
         assert np.array_equal(whole[key], cut[key], equal_nan=True), key
+
+
+@pytest.mark.parametrize("n,nd,ratio,side", [(1300, 5, 1.2, 20.0), (3600, 4, 1.0, 20.0), (1600, 4, 3.0, 1.0), (1100, 6, 1.2, 20.0)])
+def test_paths_chosen_by_the_share_of_builds_give_the_same_run(cuda_device, native, n, nd, ratio, side):
+    """Sizes above the line from which few builds decide: by slices of either path, as one run of the step graph."""
+    import rcpgenerator_b200 as rb
+    inp, cfg = _packing(n, nd, ratio, [0] * nd, side)
+    cfg["neighbor_max"] = 3000
+    runs = []
+    for step_graph in (0, 1):
+        eng = rb.PackingEngine(inp, cfg, {"max_steps": 500})
+        native.lib.rcpg_engine_step_graph(eng._h, step_graph)
+        eng.advance(0)
+        runs.append(eng.result())
+        eng.close()
+    a, b = runs
+    for key in ("positions", "diameters", "phi_history", "force_history", "energy_history", "max_overlap_history"):
+        assert np.array_equal(a[key], b[key], equal_nan=True), key
