@@ -321,10 +321,11 @@ __device__ __forceinline__ bool use_cells(const DevArrays& a) {
 }
 
 // Builds with sorted rows but without the tiled search, and large packings in
-// cell-order storage: the members of each cell in ascending particle order in work (the atomic ranks of k_build_bin are arrival order;
-// row slots and per-block force sums must not depend on it), and a copy of
-// their positions in that order (spos), so the search reads each cell's
-// candidates from contiguous memory. The tiled search orders its cells itself.
+// cell-order storage: the members of each cell in ascending particle order in
+// work (the atomic ranks of k_build_bin are arrival order; row slots and
+// per-block force sums must not depend on it), and a copy of their positions in
+// that order (spos), so the search reads each cell's candidates from contiguous
+// memory. The tiled search orders its cells itself.
 template <int ND>
 __global__ void __launch_bounds__(256) k_build_cell_sort(DevArrays a) {
     const DevCtl* ctl = a.ctl;
@@ -2378,11 +2379,16 @@ void launch_warp_search(const DevArrays& a, cudaStream_t st) {
 // Lanes per particle of k_build_rows (the smallest size class): one once the
 // packing alone fills the GPU, more below that. Measured per build on one
 // B200: 3-D log-normal N = 50,003 85 us (1 lane) against 91 (2); N = 12,000 31
-// us (4) against 40 (2), 38 (8) and 46 (16). In 4-D a particle has ten times
-// the candidates and more as it grows: log-normal N = 12,001 over 240 steps 126
-// us (16) against 124 (4, but 155 at the end against 138) and 136 (8); N =
-// 30,000 182 us (8) against 193 (16). Below 8,192 particles only the first build of a run and those
-// after a spatial reorder come here.
+// us (4) against 40 (2), 38 (8) and 46 (16). 2-D bidisperse N = 8,193 14 us (4)
+// against 18 (1), 16 (2), 14 (8); power law N = 16,000 23 (4) against 28 (1), 28
+// (2), 32 (8); N = 40,000 34 (1) against 40 (2), 46 (4); the line lies a little
+// high there (log-normal N = 30,000: 46 against 32 with one lane). In 4-D a
+// particle has ten times the candidates and more as it grows: log-normal N =
+// 12,001 over 240 steps 126 us (16) against 124 (4, but 155 at the end against
+// 138) and 136 (8); N = 30,000 182 us (8) against 193 (16). 5-D and 6-D N =
+// 9,000: 77 and 233 us (16) against 122 and 429 (8). Packings that the cluster
+// kernel steps come here for the first build of a run and after a spatial
+// reorder only.
 template <int ND>
 int search_lanes(std::uint64_t N) {
     if (ND <= 3) return N >= 32768 ? 1 : (N >= 4096 ? 4 : 32);
@@ -2392,8 +2398,9 @@ int search_lanes(std::uint64_t N) {
 // Grid: resident blocks that walk the units with a stride leave SMs idle in the
 // last round (4-D N = 12,001: 1,501 units on 592 resident blocks, the third
 // round half empty), so groups of lanes get twice that many blocks, dealt out as
-// others finish: a run of 250 steps 65.5 -> 62.4 ms (62.9 with three or four
-// times). A thread per particle (power law N = 300,007): 49.5 ms against 51.
+// others finish: 5 % of that packing's step (no more with three or four
+// times). A thread per particle keeps the resident grid: twice the blocks cost
+// 3 % of a step of the power law at N = 300,007.
 template <int ND>
 void launch_rows(const DevArrays& a, cudaStream_t st) {
     const int g0 = search_lanes<ND>(a.N);

@@ -22,9 +22,10 @@
 // Bound by latency: two barriers, the chain partner index -> record -> square
 // root -> division of the longest row, and the controller's serial divisions;
 // what is known earlier (bias corrections, boost) is computed beside them.
-// Whole calls on one B200, set-up included: N = 64 2-D, 3,000 steps 131 -> 28.8
-// ms; N = 2,000 3-D, 1,500 steps of which 1,150 rebuild 118.6 -> 50.7 ms;
-// a batch of 96 packings of up to 4,096 particles (400 steps) 1,284 -> 459 ms.
+// Per step on one B200, set-up included, against the step graph of that time:
+// N = 64 2-D 39.6 -> 9.3 us; N = 2,000 3-D, builds in three steps of four, 75 ->
+// 33 us; a batch of 96 packings of up to 4,096 particles 2.7 times as fast.
+// Where it runs: small_steps_ok, small_always, Engine::by_cluster.
 //
 // Work is dealt out by warps of 32 consecutive particles: warp w of the
 // packing belongs to block w mod C. N <= kSmallN, so that a thread has at most

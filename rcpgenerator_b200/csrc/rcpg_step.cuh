@@ -418,7 +418,7 @@ __device__ __forceinline__ std::uint32_t search_row_one(const DevArrays& a, cons
     const std::uint64_t N = a.N;
     const std::uint32_t S = a.S;
     const float* const fpos = a.fpos;
-        RowSearch<ND, NC> rs;
+    RowSearch<ND, NC> rs;
     rs.begin(a, t, sp.kap, sp.t_shell, sp.widest);
     auto flush = [&]() {
         for (std::uint32_t k = 0; k < rs.listed; ++k) {
