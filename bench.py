@@ -42,9 +42,9 @@ PEAKS = REPO / "MEASURED_PEAKS.json"
 # the N = 1M launch is too large to capture with the full metric set
 FORCES_TRAFFIC_PER_ALG_BYTE = 23.2 / 20.26
 # the same for the cell-unit build with fused forces, k_cells<2, mixed>
-# (profiles/k_cells_bidisperse2d_n3e5_mixed.md: 12.3 MB for 22.7 MB at N = 300k; the rows and
+# (profiles/k_cells_bidisperse2d_n3e5_mixed.md: 16.7 MB for 22.7 MB at N = 300k; the rows and
 # forces it writes are still in L2 when the launch ends)
-BUILD_TRAFFIC_PER_ALG_BYTE = 12.3 / 22.7
+BUILD_TRAFFIC_PER_ALG_BYTE = 16.7 / 22.7
 
 
 def workload_name(n: int) -> str:
