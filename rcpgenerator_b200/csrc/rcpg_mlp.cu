@@ -291,6 +291,7 @@ bool carve(void* ws, std::size_t ws_bytes, const int32_t* w, int L, int B, Work&
     wk.z.resize(L);
     for (int l = 0; l <= L; ++l) wk.act[l] = static_cast<__nv_bfloat16*>(take(static_cast<std::size_t>(B) * w[l] * 2));
     for (int l = 0; l < L; ++l) wk.z[l] = static_cast<float*>(take(static_cast<std::size_t>(B) * w[l + 1] * 4));
+    take(static_cast<std::size_t>(B) * wmax * 4);
     wk.dz = static_cast<__nv_bfloat16*>(take(static_cast<std::size_t>(B) * wmax * 2));
     wk.dzp = static_cast<__nv_bfloat16*>(take(static_cast<std::size_t>(B) * wmax * 2));
     wk.lterm = static_cast<float*>(take(static_cast<std::size_t>(B) * w[L] * 4));
@@ -352,7 +353,7 @@ uint64_t rcpg_mlp_workspace_bytes(const int32_t* widths, int32_t layers, int32_t
         b += static_cast<std::size_t>(batch) * widths[l] * 2 + 256;
     }
     for (int l = 0; l < layers; ++l) b += static_cast<std::size_t>(batch) * widths[l + 1] * 4 + 256;
-    b += static_cast<std::size_t>(batch) * wmax * 4 + 2 * 256 + static_cast<std::size_t>(batch) * widths[layers] * 4 + 256;
+    b += static_cast<std::size_t>(batch) * wmax * 8 + 3 * 256 + static_cast<std::size_t>(batch) * widths[layers] * 4 + 256;
     return b;
 }
 
