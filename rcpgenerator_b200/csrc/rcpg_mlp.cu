@@ -291,7 +291,7 @@ bool carve(void* ws, std::size_t ws_bytes, const int32_t* w, int L, int B, Work&
     wk.z.resize(L);
     for (int l = 0; l <= L; ++l) wk.act[l] = static_cast<__nv_bfloat16*>(take(static_cast<std::size_t>(B) * w[l] * 2));
     for (int l = 0; l < L; ++l) wk.z[l] = static_cast<float*>(take(static_cast<std::size_t>(B) * w[l + 1] * 4));
-    take(static_cast<std::size_t>(B) * wmax * 4);
+    take(static_cast<std::size_t>(B) * wmax * 4);  // unused; rcpg_mlp_workspace_bytes keeps the size it has always returned
     wk.dz = static_cast<__nv_bfloat16*>(take(static_cast<std::size_t>(B) * wmax * 2));
     wk.dzp = static_cast<__nv_bfloat16*>(take(static_cast<std::size_t>(B) * wmax * 2));
     wk.lterm = static_cast<float*>(take(static_cast<std::size_t>(B) * w[L] * 4));
